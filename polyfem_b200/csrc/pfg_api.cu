@@ -1571,6 +1571,35 @@ static int system_pattern(pfg_context *c, int system, int &n, long long &nnz, co
 	return fail(c, PFG_ERR_INVALID, "bad system");
 }
 
+// Rest position of the node of every column of a system (3 n doubles): the geometric
+// node, or the midpoint of the edge a P2 node sits on.
+static int column_positions(pfg_context *c, int system, int n, std::vector<double> &pos)
+{
+	const int E = c->m.E, N = c->m.N, Ng = c->m.Ng, nn = c->n;
+	std::vector<double> X(3 * (size_t)std::max(Ng, 1)), node(3 * (size_t)std::max(N, 1), 0.0);
+	std::vector<int> gc((size_t)std::max(E, 1) * c->ng), free_dofs((size_t)std::max(n, 1));
+	if (Ng) PFG_CUDA(c, cudaMemcpy(X.data(), c->m.X, sizeof(double) * 3 * (size_t)Ng, cudaMemcpyDeviceToHost));
+	if (E) PFG_CUDA(c, cudaMemcpy(gc.data(), c->m.gconn, sizeof(int) * (size_t)E * c->ng, cudaMemcpyDeviceToHost));
+	static const int edges[6][2] = {{0, 1}, {1, 2}, {2, 0}, {0, 3}, {1, 3}, {2, 3}};
+	for (int e = 0; e < E; ++e)
+		for (int a = 0; a < nn; ++a)
+		{
+			const int v0 = a < c->ng ? a : edges[a - 4][0], v1 = a < c->ng ? a : edges[a - 4][1];
+			const double *x0 = X.data() + 3 * (size_t)gc[(size_t)v0 * E + e], *x1 = X.data() + 3 * (size_t)gc[(size_t)v1 * E + e];
+			double *x = node.data() + 3 * (size_t)c->h_conn[(size_t)e * nn + a];
+			for (int d = 0; d < 3; ++d) x[d] = 0.5 * (x0[d] + x1[d]);
+		}
+	pos.assign(3 * (size_t)std::max(n, 1), 0.0);
+	if (system == PFG_SYS_REDUCED && n)
+		PFG_CUDA(c, cudaMemcpy(free_dofs.data(), c->d_free, sizeof(int) * (size_t)n, cudaMemcpyDeviceToHost));
+	for (int j = 0; j < n; ++j)
+	{
+		const int dof = system == PFG_SYS_REDUCED ? free_dofs[j] : j;
+		for (int d = 0; d < 3; ++d) pos[3 * (size_t)j + d] = node[3 * (size_t)(dof / 3) + d];
+	}
+	return PFG_OK;
+}
+
 int pfg_direct_analyze(pfg_context *c, int system)
 {
 	if (!c) return fail(c, PFG_ERR_INVALID, "bad arguments");
@@ -1585,9 +1614,11 @@ int pfg_direct_analyze(pfg_context *c, int system)
 	PFG_CUDA(c, cudaStreamSynchronize(c->stream));
 	PFG_CUDA(c, cudaMemcpy(outer.data(), d_outer, sizeof(int) * ((size_t)n + 1), cudaMemcpyDeviceToHost));
 	if (nnz) PFG_CUDA(c, cudaMemcpy(inner.data(), d_inner, sizeof(int) * (size_t)nnz, cudaMemcpyDeviceToHost));
+	std::vector<double> pos;
+	if (int st = column_positions(c, system, n, pos)) return st;
 	pfg::DirectFactor *f = nullptr;
 	std::string msg;
-	if (int st = direct_symbolic(n, outer.data(), inner.data(), &f, msg)) return fail(c, st, msg);
+	if (int st = direct_symbolic(n, outer.data(), inner.data(), pos.data(), &f, msg)) return fail(c, st, msg);
 	if (int st = direct_upload(f, msg))
 	{
 		direct_destroy(f);
@@ -1670,7 +1701,7 @@ int pfg_direct_symbolic(int n, const int *outer, const int *inner, long long *st
 	}
 	pfg::DirectFactor *f = nullptr;
 	std::string msg;
-	if (int st = direct_symbolic(n, outer, inner, &f, msg)) return fail(nullptr, st, msg);
+	if (int st = direct_symbolic(n, outer, inner, nullptr, &f, msg)) return fail(nullptr, st, msg);
 	direct_stats(f, stats);
 	direct_destroy(f);
 	return PFG_OK;

@@ -207,13 +207,14 @@ cudaError_t launch_cg_iterations(int n, int count, int ngroups, const int *group
 void set_global_error(const std::string &msg);
 
 // Sparse direct solve (pfg_direct.cu): multifrontal Cholesky of an SPD matrix in a
-// CSC pattern.  direct_symbolic analyses a host pattern (0 or a PFG error code),
+// CSC pattern.  direct_symbolic analyses a host pattern, with the columns' positions
+// (3 n doubles) where they are known (0 or a PFG error code),
 // direct_upload moves its maps to the device, direct_factorize factorises device
 // values (0 ok, 1 not positive definite, 2 CUDA error in *ce), direct_solve
 // solves for device vectors (x may alias b).  direct_stats: n, fronts, levels,
 // front doubles, entries of L, largest front, flops of the factorisation.
 struct DirectFactor;
-int direct_symbolic(int n, const int *outer, const int *inner, DirectFactor **out, std::string &msg);
+int direct_symbolic(int n, const int *outer, const int *inner, const double *node_pos, DirectFactor **out, std::string &msg);
 int direct_upload(DirectFactor *f, std::string &msg);
 int direct_factorize(DirectFactor *f, const double *vals, cudaStream_t s, cudaError_t *ce);
 cudaError_t direct_solve(DirectFactor *f, const double *b, double *x, cudaStream_t s);
