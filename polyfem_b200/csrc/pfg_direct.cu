@@ -20,14 +20,15 @@
 //   factorisation (device): fronts of equal height in the tree are processed by
 //     the same launches, leaves first: A's lower entries are scattered into the
 //     zeroed fronts, the children's update matrices are added in child order,
-//     and each front is partially factorised in pairs of 32-column panels
-//     (Cholesky of each diagonal block, triangular solve of the rows below, the
-//     first panel's update of the second, then one rank-64 update of the trailing
-//     lower triangle in 64 x 64 tiles); the trailing block is the update matrix
-//     the parent adds.
+//     and each front is partially factorised in pairs of 64-column panels
+//     (Cholesky and inverse of each diagonal block, the rows below times the
+//     inverse, the first panel's update of the second, then one rank-128 update of
+//     the trailing lower triangle, all products on the FP64 tensor pipe); the
+//     trailing block is the update matrix the parent adds.
 //   solve (device): forward substitution leaves first (each front adds its
 //     children's update vectors in child order), backward substitution from the
-//     root, then the inverse permutation.
+//     root, then the inverse permutation.  The diagonal blocks hold the inverses of
+//     their triangles, so each panel step is two products in one launch.
 // Every sum is taken in a fixed order, so factor and solution are bitwise
 // deterministic.  Fronts are dense lower triangles of m (m + 1) / 2 doubles
 // (packed columns), all resident for the factor's lifetime.
@@ -47,15 +48,11 @@ namespace pfg
 namespace
 {
 
-constexpr int NB = 32;          // panel width of the triangular solves
-constexpr int NBF = 64;         // panel width of the partial factorisation
+constexpr int NBF = 64;         // panel width
 constexpr int LEAF_DOFS = 96;   // dissection stops at parts of at most this many dofs
 constexpr double MAX_HALF = 0.7; // largest share of a part that one side of a cut may keep
 constexpr double BALANCE = 1.0;  // weight of the imbalance in a cut's cost
-constexpr int TRSM_ROWS = 128;  // rows per CTA of the panel solve
-constexpr int TILE = 64;        // trailing-update tile
-constexpr int FWD_ROWS = 256;   // rows per CTA of the forward solve's panel update
-constexpr int BWD_ROWS = 512;   // rows per CTA of the backward solve's panel sums
+constexpr int ROWS_TILE = 64;   // rows per CTA of the panel solve and of the forward substitution
 
 struct DevFront
 {
@@ -77,8 +74,8 @@ __host__ __device__ __forceinline__ long long pk(int m, int j) { return (long lo
 
 struct Panel
 {
-	int lvl, j0, rows_grid, tiles_grid;
-	int fwd_grid, bwd_grid; // CTAs per front of the solve's panel steps
+	int lvl, j0;
+	int rows_grid, upd_grid, tiles_grid; // CTAs per front: rows below, update of the second panel, trailing update
 };
 
 } // namespace
@@ -95,9 +92,7 @@ struct DirectFactor
 	std::vector<long long> lvl_fbeg;   // front doubles of each level [lvl_fbeg[h], lvl_fbeg[h+1])
 	std::vector<long long> lvl_abeg;   // A-map entries of each level
 	std::vector<int> lvl_maxchild, lvl_maxrc, lvl_maxk;
-	int max_bwd_part = 0; // doubles of backward partial sums for one panel step
-	std::vector<Panel> panels;         // solve panels (NB columns) in order
-	std::vector<Panel> fpanels;        // factorisation panels (NBF columns) in order
+	std::vector<Panel> panels;         // 64-column panels, level by level, in order
 	long long front_doubles = 0, work_doubles = 0, amap_n = 0;
 	// host maps between the analysis and the upload
 	std::vector<int> h_child, h_relpos, h_rows, h_amap_src;
@@ -109,7 +104,6 @@ struct DirectFactor
 	long long *d_amap_dst = nullptr;
 	double *d_front = nullptr, *d_work = nullptr, *d_vec = nullptr; // d_vec: 2 n (permuted rhs, solution)
 	double *d_io = nullptr;                                          // n: b and x of a host-memory solve
-	double *d_part = nullptr;                                        // backward panel partial sums
 	int *d_err = nullptr;
 	bool factorized = false;
 };
@@ -377,7 +371,7 @@ void direct_destroy(DirectFactor *f)
 {
 	if (!f) return;
 	void *ptrs[] = {f->d_fr,       f->d_lvl_list, f->d_child, f->d_relpos, f->d_rows, f->d_perm, f->d_amap_src,
-					f->d_amap_dst, f->d_front,    f->d_work,  f->d_vec,    f->d_io,   f->d_err, f->d_part};
+					f->d_amap_dst, f->d_front,    f->d_work,  f->d_vec,    f->d_io,   f->d_err};
 	for (void *p : ptrs)
 		if (p) cudaFree(p); // a host-only analysis never touches the runtime
 	delete f;
@@ -614,7 +608,7 @@ int direct_symbolic(int n, const int *outer, const int *inner, const double *nod
 	f->front_doubles = fo;
 	f->work_doubles = wo;
 	f->amap_n = (long long)amap_src.size();
-	// 6. panel launches of the factorisation
+	// 6. panel launches of the factorisation and the solve
 	for (int h = 0; h < nl; ++h)
 	{
 		int maxk = 0;
@@ -622,59 +616,26 @@ int direct_symbolic(int n, const int *outer, const int *inner, const double *nod
 		f->lvl_maxk.push_back(maxk);
 		for (int j0 = 0; j0 < maxk; j0 += NBF)
 		{
-			// rows_grid: panel A's rows below; fwd_grid: rows of A's update of B (0 when
-			// no front has a panel B); bwd_grid: panel B's rows below; tiles_grid: the
-			// rank-64 trailing update
-			long long ra = 0, ru = 0, rb = 0, tg = 0;
+			// rows of 64 below the panel; of a pair's first panel: rows of 64 of its update
+			// of the second panel (0 when no front has one), tiles of the rank-128 update
+			long long rows = 0, upd = 0, tiles = 0;
 			for (int t = f->lvl_start[h]; t < f->lvl_start[h + 1]; ++t)
 			{
 				const DevFront &d = f->fr[f->lvl_list[t]];
 				if (d.k <= j0) continue;
-				const int na = std::min(NB, d.k - j0);
-				ra = std::max(ra, ((long long)d.m - j0 - na + TRSM_ROWS - 1) / TRSM_ROWS);
-				if (d.k > j0 + NB)
-				{
-					const int nbb = std::min(NB, d.k - j0 - NB);
-					ru = std::max(ru, ((long long)d.m - j0 - NB + TRSM_ROWS - 1) / TRSM_ROWS);
-					rb = std::max(rb, ((long long)d.m - j0 - NB - nbb + TRSM_ROWS - 1) / TRSM_ROWS);
-				}
-				const int nb = std::min(NBF, d.k - j0);
-				const long long below = d.m - j0 - nb;
-				const long long nt = (below + TILE - 1) / TILE;
-				tg = std::max(tg, nt * (nt + 1) / 2);
+				const int nb = std::min(NBF, d.k - j0), nb2 = std::min(2 * NBF, d.k - j0);
+				rows = std::max(rows, ((long long)d.m - j0 - nb + ROWS_TILE - 1) / ROWS_TILE);
+				if (d.k > j0 + NBF) upd = std::max(upd, ((long long)d.m - j0 - NBF + ROWS_TILE - 1) / ROWS_TILE);
+				const long long n64 = (d.m - j0 - nb2 + 63) / 64, hh = n64 / 2;
+				tiles = std::max(tiles, n64 % 2 ? (hh + 1) * (hh + 1) : hh * (hh + 1));
 			}
-			if (tg > 0x7fffffffLL)
+			if (tiles > 0x3fffffffLL)
 			{
 				msg = "direct solver front too large";
 				direct_destroy(f);
 				return PFG_ERR_UNSUPPORTED;
 			}
-			f->fpanels.push_back({h, j0, (int)ra, (int)tg, (int)ru, (int)rb});
-		}
-		for (int j0 = 0; j0 < maxk; j0 += NB)
-		{
-			long long rg = 0, tg = 0, fg = 0, bg = 1;
-			for (int t = f->lvl_start[h]; t < f->lvl_start[h + 1]; ++t)
-			{
-				const DevFront &d = f->fr[f->lvl_list[t]];
-				if (d.k <= j0) continue;
-				const int nb = std::min(NB, d.k - j0);
-				const long long below = d.m - j0 - nb;
-				rg = std::max(rg, (below + TRSM_ROWS - 1) / TRSM_ROWS);
-				const long long nt = (below + TILE - 1) / TILE;
-				tg = std::max(tg, nt * (nt + 1) / 2);
-				fg = std::max(fg, (below + FWD_ROWS - 1) / FWD_ROWS);
-				bg = std::max(bg, ((long long)d.k - j0 - nb + BWD_ROWS - 1) / BWD_ROWS);
-			}
-			if (tg > 0x7fffffffLL)
-			{
-				msg = "direct solver front too large";
-				direct_destroy(f);
-				return PFG_ERR_UNSUPPORTED;
-			}
-			f->panels.push_back({h, j0, (int)rg, (int)tg, (int)fg, (int)bg});
-			const long long nfl = f->lvl_start[h + 1] - f->lvl_start[h];
-			f->max_bwd_part = (int)std::max<long long>(f->max_bwd_part, nfl * bg * NB);
+			f->panels.push_back({h, j0, (int)rows, (int)upd, (int)tiles});
 		}
 	}
 	for (int h = 0; h < nl; ++h)
@@ -724,7 +685,7 @@ int direct_upload(DirectFactor *f, std::string &msg)
 		msg = cudaGetErrorString(e);
 		return PFG_ERR_CUDA;
 	}
-	const double need = 8.0 * (double)fo + 8.0 * (double)wo + 12.0 * (double)f->amap_n + 24.0 * n + 8.0 * f->max_bwd_part;
+	const double need = 8.0 * (double)fo + 8.0 * (double)wo + 12.0 * (double)f->amap_n + 24.0 * n;
 	if (need > 0.85 * (double)fre)
 	{
 		msg = "direct solver needs " + std::to_string((long long)(need / 1e6)) + " MB of device memory for its fronts, " +
@@ -740,7 +701,6 @@ int direct_upload(DirectFactor *f, std::string &msg)
 		(e = cudaMalloc(&f->d_work, 8 * std::max<long long>(wo, 1))) != cudaSuccess ||
 		(e = cudaMalloc(&f->d_vec, 16 * (size_t)std::max(n, 1))) != cudaSuccess ||
 		(e = cudaMalloc(&f->d_io, 8 * (size_t)std::max(n, 1))) != cudaSuccess ||
-		(e = cudaMalloc(&f->d_part, 8 * (size_t)std::max(f->max_bwd_part, 1))) != cudaSuccess ||
 		(e = cudaMalloc(&f->d_err, sizeof(int))) != cudaSuccess)
 	{
 		msg = cudaGetErrorString(e);
@@ -810,228 +770,431 @@ __global__ void __launch_bounds__(256) k_dir_extend_add(const DevFront *__restri
 	for (int a = b + lane; a < rc; a += 32) P[rp[a]] += U[a];
 }
 
-// Cholesky of the diagonal block of panel j0 (one warp per front): lane i holds row
-// i of the block in registers; column c's entries reach the other lanes by shuffle
-__global__ void __launch_bounds__(32) k_dir_potrf(const DevFront *__restrict__ fr, const int *__restrict__ list,
+__device__ __forceinline__ void cp_async8(double *dst, const double *src, bool ok)
+{
+	const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+	const int bytes = ok ? 8 : 0; // 0: the 8 bytes are zero-filled and src is not read
+	asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// c (16 x 8) += a (16 x 4) b (4 x 8) on the FP64 tensor pipe: lane t holds a[t / 4 (+ 8)][t % 4],
+// b[t % 4][t / 4] and c[t / 4 (+ 8)][2 (t % 4) + {0, 1}]
+__device__ __forceinline__ void dmma(double (&c0)[2], double (&c1)[2], double a0, double a1, double b)
+{
+	asm("mma.sync.aligned.m16n8k4.row.col.f64.f64.f64.f64 {%0,%1,%2,%3},{%4,%5},{%6},{%0,%1,%2,%3};"
+		: "+d"(c0[0]), "+d"(c0[1]), "+d"(c1[0]), "+d"(c1[1])
+		: "d"(a0), "d"(a1), "d"(b));
+}
+
+// the same with k = 8: a0..a3 are a[t / 4 (+ 8 for odd)][t % 4 (+ 4 from a2 on)], b0, b1 are b[t % 4 (+ 4)][t / 4]
+__device__ __forceinline__ void dmma_k8(double (&c0)[2], double (&c1)[2], const double (&a)[4], double b0, double b1)
+{
+	asm("mma.sync.aligned.m16n8k8.row.col.f64.f64.f64.f64 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
+		: "+d"(c0[0]), "+d"(c0[1]), "+d"(c1[0]), "+d"(c1[1])
+		: "d"(a[0]), "d"(a[1]), "d"(a[2]), "d"(a[3]), "d"(b0), "d"(b1));
+}
+// an 8 x 8 tile, c += a (8 x 4) b (4 x 8)
+__device__ __forceinline__ void dmma_8x8(double (&c)[2], double a, double b)
+{
+	asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
+}
+
+// 1 / d of a positive finite d: hardware approximation and two Newton steps where its
+// flush-to-zero range is safe, else the division
+__device__ __forceinline__ double pivot_rcp(double d)
+{
+	if (!(d > 1e-290 && d < 1e290)) return 1.0 / d;
+	double r;
+	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+	r = fma(fma(-d, r, 1.0), r, r);
+	return fma(fma(-d, r, 1.0), r, r);
+}
+
+// The factorisation runs in panels of 64 columns, two at a time:
+//   k_dir_diag: Cholesky of the 64 x 64 diagonal block; the block's place in the
+//     factor receives the inverse of its triangle, so that everything after it (the
+//     rows below, both substitutions) is a product instead of a dependent recurrence;
+//   k_dir_rows<true>: the rows below times that inverse, X = B L_d^-T;
+//   k_dir_rows<false>: the first panel's update of the second panel's columns;
+//   (the same two kernels for the second panel;)
+//   k_dir_update: the rank-128 update of the trailing lower triangle, so the
+//     trailing matrix is read and written once per 128 columns.
+//
+// k_dir_diag, one CTA per front, the block in shared memory.  One warp factorises eight
+// columns (two rows per lane, pivots and multipliers by shuffle), then all warps apply
+// them to the rest in 8 x 8 tiles on the FP64 tensor pipe.  The triangle's inverse is
+// put together from the inverses of its eight 8 x 8 blocks by doubling:
+// [A 0; B C]^-1 = [A^-1 0; -C^-1 B A^-1 C^-1].  Bound by the 64 dependent pivot steps.
+// One barrier and one rank-1 update of all entries per column took 28 us a block at
+// P2 24^3 (two one-warp 32-column blocks with a substitution each: 60 us); this takes 20.
+constexpr int DIAG_LD = NBF + 4; // 4 mod 16: a fragment's rows fall on distinct banks
+constexpr int DIAG_SLD = 12;     // the same for the eight scaled panel columns
+constexpr size_t DIAG_SMEM = (2 * NBF * DIAG_LD + NBF * DIAG_SLD + NBF) * sizeof(double);
+__global__ void __launch_bounds__(256) k_dir_diag(const DevFront *__restrict__ fr, const int *__restrict__ list,
 												  double *__restrict__ F, int j0, int *__restrict__ err)
 {
 	constexpr unsigned FULL = 0xffffffffu;
 	const DevFront f = fr[list[blockIdx.x]];
 	if (j0 >= f.k) return;
-	const int nb = min(NB, f.k - j0), lane = threadIdx.x;
-	double *Fb = F + f.foff;
-	const bool row = lane < nb;
-	double v[NB];
-	{
-		long long cb = pk(f.m, j0) + j0 + lane; // entry (j0 + lane, j0 + c)
+	const int nb = min(NBF, f.k - j0), tid = threadIdx.x, r = tid % NBF, g = tid / NBF;
+	const int lane = tid & 31, warp = tid >> 5, fk = lane & 3, fr_ = lane >> 2;
+	double *Fb = F + f.foff + pk(f.m, j0) + j0; // entry (j0 + i, j0 + l) at l (m - j0) - l (l + 1) / 2 + i
+	const int ld = f.m - j0;
+	extern __shared__ __align__(16) double dsm[];
+	double(*M)[DIAG_LD] = reinterpret_cast<double(*)[DIAG_LD]>(dsm);                  // the block, by rows
+	double(*V)[DIAG_LD] = reinterpret_cast<double(*)[DIAG_LD]>(dsm + NBF * DIAG_LD);  // its triangle's inverse
+	double(*S)[DIAG_SLD] = reinterpret_cast<double(*)[DIAG_SLD]>(dsm + 2 * NBF * DIAG_LD); // panel columns over their pivots
+	double *rs = dsm + 2 * NBF * DIAG_LD + NBF * DIAG_SLD;                            // pivots, then 1 / sqrt
 #pragma unroll
-		for (int c = 0; c < NB; ++c)
-		{
-			v[c] = row && c <= lane && c < nb ? Fb[cb] : 0.0;
-			cb += f.m - (j0 + c) - 1;
-		}
-	}
-	bool bad = false;
-#pragma unroll
-	for (int c = 0; c < NB; ++c)
+	for (int i = 0; i < 16; ++i)
 	{
-		if (c >= nb) break;
-		double d = __shfl_sync(FULL, v[c], c);
-		if (!(d > 0.0) || !(d <= 1.7976931348623157e308))
-		{
-			bad = true;
-			d = 1.0;
-		}
-		d = sqrt(d);
-		const double lc = lane == c ? d : (lane > c ? v[c] / d : 0.0); // L[lane][c]
-		if (lane >= c) v[c] = lc;
-#pragma unroll
-		for (int l = c + 1; l < NB; ++l)
-		{
-			const double llc = __shfl_sync(FULL, lc, l); // L[l][c]
-			if (lane >= l && l < nb) v[l] = fma(-lc, llc, v[l]);
-		}
-	}
-	if (bad && lane == 0) atomicExch(err, 1);
-	{
-		long long cb = pk(f.m, j0) + j0 + lane;
-#pragma unroll
-		for (int c = 0; c < NB; ++c)
-		{
-			if (row && c <= lane && c < nb) Fb[cb] = v[c];
-			cb += f.m - (j0 + c) - 1;
-		}
-	}
-}
-
-// rows below the panel: X L_d^T = B, one row per thread
-__global__ void __launch_bounds__(TRSM_ROWS) k_dir_trsm(const DevFront *__restrict__ fr, const int *__restrict__ list,
-														double *__restrict__ F, int j0)
-{
-	const DevFront f = fr[list[blockIdx.y]];
-	if (j0 >= f.k) return;
-	const int nb = min(NB, f.k - j0);
-	__shared__ double D[NB][NB + 1];
-	double *Fb = F + f.foff;
-	for (int t = threadIdx.x; t < nb * nb; t += TRSM_ROWS)
-	{
-		const int r = t % nb, c = t / nb;
-		if (r >= c) D[r][c] = Fb[(size_t)(j0 + r) + pk(f.m, j0 + c)];
+		const int l = 4 * i + g;
+		// rows past the block's end continue it as the identity
+		M[r][l] = r < nb && l <= r ? Fb[l * ld - l * (l + 1) / 2 + r] : (r == l ? 1.0 : 0.0);
+		V[r][l] = 0.0;
 	}
 	__syncthreads();
-	const long long i = (long long)j0 + nb + (long long)blockIdx.x * TRSM_ROWS + threadIdx.x;
-	if (i >= f.m) return;
-	double x[NB];
-	const long long c0 = pk(f.m, j0) + i; // entry (i, j0); column j0 + l + 1 starts m - (j0 + l) - 1 later
+#pragma unroll 1
+	for (int cb = 0; cb < 8; ++cb)
 	{
-		long long cb = c0;
-#pragma unroll
-		for (int l = 0; l < NB; ++l)
+		const int c0 = 8 * cb;
+		if (warp == 0)
 		{
-			if (l < nb) x[l] = Fb[cb];
-			cb += f.m - (j0 + l) - 1;
-		}
-	}
+			double p[2][8], s[2][8];
 #pragma unroll
-	for (int l = 0; l < NB; ++l)
-		if (l < nb)
+			for (int q = 0; q < 8; ++q)
+			{
+				p[0][q] = M[lane][c0 + q];
+				p[1][q] = M[lane + 32][c0 + q];
+			}
+			bool bad = false;
+			const bool up = c0 >= 32; // the panel's diagonal rows sit in the upper half of the lanes' rows
+#pragma unroll
+			for (int q = 0; q < 8; ++q)
+			{
+				const double x = up ? p[1][q] : p[0][q];
+				double d = __shfl_sync(FULL, x, (c0 + q) & 31);
+				if (!(d > 0.0) || !(d <= 1.7976931348623157e308))
+				{
+					bad = true;
+					d = 1.0;
+				}
+				if (lane == 0) rs[c0 + q] = d;
+				const double rd = pivot_rcp(d);
+				s[0][q] = p[0][q] * rd;
+				s[1][q] = p[1][q] * rd;
+#pragma unroll
+				for (int l = q + 1; l < 8; ++l)
+				{
+					const double y = __shfl_sync(FULL, x, (c0 + l) & 31);
+					p[0][l] = fma(-s[0][q], y, p[0][l]);
+					p[1][l] = fma(-s[1][q], y, p[1][l]);
+				}
+			}
+#pragma unroll
+			for (int q = 0; q < 8; ++q)
+			{
+				M[lane][c0 + q] = p[0][q];
+				M[lane + 32][c0 + q] = p[1][q];
+				S[lane][q] = s[0][q];
+				S[lane + 32][q] = s[1][q];
+			}
+			if (bad && lane == 0) atomicExch(err, 1);
+		}
+		__syncthreads();
+		// M -= S (panel)^T over the 8 x 8 tiles (i, j), cb < j <= i < 8
+		const int nt = 7 - cb;
+		for (int x = warp; x < nt * (nt + 1) / 2; x += 8)
 		{
-			double s = x[l];
-#pragma unroll
-			for (int t = 0; t < l; ++t) s = fma(-x[t], D[l][t], s);
-			x[l] = s / D[l][l];
+			int i = 0, j = x;
+			while (j > i) j -= ++i;
+			i = 8 * (cb + 1 + i);
+			j = 8 * (cb + 1 + j);
+			double2 *C = reinterpret_cast<double2 *>(&M[i + fr_][j + 2 * fk]);
+			const double2 v = *C;
+			double c[2] = {v.x, v.y};
+			dmma_8x8(c, -S[i + fr_][fk], M[j + fr_][c0 + fk]);
+			dmma_8x8(c, -S[i + fr_][4 + fk], M[j + fr_][c0 + 4 + fk]);
+			*C = make_double2(c[0], c[1]);
 		}
-	{
-		long long cb = c0;
-#pragma unroll
-		for (int l = 0; l < NB; ++l)
-		{
-			if (l < nb) Fb[cb] = x[l];
-			cb += f.m - (j0 + l) - 1;
-		}
+		__syncthreads();
 	}
-}
-
-// The factorisation runs in pairs of 32-column panels A = [j0, j0+32) and
-// B = [j0+32, j0+64): A is factorised (k_dir_potrf, k_dir_trsm), its update is
-// applied to B's columns alone (k_dir_panel_update), B is factorised, and one
-// rank-64 update of the trailing lower triangle by both panels follows
-// (k_dir_syrk64), so the trailing matrix is read and written once per 64 columns.
-// k_dir_panel_update: F[i][j0+32+c] -= sum_l F[i][j0+l] F[j0+32+c][j0+l] for the
-// rows i >= j0+32+c, a thread per row, A's rows of B's columns in shared memory.
-__global__ void __launch_bounds__(TRSM_ROWS) k_dir_panel_update(const DevFront *__restrict__ fr,
-																const int *__restrict__ list, double *__restrict__ F,
-																int j0)
-{
-	const DevFront f = fr[list[blockIdx.y]];
-	const int jb = j0 + NB;
-	if (jb >= f.k) return;
-	const int nc = min(NB, f.k - jb);
-	__shared__ double M[NB][NB + 1]; // M[c][l] = F[jb + c][j0 + l]
-	__shared__ long long cofs[NB];   // pk of columns j0 + l
-	double *Fb = F + f.foff;
-	if (threadIdx.x < NB) cofs[threadIdx.x] = pk(f.m, j0 + threadIdx.x);
-	__syncthreads();
-	for (int t = threadIdx.x; t < NB * NB; t += TRSM_ROWS)
+	if (tid < NBF)
 	{
-		const int c = t % NB, l = t / NB;
-		M[c][l] = c < nc ? Fb[cofs[l] + jb + c] : 0.0;
+		const double d = rs[tid];
+		rs[tid] = sqrt(d) / d; // 1 / l_cc
 	}
 	__syncthreads();
-	const long long i = (long long)jb + (long long)blockIdx.x * TRSM_ROWS + threadIdx.x;
-	if (i >= f.m) return;
-	double x[NB];
-#pragma unroll
-	for (int l = 0; l < NB; ++l) x[l] = Fb[cofs[l] + i];
-	long long cb = pk(f.m, jb) + i; // entry (i, jb + c)
-	for (int c = 0; c < nc; ++c)
-	{
-		if (i < jb + c) break; // upper part of B's block
-		double a = 0.0;
-#pragma unroll
-		for (int l = 0; l < NB; ++l) a = fma(x[l], M[c][l], a);
-		Fb[cb] -= a;
-		cb += f.m - (jb + c) - 1;
-	}
-}
-
-// trailing lower triangle -= P P^T for the pair's rows P below it (up to 64 columns),
-// 64 x 64 tiles of the lower triangle, the two 64 x 64 row blocks of P in shared
-// memory, 4 x 4 entries per thread
-constexpr size_t SYRK64_SMEM = 2 * NBF * (TILE + 1) * sizeof(double);
-__global__ void __launch_bounds__(256, 3) k_dir_syrk64(const DevFront *__restrict__ fr, const int *__restrict__ list,
-													double *__restrict__ F, int j0)
-{
-	const DevFront f = fr[list[blockIdx.y]];
-	if (j0 >= f.k) return;
-	const int nb = min(NBF, f.k - j0);
-	const int o = j0 + nb, t = f.m - o;
-	if (t <= 0) return;
-	const long long nt = (t + TILE - 1) / TILE;
-	const long long tile = blockIdx.x;
-	if (tile >= nt * (nt + 1) / 2) return;
-	long long ti = (long long)((sqrt(8.0 * (double)tile + 1.0) - 1.0) * 0.5);
-	while (ti * (ti + 1) / 2 > tile) --ti;
-	while ((ti + 1) * (ti + 2) / 2 <= tile) ++ti;
-	const long long tj = tile - ti * (ti + 1) / 2;
-	extern __shared__ __align__(16) double sy[];
-	double(*Pi)[TILE + 1] = reinterpret_cast<double(*)[TILE + 1]>(sy);
-	double(*Pj)[TILE + 1] = reinterpret_cast<double(*)[TILE + 1]>(sy + NBF * (TILE + 1));
-	double *Fb = F + f.foff;
-	__shared__ long long cofs[NBF]; // pk of columns j0 + l
-	if (threadIdx.x < NBF) cofs[threadIdx.x] = pk(f.m, j0 + threadIdx.x);
-	__syncthreads();
-	// all of a thread's staging loads are issued before any is stored
-	constexpr int SQ = NBF * TILE / 256;
-	double vi[SQ], vj[SQ];
-	const int r = threadIdx.x % TILE, l0 = threadIdx.x / TILE;
-	const long long gi = ti * TILE + r, gj = tj * TILE + r;
-#pragma unroll
-	for (int q = 0; q < SQ; ++q)
-	{
-		const int l = l0 + q * (256 / TILE);
-		const bool ok = l < nb;
-		vi[q] = ok && gi < t ? Fb[cofs[l] + o + gi] : 0.0;
-		vj[q] = ok && gj < t ? Fb[cofs[l] + o + gj] : 0.0;
-	}
-#pragma unroll
-	for (int q = 0; q < SQ; ++q)
-	{
-		const int l = l0 + q * (256 / TILE);
-		Pi[l][r] = vi[q];
-		Pj[l][r] = vj[q];
-	}
-	__syncthreads();
-	const int tr = (threadIdx.x % 16) * 4, tc = (threadIdx.x / 16) * 4;
-	double acc[4][4] = {};
 #pragma unroll 4
-	for (int l = 0; l < NBF; ++l)
+	for (int i = 0; i < 16; ++i)
+	{
+		const int l = 4 * i + g;
+		M[r][l] *= rs[l]; // above the diagonal: never read
+	}
+	__syncthreads();
+	if (lane < 8)
+	{
+		// inverse of the warp's 8 x 8 diagonal triangle, a column per lane
+		const int h = 8 * warp;
+		double x[8];
+#pragma unroll
+		for (int i = 0; i < 8; ++i) x[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+		for (int i = 0; i < 8; ++i)
+		{
+			x[i] *= rs[h + i];
+#pragma unroll
+			for (int l = i + 1; l < 8; ++l) x[l] = fma(-M[h + l][h + i], x[i], x[l]);
+		}
+#pragma unroll
+		for (int i = 0; i < 8; ++i) V[h + i][h + lane] = x[i];
+	}
+#pragma unroll 1
+	for (int w = 8; w < NBF; w *= 2)
+	{
+		const int tw = w / 8, tiles = NBF / (2 * w) * tw * tw; // 8 x 8 tiles of all pairs of w x w blocks
+		__syncthreads();
+		for (int x = warp; x < tiles; x += 8) // B A^-1 into the block above the diagonal
+		{
+			const int h = x / (tw * tw) * 2 * w, i = h + w + 8 * (x / tw % tw), j = h + 8 * (x % tw);
+			double c[2] = {};
+			for (int k = 0; k < w; k += 4) dmma_8x8(c, M[i + fr_][h + k + fk], V[h + k + fk][j + fr_]);
+			*reinterpret_cast<double2 *>(&M[i - w + fr_][j + w + 2 * fk]) = make_double2(c[0], c[1]);
+		}
+		__syncthreads();
+		for (int x = warp; x < tiles; x += 8) // -C^-1 (B A^-1)
+		{
+			const int h = x / (tw * tw) * 2 * w, i = h + w + 8 * (x / tw % tw), j = h + 8 * (x % tw);
+			double c[2] = {};
+			for (int k = 0; k < w; k += 4) dmma_8x8(c, -V[i + fr_][h + w + k + fk], M[h + k + fk][j + w + fr_]);
+			*reinterpret_cast<double2 *>(&V[i + fr_][j + 2 * fk]) = make_double2(c[0], c[1]);
+		}
+	}
+	__syncthreads();
+#pragma unroll 4
+	for (int i = 0; i < 16; ++i)
+	{
+		const int l = 4 * i + g;
+		if (r < nb && l <= r) Fb[l * ld - l * (l + 1) / 2 + r] = V[r][l];
+	}
+}
+
+// 64 rows below the panel per CTA on the FP64 tensor pipe, K = 64 staged at once:
+//   INV: X = B V^T in place, V the inverse k_dir_diag left in the diagonal block;
+//   else the panel's update of the next panel's columns, C -= P Q^T with Q the rows of P
+//   that belong to those columns (rows and columns from j0 + 64 on).
+// Bound by latency: one wave of CTAs that load, multiply and store once.  A thread-per-row
+// substitution took 14.7 us and a thread-per-row update 22 us for 32 columns at P2 24^3;
+// these take 6 and 8 us for 64 on the last front (7,056 rows).
+constexpr int ROWS_LD = NBF + 4; // 4 mod 16: the four k rows of a fragment fall on distinct banks
+constexpr size_t ROWS_SMEM = 2 * NBF * ROWS_LD * sizeof(double);
+template <bool INV>
+__global__ void __launch_bounds__(128, 3) k_dir_rows(const DevFront *__restrict__ fr, const int *__restrict__ list,
+													 double *__restrict__ F, int j0)
+{
+	const DevFront f = fr[list[blockIdx.y]];
+	if (f.k <= (INV ? j0 : j0 + NBF)) return;
+	const int nb = min(NBF, f.k - j0), o = j0 + nb, i0 = blockIdx.x * ROWS_TILE, t = f.m - o;
+	if (i0 >= t) return;
+	// column l of the panel from row o on: P + l ld - l (l + 1) / 2
+	double *P = F + f.foff + pk(f.m, j0) + o;
+	const int ld = f.m - j0;
+	const int nc = INV ? nb : min(NBF, f.k - o); // columns of the result
+	extern __shared__ __align__(16) double dsm[];
+	double(*A)[ROWS_LD] = reinterpret_cast<double(*)[ROWS_LD]>(dsm);
+	double(*B)[ROWS_LD] = reinterpret_cast<double(*)[ROWS_LD]>(dsm + NBF * ROWS_LD);
+	const int tid = threadIdx.x, r = tid % NBF, l1 = tid / NBF;
+	{
+		int off = l1 * ld - l1; // l1 is 0 or 1
+		int step = 2 * ld - 2 * l1 - 3;
+		const bool ra = i0 + r < t;
+#pragma unroll 8
+		for (int q = 0; q < NBF / 2; ++q)
+		{
+			const int l = l1 + 2 * q;
+			const bool oa = l < nb && ra, ob = l < nb && (INV ? r >= l && r < nb : r < nc);
+			cp_async8(&A[l][r], P + (oa ? off + i0 + r : 0), oa);
+			cp_async8(&B[l][r], P + (ob ? off + (INV ? r - nb : r) : 0), ob); // INV: B[l][c] = V(c, l)
+			off += step;
+			step -= 4;
+		}
+	}
+	cp_async_commit();
+	const int lane = tid & 31, warp = tid >> 5, wr = (warp & 1) * 32, wc = (warp >> 1) * 32;
+	const int fk = lane & 3, fr_ = lane >> 2;
+	// the result: INV overwrites the panel's columns, else columns o .. of the front
+	double *C = INV ? P + i0 : F + f.foff + pk(f.m, o) + o + i0;
+	const int ldc = INV ? ld : t;
+	double acc[4][4][2];
+#pragma unroll
+	for (int q = 0; q < 4; ++q)
+#pragma unroll
+		for (int e = 0; e < 2; ++e)
+		{
+			const int c = wc + 8 * q + 2 * fk + e;
+			const double *src = C + (c * ldc - c * (c + 1) / 2);
+#pragma unroll
+			for (int p = 0; p < 4; ++p)
+			{
+				const int i = wr + 8 * p + fr_;
+				acc[p][q][e] = !INV && c < nc && i0 + i < t && i0 + i >= c ? -src[i] : 0.0;
+			}
+		}
+	cp_async_wait<0>();
+	__syncthreads();
+	const int ke = INV ? wc + 32 : NBF; // the inverse is lower triangular: column c needs l <= c
+#pragma unroll 4
+	for (int k = 0; k < ke; k += 4)
 	{
 		double a[4], b[4];
 #pragma unroll
 		for (int q = 0; q < 4; ++q)
 		{
-			a[q] = Pi[l][tr + q];
-			b[q] = Pj[l][tc + q];
+			a[q] = A[k + fk][wr + 8 * q + fr_];
+			b[q] = B[k + fk][wc + 8 * q + fr_];
 		}
 #pragma unroll
-		for (int p = 0; p < 4; ++p)
+		for (int p = 0; p < 4; p += 2)
 #pragma unroll
-			for (int q = 0; q < 4; ++q) acc[p][q] = fma(a[p], b[q], acc[p][q]);
+			for (int q = 0; q < 4; ++q) dmma(acc[p][q], acc[p + 1][q], a[p], a[p + 1], b[q]);
 	}
-	long long cb = pk(f.m, (int)(o + tj * TILE + tc)) + o + ti * TILE + tr; // entry (o + gr, o + gc) at p = q = 0
 #pragma unroll
 	for (int q = 0; q < 4; ++q)
-	{
-		const long long gc = tj * TILE + tc + q;
 #pragma unroll
-		for (int p = 0; p < 4; ++p)
+		for (int e = 0; e < 2; ++e)
 		{
-			const long long gr = ti * TILE + tr + p;
-			if (gr < t && gc < t && gr >= gc) Fb[cb + p] -= acc[p][q];
+			const int c = wc + 8 * q + 2 * fk + e;
+			double *dst = C + (c * ldc - c * (c + 1) / 2);
+#pragma unroll
+			for (int p = 0; p < 4; ++p)
+			{
+				const int i = wr + 8 * p + fr_;
+				if (c < nc && i0 + i < t && (INV || i0 + i >= c)) dst[i] = INV ? acc[p][q][e] : -acc[p][q][e];
+			}
 		}
-		cb += f.m - (o + gc) - 1;
+}
+
+// Trailing lower triangle C -= P P^T, P the rows below of up to 128 panel columns from
+// j0.  128 x 64 tiles, four warps of 64 x 32 on the FP64 tensor pipe; the accumulators
+// start from -C, so its loads overlap the first panel chunks, which arrive through a
+// four-deep cp.async ring of 8 columns (8-byte copies: packed columns have no 16-byte
+// alignment) addressed by running 32-bit offsets.
+// Bound by the FP64 pipe: 29 of 37 TFLOP/s on fronts of order 10,512 (P2 24^3), where
+// 64 x 64 tiles of 4 x 4 multiply-adds per thread reached 9.  Two CTAs per SM instead of
+// three: +6%; 16 columns per ring stage: +1%; m16n8k4 steps: +3% of the factorisation.
+constexpr int UT_M = 128, UT_N = 64, UT_K = 8, UT_ST = 4;
+constexpr int UT_LA = UT_M + 4, UT_LB = UT_N + 4; // 4 mod 16, as above
+static_assert(UT_K == 8, "one m16n8k8 step per ring stage");
+constexpr size_t UPDATE_SMEM = (size_t)UT_ST * UT_K * (UT_LA + UT_LB) * sizeof(double);
+__global__ void __launch_bounds__(128, 3) k_dir_update(const DevFront *__restrict__ fr, const int *__restrict__ list,
+													   double *__restrict__ F, int j0)
+{
+	const DevFront f = fr[list[blockIdx.y]];
+	if (f.k <= j0) return;
+	const int K = min(2 * NBF, f.k - j0);
+	const int o = j0 + K, t = f.m - o; // rows and columns o .. m-1, counted from 0 below
+	int c0, r0;
+	{
+		// column block q from the last has ceil((q + 1) / 2) tiles of 128 rows from its
+		// diagonal on; h (h + 1) tiles lie before q = 2 h, (h + 1)^2 before q = 2 h + 1
+		const int n64 = (t + UT_N - 1) / UT_N, x = blockIdx.x;
+		int h = (int)((sqrtf(4.f * (float)x + 1.f) - 1.f) * 0.5f);
+		while ((long long)h * (h + 1) > x) --h;
+		while ((long long)(h + 1) * (h + 2) <= x) ++h;
+		const int odd = (long long)(h + 1) * (h + 1) <= x;
+		const int q = 2 * h + odd, i = x - (odd ? (h + 1) * (h + 1) : h * (h + 1));
+		if (q >= n64) return;
+		c0 = (n64 - 1 - q) * UT_N;
+		r0 = c0 + i * UT_M;
+		if (r0 >= t) return;
 	}
+	extern __shared__ __align__(16) double dsm[];
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	const int wr = (warp & 1) * 64, wc = (warp >> 1) * 32, fk = lane & 3, fr_ = lane >> 2;
+	const int nch = (K + UT_K - 1) / UT_K;
+	// staging: this thread copies row tid of A, and row tid % 64 of B in the columns of
+	// parity tid / 64; the offset of the next column, and its distance to the one after
+	const double *P = F + f.foff + pk(f.m, j0) + o;
+	const int ld = f.m - j0, l1 = tid / UT_N;
+	const bool oka = r0 + tid < t, okb = c0 + tid % UT_N < t;
+	int offa = r0 + tid, stepa = ld - 1;
+	int offb = c0 + tid % UT_N + l1 * ld - l1, stepb = 2 * ld - 2 * l1 - 3;
+	double *sA = dsm + tid, *sB = dsm + UT_ST * UT_K * UT_LA + l1 * UT_LB + tid % UT_N;
+	const auto stage = [&](int ch) {
+		const int s = (ch % UT_ST) * UT_K, left = K - ch * UT_K;
+#pragma unroll
+		for (int q = 0; q < UT_K; ++q)
+		{
+			const bool ok = oka && q < left;
+			cp_async8(sA + (s + q) * UT_LA, P + (ok ? offa : 0), ok);
+			offa += stepa;
+			--stepa;
+		}
+#pragma unroll
+		for (int q = 0; q < UT_K; q += 2)
+		{
+			const bool ok = okb && q + l1 < left;
+			cp_async8(sB + (s + q) * UT_LB, P + (ok ? offb : 0), ok);
+			offb += stepb;
+			stepb -= 4;
+		}
+	};
+#pragma unroll
+	for (int ch = 0; ch < UT_ST - 1; ++ch)
+	{
+		if (ch < nch) stage(ch);
+		cp_async_commit();
+	}
+	double *C = F + f.foff + o + r0 + wr + fr_;
+	double acc[8][4][2];
+#pragma unroll
+	for (int q = 0; q < 4; ++q)
+#pragma unroll
+		for (int e = 0; e < 2; ++e)
+		{
+			const int c = c0 + wc + 8 * q + 2 * fk + e, i0 = r0 + wr + fr_;
+			const double *src = C + pk(f.m, o + min(c, t - 1));
+#pragma unroll
+			for (int p = 0; p < 8; ++p) acc[p][q][e] = i0 + 8 * p < t && i0 + 8 * p >= c ? -src[8 * p] : 0.0;
+		}
+	const double *fA = dsm + fk * UT_LA + wr + fr_, *fB = dsm + UT_ST * UT_K * UT_LA + fk * UT_LB + wc + fr_;
+#pragma unroll 1
+	for (int ch = 0; ch < nch; ++ch)
+	{
+		cp_async_wait<UT_ST - 2>();
+		__syncthreads();
+		if (ch + UT_ST - 1 < nch) stage(ch + UT_ST - 1);
+		cp_async_commit();
+		const double *cA = fA + (ch % UT_ST) * UT_K * UT_LA, *cB = fB + (ch % UT_ST) * UT_K * UT_LB;
+		double b[4][2];
+#pragma unroll
+		for (int q = 0; q < 4; ++q)
+		{
+			b[q][0] = cB[8 * q];
+			b[q][1] = cB[4 * UT_LB + 8 * q];
+		}
+#pragma unroll
+		for (int p = 0; p < 8; p += 2)
+		{
+			const double a[4] = {cA[8 * p], cA[8 * p + 8], cA[4 * UT_LA + 8 * p], cA[4 * UT_LA + 8 * p + 8]};
+#pragma unroll
+			for (int q = 0; q < 4; ++q) dmma_k8(acc[p][q], acc[p + 1][q], a, b[q][0], b[q][1]);
+		}
+	}
+#pragma unroll
+	for (int q = 0; q < 4; ++q)
+#pragma unroll
+		for (int e = 0; e < 2; ++e)
+		{
+			const int c = c0 + wc + 8 * q + 2 * fk + e, i0 = r0 + wr + fr_;
+			double *dst = C + pk(f.m, o + min(c, t - 1));
+#pragma unroll
+			for (int p = 0; p < 8; ++p)
+				if (i0 + 8 * p < t && i0 + 8 * p >= c) dst[8 * p] = -acc[p][q][e];
+		}
 }
 
 __global__ void k_dir_permute_in(int n, const int *__restrict__ perm, const double *__restrict__ b, double *__restrict__ bp)
@@ -1047,10 +1210,12 @@ __global__ void k_dir_permute_out(int n, const int *__restrict__ perm, const dou
 }
 
 // Forward substitution, level by level from the leaves, in the factorisation's
-// 32-column panels.  k_fwd_init: w = [b_cols; 0] plus the children's update
-// vectors (one CTA per front, children in order); per panel, k_fwd_diag (one warp
-// per front) solves the diagonal block in registers and k_fwd_rows updates the
-// rows below it (a thread per row, several CTAs per front, coalesced columns of L).
+// 64-column panels.  k_fwd_init: w = [b_cols; 0] plus the children's update vectors
+// (one CTA per front, children in order); k_fwd_step, one launch per panel: every CTA
+// multiplies the panel's right-hand side by the diagonal block's inverse (y, written to
+// Y once) and updates its own 64 rows below.  The loads of its 64 x 64 block of L are
+// issued before y is known.  Two launches per 32-column panel with a substitution in
+// one warp took 28 us each panel at P2 24^3.
 __global__ void __launch_bounds__(256) k_fwd_init(const DevFront *__restrict__ fr, const int *__restrict__ list,
 												  const int *__restrict__ child, const int *__restrict__ relpos,
 												  const double *__restrict__ bp, double *__restrict__ W)
@@ -1070,47 +1235,48 @@ __global__ void __launch_bounds__(256) k_fwd_init(const DevFront *__restrict__ f
 	}
 }
 
-__global__ void __launch_bounds__(32) k_fwd_diag(const DevFront *__restrict__ fr, const int *__restrict__ list,
-												 const double *__restrict__ F, double *__restrict__ W, int j0)
-{
-	const DevFront f = fr[list[blockIdx.x]];
-	if (j0 >= f.k) return;
-	const int nb = min(NB, f.k - j0), lane = threadIdx.x;
-	double *w = W + f.woff;
-	const double *L = F + f.foff;
-	double v = lane < nb ? w[j0 + lane] : 0.0;
-	long long cb = pk(f.m, j0) + j0; // column j0 + c, row j0
-	for (int c = 0; c < nb; ++c)
-	{
-		const double yc = __shfl_sync(0xffffffffu, v, c) / L[cb + c];
-		if (lane == c) v = yc;
-		if (lane > c && lane < nb) v = fma(-L[cb + lane], yc, v);
-		cb += f.m - (j0 + c) - 1;
-	}
-	if (lane < nb) w[j0 + lane] = v;
-}
-
-__global__ void __launch_bounds__(FWD_ROWS) k_fwd_rows(const DevFront *__restrict__ fr, const int *__restrict__ list,
-													   const double *__restrict__ F, double *__restrict__ W, int j0)
+__global__ void __launch_bounds__(256) k_fwd_step(const DevFront *__restrict__ fr, const int *__restrict__ list,
+												  const double *__restrict__ F, double *__restrict__ W,
+												  double *__restrict__ Y, int j0)
 {
 	const DevFront f = fr[list[blockIdx.y]];
 	if (j0 >= f.k) return;
-	const int nb = min(NB, f.k - j0);
+	const int nb = min(NBF, f.k - j0), i0 = j0 + nb + blockIdx.x * ROWS_TILE;
+	if (blockIdx.x && i0 >= f.m) return;
+	const int r = threadIdx.x % NBF, g = threadIdx.x / NBF; // a row, columns 16 g .. 16 g + 15
 	double *w = W + f.woff;
 	const double *L = F + f.foff;
-	__shared__ double yb[NB];
-	if (threadIdx.x < nb) yb[threadIdx.x] = w[j0 + threadIdx.x];
-	__syncthreads();
-	const long long i = (long long)j0 + nb + (long long)blockIdx.x * FWD_ROWS + threadIdx.x;
-	if (i >= f.m) return;
-	double a = w[i];
-	long long cb = pk(f.m, j0) + i;
-	for (int c = 0; c < nb; ++c)
+	__shared__ double wb[NBF], y[NBF], part[4][NBF];
+	if (g == 0) wb[r] = r < nb ? w[j0 + r] : 0.0;
+	const bool row = i0 + r < f.m;
+	double v[16], b[16];
+#pragma unroll
+	for (int q = 0; q < 16; ++q)
 	{
-		a = fma(-L[cb], yb[c], a);
-		cb += f.m - (j0 + c) - 1;
+		const int c = 16 * g + q;
+		const double *Lc = L + pk(f.m, j0 + min(c, nb - 1));
+		v[q] = c < nb && r >= c && r < nb ? Lc[j0 + r] : 0.0;
+		b[q] = c < nb && row ? Lc[i0 + r] : 0.0;
 	}
-	w[i] = a;
+	__syncthreads();
+	double s = 0.0;
+#pragma unroll
+	for (int q = 0; q < 16; ++q) s = fma(v[q], wb[16 * g + q], s);
+	part[g][r] = s;
+	__syncthreads();
+	if (g == 0)
+	{
+		const double yr = (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
+		y[r] = yr;
+		if (blockIdx.x == 0 && r < nb) Y[f.col0 + j0 + r] = yr;
+	}
+	__syncthreads();
+	s = 0.0;
+#pragma unroll
+	for (int q = 0; q < 16; ++q) s = fma(b[q], y[16 * g + q], s);
+	part[g][r] = s;
+	__syncthreads();
+	if (g == 0 && row) w[i0 + r] -= (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
 }
 
 __device__ __forceinline__ double warp_sum_d(double v)
@@ -1120,13 +1286,12 @@ __device__ __forceinline__ double warp_sum_d(double v)
 	return v;
 }
 
-// Backward substitution, level by level from the root.  k_bwd_gather: w2 = the
-// rows' solution (ancestors, already solved); k_bwd_l21: w1 -= L21^T w2 (a warp
-// per column); per panel from the last, k_bwd_cols sums L[i][j] x_i over the
-// solved columns i below the panel in row chunks of BWD_ROWS (one partial per
-// chunk and column) and k_bwd_diag (one warp per front) adds the partials in chunk
-// order and solves the transposed diagonal block in registers; k_bwd_store writes
-// x1.
+// Backward substitution, level by level from the root.  k_bwd_gather: w2 = the rows'
+// solution (ancestors, already solved); k_bwd_l21: w1 = y - L21^T w2 (a warp per
+// column); k_bwd_step, one launch per panel from the last: every CTA multiplies the
+// panel's w1 by the transposed inverse of the diagonal block (x, written to X once) and
+// subtracts the panel's rows times x from its own 64 earlier columns, a warp per
+// column, the loads issued before x is known.
 __global__ void __launch_bounds__(256) k_bwd_gather(const DevFront *__restrict__ fr, const int *__restrict__ list,
 													const int *__restrict__ rows, const double *__restrict__ X,
 													double *__restrict__ W)
@@ -1138,7 +1303,8 @@ __global__ void __launch_bounds__(256) k_bwd_gather(const DevFront *__restrict__
 }
 
 __global__ void __launch_bounds__(256) k_bwd_l21(const DevFront *__restrict__ fr, const int *__restrict__ list,
-												 const double *__restrict__ F, double *__restrict__ W)
+												 const double *__restrict__ F, const double *__restrict__ Y,
+												 double *__restrict__ W)
 {
 	const DevFront f = fr[list[blockIdx.y]];
 	const int j = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -1147,71 +1313,58 @@ __global__ void __launch_bounds__(256) k_bwd_l21(const DevFront *__restrict__ fr
 	const int r = f.m - f.k;
 	const double *Lj = F + f.foff + pk(f.m, j) + f.k;
 	double s = 0.0;
+#pragma unroll 4
 	for (int i = lane; i < r; i += 32) s = fma(Lj[i], w[f.k + i], s);
 	s = warp_sum_d(s);
-	if (lane == 0) w[j] -= s;
+	if (lane == 0) w[j] = Y[f.col0 + j] - s;
 }
 
-__global__ void __launch_bounds__(256) k_bwd_cols(const DevFront *__restrict__ fr, const int *__restrict__ list,
-												  const double *__restrict__ F, const double *__restrict__ W,
-												  double *__restrict__ part, int j0)
+__global__ void __launch_bounds__(256) k_bwd_step(const DevFront *__restrict__ fr, const int *__restrict__ list,
+												  const double *__restrict__ F, double *__restrict__ W,
+												  double *__restrict__ X, int j0)
 {
 	const DevFront f = fr[list[blockIdx.y]];
 	if (j0 >= f.k) return;
-	const int nb = min(NB, f.k - j0), e = j0 + nb;
-	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-	const double *w = W + f.woff;
-	const double *L = F + f.foff;
-	const int i0 = e + blockIdx.x * BWD_ROWS, i1 = min(f.k, i0 + BWD_ROWS);
-	double *pp = part + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * NB;
-	for (int c = warp; c < NB; c += 8)
-	{
-		double s = 0.0;
-		if (c < nb)
-		{
-			const double *Lc = L + pk(f.m, j0 + c);
-			for (int i = i0 + lane; i < i1; i += 32) s = fma(Lc[i], w[i], s);
-		}
-		s = warp_sum_d(s);
-		if (lane == 0) pp[c] = s;
-	}
-}
-
-__global__ void __launch_bounds__(32) k_bwd_diag(const DevFront *__restrict__ fr, const int *__restrict__ list,
-												 const double *__restrict__ F, double *__restrict__ W,
-												 const double *__restrict__ part, int nchunk, int j0)
-{
-	const DevFront f = fr[list[blockIdx.x]];
-	if (j0 >= f.k) return;
-	const int nb = min(NB, f.k - j0), lane = threadIdx.x;
+	const int nb = min(NBF, f.k - j0), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	const int c0 = blockIdx.x * NBF + warp * 8; // this warp's eight earlier columns
+	if (blockIdx.x && blockIdx.x * NBF >= j0) return;
 	double *w = W + f.woff;
 	const double *L = F + f.foff;
-	double v = 0.0;
-	if (lane < nb)
+	__shared__ double x[NBF];
+	const bool lo = lane < nb, hi = lane + 32 < nb;
+	double b[8][2], v[8][2];
+#pragma unroll
+	for (int q = 0; q < 8; ++q)
 	{
-		const double *pp = part + (size_t)blockIdx.x * nchunk * NB + lane;
-		double s = 0.0;
-		for (int q = 0; q < nchunk; ++q) s += pp[(size_t)q * NB];
-		v = w[j0 + lane] - s;
+		const int l = warp * 8 + q; // column of the diagonal block
+		const double *Lv = L + pk(f.m, j0 + min(l, nb - 1)) + j0;
+		v[q][0] = l < nb && lo && lane >= l ? Lv[lane] : 0.0;
+		v[q][1] = l < nb && hi && lane + 32 >= l ? Lv[lane + 32] : 0.0;
+		const bool on = c0 + q < j0;
+		const double *Lc = L + pk(f.m, on ? c0 + q : 0) + j0;
+		b[q][0] = on && lo ? Lc[lane] : 0.0;
+		b[q][1] = on && hi ? Lc[lane + 32] : 0.0;
 	}
-	for (int c = nb - 1; c >= 0; --c)
+	const double w0 = lo ? w[j0 + lane] : 0.0, w1 = hi ? w[j0 + lane + 32] : 0.0;
+#pragma unroll
+	for (int q = 0; q < 8; ++q)
 	{
-		// x_c = (v_c - sum_{c' > c} L[c'][c] x_c') / L[c][c]; lanes c' > c hold x_c'
-		const double *Lc = L + pk(f.m, j0 + c) + j0;
-		const double t = lane > c && lane < nb ? Lc[lane] * v : 0.0;
-		const double sum = warp_sum_d(t);
-		const double xc = (__shfl_sync(0xffffffffu, v, c) - sum) / Lc[c];
-		if (lane == c) v = xc;
+		const double s = warp_sum_d(fma(v[q][0], w0, v[q][1] * w1));
+		if (lane == 0) x[warp * 8 + q] = s;
 	}
-	if (lane < nb) w[j0 + lane] = v;
-}
-
-__global__ void __launch_bounds__(256) k_bwd_store(const DevFront *__restrict__ fr, const int *__restrict__ list,
-												   const double *__restrict__ W, double *__restrict__ X)
-{
-	const DevFront f = fr[list[blockIdx.x]];
-	const double *w = W + f.woff;
-	for (int j = threadIdx.x; j < f.k; j += 256) X[f.col0 + j] = w[j];
+	__syncthreads();
+	const double x0 = x[lane], x1 = x[lane + 32];
+	if (blockIdx.x == 0 && warp == 0)
+	{
+		if (lo) X[f.col0 + j0 + lane] = x0;
+		if (hi) X[f.col0 + j0 + lane + 32] = x1;
+	}
+#pragma unroll
+	for (int q = 0; q < 8; ++q)
+	{
+		const double s = warp_sum_d(fma(b[q][0], x0, b[q][1] * x1));
+		if (lane == 0 && c0 + q < j0) w[c0 + q] -= s;
+	}
 }
 
 } // namespace
@@ -1224,8 +1377,11 @@ int direct_factorize(DirectFactor *f, const double *vals, cudaStream_t s, cudaEr
 	f->factorized = false;
 	const int nl = (int)f->lvl_start.size() - 1;
 	if ((*ce = cudaMemsetAsync(f->d_err, 0, sizeof(int), s)) != cudaSuccess) return 2;
-	if ((*ce = cudaFuncSetAttribute(k_dir_syrk64, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SYRK64_SMEM)) !=
-		cudaSuccess)
+	const auto smem = [&](const void *k, size_t bytes) {
+		return (*ce = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)) == cudaSuccess;
+	};
+	if (!smem((const void *)k_dir_diag, DIAG_SMEM) || !smem((const void *)k_dir_rows<true>, ROWS_SMEM) ||
+		!smem((const void *)k_dir_rows<false>, ROWS_SMEM) || !smem((const void *)k_dir_update, UPDATE_SMEM))
 		return 2;
 	size_t pi = 0;
 	for (int h = 0; h < nl; ++h)
@@ -1242,22 +1398,18 @@ int direct_factorize(DirectFactor *f, const double *vals, cudaStream_t s, cudaEr
 			if (f->lvl_maxrc[h] > 0)
 				k_dir_extend_add<<<dim3((f->lvl_maxrc[h] + 7) / 8, nf), 256, 0, s>>>(f->d_fr, list, f->d_child,
 																					 f->d_relpos, f->d_front, ci);
-		for (; pi < f->fpanels.size() && f->fpanels[pi].lvl == h; ++pi)
+		for (; pi < f->panels.size() && f->panels[pi].lvl == h; ++pi)
 		{
-			const Panel &p = f->fpanels[pi];
-			// panel A
-			k_dir_potrf<<<nf, 32, 0, s>>>(f->d_fr, list, f->d_front, p.j0, f->d_err);
-			if (p.rows_grid > 0) k_dir_trsm<<<dim3(p.rows_grid, nf), TRSM_ROWS, 0, s>>>(f->d_fr, list, f->d_front, p.j0);
-			// A's update of B, then panel B
-			if (p.fwd_grid > 0)
-			{
-				k_dir_panel_update<<<dim3(p.fwd_grid, nf), TRSM_ROWS, 0, s>>>(f->d_fr, list, f->d_front, p.j0);
-				k_dir_potrf<<<nf, 32, 0, s>>>(f->d_fr, list, f->d_front, p.j0 + NB, f->d_err);
-				if (p.bwd_grid > 0)
-					k_dir_trsm<<<dim3(p.bwd_grid, nf), TRSM_ROWS, 0, s>>>(f->d_fr, list, f->d_front, p.j0 + NB);
-			}
-			if (p.tiles_grid > 0)
-				k_dir_syrk64<<<dim3(p.tiles_grid, nf), 256, SYRK64_SMEM, s>>>(f->d_fr, list, f->d_front, p.j0);
+			const Panel &p = f->panels[pi];
+			const bool second = (p.j0 / NBF) & 1;
+			k_dir_diag<<<nf, 256, DIAG_SMEM, s>>>(f->d_fr, list, f->d_front, p.j0, f->d_err);
+			if (p.rows_grid > 0) k_dir_rows<true><<<dim3(p.rows_grid, nf), 128, ROWS_SMEM, s>>>(f->d_fr, list, f->d_front, p.j0);
+			if (!second && p.upd_grid > 0)
+				k_dir_rows<false><<<dim3(p.upd_grid, nf), 128, ROWS_SMEM, s>>>(f->d_fr, list, f->d_front, p.j0);
+			// the pair's trailing update, after its last panel on this level
+			const Panel &p0 = second ? f->panels[pi - 1] : p;
+			if ((second || p.upd_grid == 0) && p0.tiles_grid > 0)
+				k_dir_update<<<dim3(p0.tiles_grid, nf), 128, UPDATE_SMEM, s>>>(f->d_fr, list, f->d_front, p0.j0);
 		}
 		if ((*ce = cudaGetLastError()) != cudaSuccess) return 2;
 	}
@@ -1274,7 +1426,7 @@ cudaError_t direct_solve(DirectFactor *f, const double *b, double *x, cudaStream
 {
 	const int n = f->n;
 	if (n == 0) return cudaSuccess;
-	double *bp = f->d_vec, *xp = f->d_vec + n;
+	double *bp = f->d_vec, *xp = f->d_vec + n; // bp: permuted right-hand side, then y
 	const int nl = (int)f->lvl_start.size() - 1;
 	k_dir_permute_in<<<(n + 255) / 256, 256, 0, s>>>(n, f->d_perm, b, bp);
 	size_t pi = 0;
@@ -1284,12 +1436,8 @@ cudaError_t direct_solve(DirectFactor *f, const double *b, double *x, cudaStream
 		const int *list = f->d_lvl_list + f->lvl_start[h];
 		k_fwd_init<<<nf, 256, 0, s>>>(f->d_fr, list, f->d_child, f->d_relpos, bp, f->d_work);
 		for (; pi < f->panels.size() && f->panels[pi].lvl == h; ++pi)
-		{
-			const Panel &p = f->panels[pi];
-			k_fwd_diag<<<nf, 32, 0, s>>>(f->d_fr, list, f->d_front, f->d_work, p.j0);
-			if (p.fwd_grid > 0)
-				k_fwd_rows<<<dim3(p.fwd_grid, nf), FWD_ROWS, 0, s>>>(f->d_fr, list, f->d_front, f->d_work, p.j0);
-		}
+			k_fwd_step<<<dim3(std::max(f->panels[pi].rows_grid, 1), nf), 256, 0, s>>>(f->d_fr, list, f->d_front, f->d_work, bp,
+																					  f->panels[pi].j0);
 	}
 	for (int h = nl - 1; h >= 0; --h)
 	{
@@ -1297,19 +1445,12 @@ cudaError_t direct_solve(DirectFactor *f, const double *b, double *x, cudaStream
 		const int *list = f->d_lvl_list + f->lvl_start[h];
 		k_bwd_gather<<<nf, 256, 0, s>>>(f->d_fr, list, f->d_rows, xp, f->d_work);
 		if (f->lvl_maxk[h] > 0)
-			k_bwd_l21<<<dim3((f->lvl_maxk[h] + 7) / 8, nf), 256, 0, s>>>(f->d_fr, list, f->d_front, f->d_work);
-		// this level's panels, last first
-		size_t p1 = 0;
-		while (p1 < f->panels.size() && f->panels[p1].lvl < h) ++p1;
-		size_t p2 = p1;
-		while (p2 < f->panels.size() && f->panels[p2].lvl == h) ++p2;
-		for (size_t q = p2; q > p1; --q)
+			k_bwd_l21<<<dim3((f->lvl_maxk[h] + 7) / 8, nf), 256, 0, s>>>(f->d_fr, list, f->d_front, bp, f->d_work);
+		for (; pi > 0 && f->panels[pi - 1].lvl == h; --pi) // this level's panels, last first
 		{
-			const Panel &p = f->panels[q - 1];
-			k_bwd_cols<<<dim3(p.bwd_grid, nf), 256, 0, s>>>(f->d_fr, list, f->d_front, f->d_work, f->d_part, p.j0);
-			k_bwd_diag<<<nf, 32, 0, s>>>(f->d_fr, list, f->d_front, f->d_work, f->d_part, p.bwd_grid, p.j0);
+			const int j0 = f->panels[pi - 1].j0;
+			k_bwd_step<<<dim3(std::max((j0 + NBF - 1) / NBF, 1), nf), 256, 0, s>>>(f->d_fr, list, f->d_front, f->d_work, xp, j0);
 		}
-		k_bwd_store<<<nf, 256, 0, s>>>(f->d_fr, list, f->d_work, xp);
 	}
 	k_dir_permute_out<<<(n + 255) / 256, 256, 0, s>>>(n, f->d_perm, xp, x);
 	return cudaGetLastError();

@@ -190,3 +190,32 @@ def test_position_ordering_on_shuffled_and_flat_meshes(require_gpu, et, g):
         scale = abs(H).sum(axis=1).max() * np.abs(x).max()  # normwise backward error
         assert np.abs(b - H @ x).max() <= 1e-13 * scale
         asm.close()
+
+
+@pytest.mark.parametrize("et,g,n", [(M.P1_TET, 2, n) for n in (1, 7, 8, 9, 31, 32, 33, 63, 64, 65, 81)]
+                         + [(M.Q1_HEX, 8, n) for n in (1900, 2100, 2187)] + [(M.P2_TET, 4, n) for n in (2049, 2187)])
+def test_front_sizes_around_the_panel_edges(require_gpu, et, g, n):
+    """Free dofs chosen at random give fronts whose column counts fall on and beside the
+    edges of the 8-column, 64-column and 128-column steps (the 81-dof meshes are one
+    front).  Normwise backward error of the solve at rounding level."""
+    mesh, lam, mu, u, _ = make_case(et, g, seed=6)
+    asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
+    rng = np.random.default_rng(n)
+    asm.set_dirichlet(np.sort(rng.permutation(mesh.n_dofs)[: mesh.n_dofs - n]))
+    asm.assemble_hessian_reduced(u, "fp64", project_to_psd=True)
+    outer, inner = asm.reduced_pattern()
+    # any symmetric positive definite values in the pattern: a random diagonally dominant matrix
+    A = sp.csc_matrix((rng.standard_normal(inner.size), inner, outer), shape=(n, n))
+    A = ((A + A.T) * 0.5).tocsc()
+    A.sort_indices()
+    A.setdiag(np.asarray(abs(A).sum(axis=0)).ravel() + rng.uniform(0.5, 2.0, n))
+    import torch
+    ds = DirectSolver(asm, "reduced")
+    ds.analyze_pattern()
+    assert np.array_equal(A.indices, inner)
+    ds.factorize(torch.tensor(A.data, device="cuda"))
+    b = rng.standard_normal(n)
+    x = ds.solve(b)
+    scale = abs(A).sum(axis=1).max() * np.abs(x).max()
+    assert np.abs(b - A @ x).max() <= 1e-13 * scale
+    asm.close()
