@@ -63,10 +63,12 @@ struct pfg_context
 	double *d_result = nullptr;
 	double *d_u = nullptr, *d_p = nullptr, *d_out = nullptr;
 	size_t out_cap = 0;
-	// conjugate gradient (pfg_cg_solve): r, z, p, q, invd, b, x (cg_n doubles each),
-	// the per-block partials and the scalars; a pinned host copy of the scalars
+	// conjugate gradient (pfg_cg_solve): seven slot vectors, four dense ones, the partials and
+	// the scalars (cg_n doubles in all); a pinned host copy of the scalars; the plans of the
+	// full and the reduced pattern (built by the first solve)
 	double *d_cg = nullptr;
 	size_t cg_n = 0;
+	CgPlan cg_plan[2];
 	// mass matrix (pfg_mass_matrix): values for host-mode calls, staged densities
 	double *d_mass = nullptr, *d_rho = nullptr;
 	// lumped diagonal for host-mode pfg_lump_matrix calls (3N doubles)
@@ -281,8 +283,8 @@ int check_kernel_flag(pfg_context *c)
 	if (v)
 	{
 		PFG_CUDA(c, cudaMemset(c->d_err, 0, sizeof(int)));
-		return fail(c, PFG_ERR_CUDA, "a tensor-core kernel gave up waiting for its MMA or bulk copy; the results of "
-									 "the calls since the last synchronisation are invalid");
+		return fail(c, PFG_ERR_CUDA, "a kernel gave up a bounded wait (an MMA, a bulk copy or a grid barrier); the results "
+									 "of the calls since the last synchronisation are invalid");
 	}
 	return PFG_OK;
 }
@@ -474,6 +476,7 @@ void free_direct(pfg_context *c)
 void free_dirichlet(pfg_context *c)
 {
 	if (c->direct_system == PFG_SYS_REDUCED) free_direct(c);
+	free_cg_plan(&c->cg_plan[PFG_SYS_REDUCED]);
 	void *rptrs[] = {c->d_old_to_new, c->d_free, c->d_red_col_start, c->d_red_outer, c->d_red_inner, c->d_red_row_off,
 					 c->d_red_values, c->d_red_groups};
 	for (void *p : rptrs)
@@ -681,6 +684,7 @@ void free_all(pfg_context *c)
 	for (void *p : rptrs)
 		if (p) cudaFree(p);
 	if (c->d_cg) cudaFree(c->d_cg);
+	for (CgPlan &p : c->cg_plan) free_cg_plan(&p);
 	free_direct(c);
 	if (c->h_cg_sc) cudaFreeHost(c->h_cg_sc);
 	if (c->d_mass) cudaFree(c->d_mass);
@@ -1478,25 +1482,30 @@ int pfg_cg_solve(pfg_context *c, int system, const double *values, const double 
 	}
 	if (n > 0 && (!b || !x)) return fail(c, PFG_ERR_INVALID, "b or x NULL");
 	DeviceGuard g(c->device);
-	const size_t nn = std::max<size_t>(n, 1);
-	if (c->cg_n < nn)
+	CgPlan &plan = c->cg_plan[system];
+	if (n > 0 && !plan.run) PFG_CUDA(c, build_cg_plan(n, ngroups, groups, outer, inner, &plan, c->stream));
+	const size_t nn = std::max<size_t>(n, 1), ns = 4 * (size_t)std::max(ngroups, 1);
+	const size_t need = 7 * ns + 4 * nn + cg_partials_doubles() + CG_NSC;
+	if (c->cg_n < need)
 	{
 		if (c->d_cg) cudaFree(c->d_cg);
 		c->d_cg = nullptr;
 		c->cg_n = 0;
-		PFG_CUDA(c, cudaMalloc(&c->d_cg, sizeof(double) * (7 * nn + cg_partials_doubles() + CG_NSC)));
-		c->cg_n = nn;
+		PFG_CUDA(c, cudaMalloc(&c->d_cg, sizeof(double) * need));
+		c->cg_n = need;
 	}
 	if (!c->h_cg_sc) PFG_CUDA(c, cudaMallocHost(&c->h_cg_sc, sizeof(double) * CG_NSC));
 	CgWork w;
-	const size_t cn = c->cg_n;
-	w.r = c->d_cg;
-	w.z = w.r + cn;
-	w.p = w.z + cn;
-	w.q = w.p + cn;
-	w.invd = w.q + cn;
-	double *db = w.invd + cn, *dx = db + cn;
-	w.part = dx + cn;
+	w.x = c->d_cg; // slots first: 32-byte aligned
+	w.r = w.x + ns;
+	w.z = w.r + ns;
+	w.p = w.z + ns;
+	w.p2 = w.p + ns;
+	w.q = w.p2 + ns;
+	w.invd = w.q + ns;
+	w.dense = w.invd + ns;
+	double *db = w.dense + 2 * nn, *dx = db + nn;
+	w.part = dx + nn;
 	w.sc = w.part + cg_partials_doubles();
 	if (mem == PFG_MEM_HOST)
 	{
@@ -1518,19 +1527,21 @@ int pfg_cg_solve(pfg_context *c, int system, const double *values, const double 
 			return PFG_OK;
 		};
 		int st;
-		PFG_CUDA(c, launch_cg_diag_inv(n, outer, inner, vals, w.invd, c->stream));
 		PFG_CUDA(c, launch_cg_start(n, ngroups, groups, outer, inner, vals, db, guess != 0, tol, dx, w, c->stream));
-		// iterations in batches of CG_BATCH; the device stops them at convergence
-		constexpr int CG_BATCH = 8;
+		// iterations in batches, stopped on the device at convergence: one launch and one
+		// read of the scalars each; a batch of the largest matrix takes about a second
+		constexpr int CG_BATCH = 256;
 		int queued = 0;
 		for (;;)
 		{
+			const int k = std::min(CG_BATCH, max_iter - queued);
+			if (k > 0) PFG_CUDA(c, launch_cg_iterations(k, plan, vals, w, c->d_err, c->stream));
+			queued += std::max(k, 0);
 			if ((st = read_scalars())) return st;
 			if (c->h_cg_sc[CG_DONE] != 0.0 || queued >= max_iter) break;
-			const int k = std::min(CG_BATCH, max_iter - queued);
-			PFG_CUDA(c, launch_cg_iterations(n, k, ngroups, groups, outer, inner, vals, dx, w, c->stream));
-			queued += k;
 		}
+		if (c->h_cg_sc[CG_DONE] == 2.0 && (st = check_kernel_flag(c))) return st;
+		PFG_CUDA(c, launch_cg_unpack(ngroups, groups, w, dx, c->stream));
 		const double rhs2 = c->h_cg_sc[CG_RHS2];
 		it = (int)c->h_cg_sc[CG_ITER];
 		if (rhs2 == 0.0)

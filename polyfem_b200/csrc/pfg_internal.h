@@ -164,8 +164,7 @@ cudaError_t tc_tables_setup(int device);
 cudaError_t launch_hessian_blocks_tc(const DevMesh &m, const double *u, float *stage, cudaStream_t s);
 size_t tc_smem_bytes(int et);
 
-// Device conjugate gradient (pfg_solve.cu).  Work vectors of n doubles (r, z, p, q,
-// invd), cg_partials_doubles() per-block partial sums and the scalars sc[CG_NSC].
+// Device conjugate gradient (pfg_solve.cu).
 enum
 {
 	CG_RZ = 0,    // r.z of the current iterate
@@ -174,14 +173,33 @@ enum
 	CG_RR = 3,    // |r|^2 of the current iterate
 	CG_RHS2 = 4,  // |b|^2
 	CG_THR = 5,   // stopping threshold on |r|^2
-	CG_DONE = 6,  // 1 once |r|^2 < threshold: every later kernel of the iteration returns at once
+	CG_DONE = 6,  // 1 once |r|^2 < threshold, 2 when a bounded wait gave up: later launches return at once
 	CG_ITER = 7,  // iterations counted as Eigen counts them (not the one that stopped)
 	CG_NSC = 8
 };
+// Vectors in slots of four doubles per column group (the group's up to three dofs, zeros
+// behind); dense: 2 n doubles of set-up scratch
 struct CgWork
 {
-	double *r = nullptr, *z = nullptr, *p = nullptr, *q = nullptr, *invd = nullptr, *part = nullptr, *sc = nullptr;
+	double *x = nullptr, *r = nullptr, *z = nullptr, *p = nullptr, *p2 = nullptr, *q = nullptr, *invd = nullptr;
+	double *dense = nullptr, *part = nullptr, *sc = nullptr;
 };
+// Static plan of a system's pattern, built once: the groups in chunks that a warp's stage
+// of k_cg holds (chunk: blob, its size, first value, values or 0 for one group too large to
+// stage; blob: descriptors and neighbour codes; big: the codes of those large groups), every
+// warp's run of chunks with its first group, and the count of grid exchanges (16 bytes)
+// followed by three arrays of 32-byte packets per CTA
+struct CgPlan
+{
+	int2 *run = nullptr;
+	int4 *chunk = nullptr, *blob = nullptr;
+	const int *big = nullptr;
+	unsigned *bar = nullptr;
+	int ctas = 0;
+	bool resident = false; // every run is at most two chunks
+};
+cudaError_t build_cg_plan(int n, int ngroups, const int *groups, const int *outer, const int *inner, CgPlan *pl, cudaStream_t s);
+void free_cg_plan(CgPlan *pl);
 size_t cg_partials_doubles();
 // invd[j] = 1 / H(j, j), or 1 where the diagonal is zero or structurally absent
 cudaError_t launch_cg_diag_inv(int n, const int *outer, const int *inner, const double *vals, double *invd,
@@ -196,12 +214,13 @@ cudaError_t launch_hessian_apply(int n_nodes, const int *outer, const int *inner
 // r = b - H x (x = 0 unless guess), p = D^-1 r; sc: r.z, |r|^2, |b|^2, the threshold
 // max(tol^2 |b|^2, smallest normal), done (|b| = 0 or |r|^2 below it), 0 iterations
 cudaError_t launch_cg_start(int n, int ngroups, const int *groups, const int *outer, const int *inner,
-							const double *vals, const double *b, bool guess, double tol, double *x, const CgWork &w,
+							const double *vals, const double *b, bool guess, double tol, const double *x, const CgWork &w,
 							cudaStream_t s);
 // `count` iterations unless done: q = H p, alpha, x += alpha p, r -= alpha q, stop
-// test, z = D^-1 r, beta, p = z + beta p, iteration count + 1
-cudaError_t launch_cg_iterations(int n, int count, int ngroups, const int *groups, const int *outer,
-								 const int *inner, const double *vals, double *x, const CgWork &w, cudaStream_t s);
+// test, z = D^-1 r, beta, p = z + beta p, iteration count + 1; *err: a wait gave up
+cudaError_t launch_cg_iterations(int count, const CgPlan &pl, const double *vals, const CgWork &w, int *err, cudaStream_t s);
+// the slots of x -> the dense x
+cudaError_t launch_cg_unpack(int ngroups, const int *groups, const CgWork &w, double *x, cudaStream_t s);
 
 // Sets the message pfg_last_error(NULL) returns on this host thread.
 void set_global_error(const std::string &msg);

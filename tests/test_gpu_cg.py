@@ -152,3 +152,50 @@ def test_argument_and_state_errors(require_gpu):
     with pytest.raises(PfgError):
         ConjugateGradient(asm, "reduced").solve(np.zeros(0))
     asm.close()
+
+
+def star_mesh(n, seed=0):
+    """P1 tetrahedra from one centre node to the triangles of a sphere's hull: the centre
+    neighbours every node."""
+    from scipy.spatial import ConvexHull
+    rng = np.random.default_rng(seed)
+    pts = rng.standard_normal((n, 3))
+    pts /= np.linalg.norm(pts, axis=1)[:, None]
+    tri = ConvexHull(pts).simplices
+    X = np.concatenate([pts, np.zeros((1, 3))])
+    tets = np.concatenate([tri, np.full((tri.shape[0], 1), n)], axis=1)
+    e = X[tets[:, 1:]] - X[tets[:, :1]]
+    flip = np.linalg.det(e) < 0
+    tets[flip, 0], tets[flip, 1] = tets[flip, 1].copy(), tets[flip, 0].copy()
+    return tets.astype(np.int32), X
+
+
+@pytest.mark.parametrize("case", ["star-20", "star-60", "star-rest-150", "P1-mixed", "P2-mixed", "Q1-mixed", "P2-long"])
+def test_group_sizes_and_partly_fixed_nodes(require_gpu, case):
+    """Column groups of every kind the iteration distinguishes: neighbours beyond one warp
+    (star-60, P2 vertices), beyond a shared-memory stage (star-rest-150), nodes with one or two
+    free dofs (random Dirichlet dofs), and a matrix that streams in several chunks a warp
+    (P2-long).  The residual against a host product, and the oracle's iteration count."""
+    if case.startswith("star"):
+        conn, X = star_mesh(int(case.split("-")[-1]))
+        asm = NeoHookeanAssembler(M.P1_TET, conn, X, 1e5, 5e4)
+        u, n_dofs = 0.01 * np.random.default_rng(1).standard_normal(3 * X.shape[0]), 3 * X.shape[0]
+        if "rest" in case:  # its thin tetrahedra would invert under u
+            u = np.zeros(n_dofs)
+    else:
+        et = {"P1": M.P1_TET, "P2": M.P2_TET, "Q1": M.Q1_HEX}[case[:2]]
+        mesh, lam, mu, u, _ = make_case(et, 13 if case == "P2-long" else 4, seed=8)
+        asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
+        n_dofs = mesh.n_dofs
+    rng = np.random.default_rng(3)
+    asm.set_dirichlet(np.sort(rng.permutation(n_dofs)[: max(12, n_dofs // 9)]))
+    H = asm.assemble_hessian_reduced(u, "fp64", project_to_psd=True)
+    b = rng.standard_normal(H.shape[0])
+    cg = ConjugateGradient(asm, "reduced")
+    cg.set_parameters({"tolerance": 1e-10, "max_iter": 20000})
+    x = cg.solve(b)
+    assert np.linalg.norm(b - H @ x) <= 2e-10 * np.linalg.norm(b)
+    _, it_o, _ = conjugate_gradient(H.indptr, H.indices, H.data, b, 1e-10, 20000)
+    assert abs(cg.get_info()["solver_iter"] - it_o) <= max(2, it_o // 20)
+    assert np.array_equal(cg.solve(b), x)
+    asm.close()
