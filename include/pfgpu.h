@@ -151,6 +151,12 @@ int pfg_hessian(pfg_context *ctx, const double *u, int mem, int prec, int projec
  * pattern (any pfg_hessian or pfg_hessian_pattern call builds it). */
 int pfg_hessian_apply(pfg_context *ctx, const double *values, const double *p, int mem, double *q);
 
+/* q = H(u) p (3N doubles each, in `mem`) of the NeoHookean Hessian at u in FP64, without
+ * assembling it: the directional derivative of the gradient along p, summed per node in
+ * a fixed order (bitwise deterministic).  The context's matrix and pattern are neither
+ * needed nor touched.  PFG_ERR_UNSUPPORTED for other materials and compositions. */
+int pfg_hessian_vector(pfg_context *ctx, const double *u, const double *p, int mem, double *q);
+
 /* Device pointers of the context-owned CSC arrays (valid until pfg_destroy). */
 int pfg_hessian_device_csc(pfg_context *ctx, const int **outer, const int **inner, double **values);
 

@@ -226,6 +226,16 @@ class NeoHookeanAssembler:
         check(lib().pfg_hessian_apply(self._h, vptr, ptrs[0], mem, optr), self._h, "pfg_hessian_apply")
         return out
 
+    def hessian_vector(self, u, p):
+        """q = H(u) p in FP64 without assembling H (pfg_hessian_vector; NeoHookean only):
+        one element pass and a gather.  Deterministic; the context's matrix is not touched."""
+        self._check_len(u, self.n_dofs, "u")
+        self._check_len(p, self.n_dofs, "p")
+        mem, ptrs, keep = self._prepare(u, p)
+        out, optr = self._alloc(mem, self.n_dofs)
+        check(lib().pfg_hessian_vector(self._h, ptrs[0], ptrs[1], mem, optr), self._h, "pfg_hessian_vector")
+        return out
+
     def assemble_hessian_into_context(self, u, precision="fp64", project_to_psd: bool = False):
         """Assemble the Hessian into the context's own device buffer (no copy out)."""
         self._check_len(u, self.n_dofs, "u")

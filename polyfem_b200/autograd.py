@@ -10,9 +10,11 @@ backward(p) returns the vector-Jacobian products of f:
       term carries a leading minus sign (term = -p . df/d(lambda, mu));
   d(p.f)/dX                  : ElasticForceDerivative::force_shape_derivative
       (ElasticForceDerivative.cpp:207-260), which equals +p . df/dX_rest;
-  d(p.f)/du                  : H p, the assembled Hessian (structurally and
-      numerically symmetric) times p, by the library's own SpMV
-      (pfg_hessian_apply): bitwise deterministic.
+  d(p.f)/du                  : H p, bitwise deterministic.  In FP64, for NeoHookean,
+      the directional derivative of the gradient along p, without the matrix
+      (pfg_hessian_vector: 72 us at P2 32^3, where assembling and applying H takes 881); in the other modes the Hessian assembled
+      in that mode (structurally and numerically symmetric) times p
+      (pfg_hessian_apply).
 Each backward term recomputes F and the basis gradients per quadrature point
 from (u, lambda, mu, X); nothing from the forward pass is stored on the device
 beyond the four inputs.
@@ -21,6 +23,7 @@ from __future__ import annotations
 
 import torch
 
+from ._lib import PFG_FP64
 from .assembler import NeoHookeanAssembler
 
 
@@ -58,8 +61,11 @@ class ElasticForce(torch.autograd.Function):
         if ctx.needs_input_grad[3]:
             g_X = asm.force_shape_derivative(u, p, ctx.precision).reshape(X.shape)
         if ctx.needs_input_grad[0]:
-            asm.assemble_hessian_into_context(u, ctx.precision)
-            g_u = asm.hessian_apply(p)
+            if asm.material == "NeoHookean" and ctx.precision in ("fp64", PFG_FP64):
+                g_u = asm.hessian_vector(u, p)
+            else:
+                asm.assemble_hessian_into_context(u, ctx.precision)
+                g_u = asm.hessian_apply(p)
         return g_u, g_lam, g_mu, g_X, None, None
 
 

@@ -1044,12 +1044,7 @@ int pfg_set_lame(pfg_context *c, const double *lambda, const double *mu, int mem
 		PFG_CUDA(c, cudaStreamSynchronize(c->stream));
 	}
 	else
-	{
-		PFG_CUDA(c, cudaMemcpy2DAsync(c->d_lame, sizeof(double2), lambda, sizeof(double), sizeof(double), E,
-									  cudaMemcpyDeviceToDevice, c->stream));
-		PFG_CUDA(c, cudaMemcpy2DAsync((char *)c->d_lame + sizeof(double), sizeof(double2), mu, sizeof(double),
-									  sizeof(double), E, cudaMemcpyDeviceToDevice, c->stream));
-	}
+		PFG_CUDA(c, launch_pack_lame((int)E, lambda, mu, c->d_lame, c->stream));
 	return PFG_OK;
 }
 
@@ -1200,6 +1195,25 @@ int pfg_hessian_apply(pfg_context *c, const double *values, const double *p, int
 	if ((st = stage_in(c, p, mem, c->d_p, ndof, &dp))) return st;
 	double *dq = mem == PFG_MEM_DEVICE ? q : c->d_out;
 	PFG_CUDA(c, launch_hessian_apply(c->m.N, c->d_outer, c->d_inner, values ? values : c->d_values, dp, dq, c->stream));
+	if (mem == PFG_MEM_HOST) return finish_host(c, q, c->d_out, ndof);
+	return PFG_OK;
+}
+
+int pfg_hessian_vector(pfg_context *c, const double *u, const double *p, int mem, double *q)
+{
+	if (!c || !check_mem(mem) || (c->m.N && (!u || !p || !q))) return fail(c, PFG_ERR_INVALID, "bad arguments");
+	if (c->composite || c->m.mat != PFG_MAT_NEOHOOKEAN)
+		return fail(c, PFG_ERR_UNSUPPORTED, "the matrix-free product exists for NeoHookean only");
+	DeviceGuard g(c->device);
+	const size_t ndof = 3 * (size_t)c->m.N;
+	int st = ensure_staging(c, std::max<size_t>(ndof, 1));
+	if (st) return st;
+	const double *du, *dp;
+	if ((st = stage_in(c, u, mem, c->d_u, ndof, &du))) return st;
+	if ((st = stage_in(c, p, mem, c->d_p, ndof, &dp))) return st;
+	if ((st = ensure_vec_stage(c))) return st;
+	double *dst = mem == PFG_MEM_DEVICE ? q : c->d_out;
+	PFG_CUDA(c, launch_hessian_vector(c->m, du, dp, dst, c->sc, c->stream));
 	if (mem == PFG_MEM_HOST) return finish_host(c, q, c->d_out, ndof);
 	return PFG_OK;
 }

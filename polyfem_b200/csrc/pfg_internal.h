@@ -153,6 +153,10 @@ cudaError_t launch_ad_blocks(const DevMesh &m, const double *u, double *stage, c
 cudaError_t launch_ad_material_vjp(const DevMesh &m, const double *u, const double *adj, double *out, cudaStream_t s);
 cudaError_t launch_ad_shape_vjp_stage(const DevMesh &m, const double *u, const double *adj, const Scratch &sc,
 									  cudaStream_t s);
+// H p of the NeoHookean Hessian at u without the matrix (FP64); sc.vec_stage as the gradient's
+cudaError_t launch_hessian_vector(const DevMesh &m, const double *u, const double *p, double *out, const Scratch &sc,
+								  cudaStream_t s);
+cudaError_t launch_pack_lame(int E, const double *lambda, const double *mu, double2 *lame, cudaStream_t s);
 cudaError_t launch_material_vjp(const DevMesh &m, const double *u, const double *adj, double *out, cudaStream_t s);
 cudaError_t launch_shape_vjp(const DevMesh &m, const double *u, const double *adj, int prec, double *out,
 							 const Scratch &sc, cudaStream_t s);

@@ -69,3 +69,32 @@ def test_backward_matches_central_differences(require_gpu):
             scale = max(abs(fd), 1e-3 * np.abs(g).max())
             assert abs(g[idx] - fd) <= 1e-5 * scale, (k, idx, g[idx], fd)
     asm.close()
+
+
+@pytest.mark.parametrize("et", [M.P1_TET, M.P2_TET, M.Q1_HEX], ids=["P1", "P2", "Q1"])
+@pytest.mark.parametrize("g", [1, 3, 4])
+def test_hessian_vector_equals_assembled_product(require_gpu, et, g):
+    """H(u) p without the matrix against the assembled FP64 Hessian times p on shuffled
+    meshes (element counts off the block size), in host and device memory; NaN exactly on
+    the rows of inverted elements; refused for another formulation."""
+    import torch
+
+    from polyfem_b200 import PfgError
+    from _cases import permuted
+    mesh, lam, mu, u, p = make_case(et, g, seed=31, jitter=0.1 if g > 1 else 0.0)
+    m2, u2, _, pe = permuted(mesh, u, seed=2)
+    asm = NeoHookeanAssembler.from_mesh(m2, lam[pe], mu[pe])
+    H = asm.assemble_hessian(u2)
+    q = asm.hessian_vector(u2, p)
+    assert rel_err(q, H @ p) <= 1e-13
+    dev = lambda a: torch.tensor(a, device="cuda")
+    assert np.array_equal(asm.hessian_vector(dev(u2), dev(p)).cpu().numpy(), q)
+    flipped = u2.copy()
+    flipped.reshape(-1, 3)[m2.conn[0, 0]] += 3.0  # inverts elements around one node
+    bad = np.isnan(asm.hessian_vector(flipped, p))
+    Hn = asm.assemble_hessian(flipped).tocsr()
+    assert np.array_equal(bad, np.isnan(Hn @ p)) and bad.any()
+    asm.set_material("SaintVenant")
+    with pytest.raises(PfgError):
+        asm.hessian_vector(u2, p)
+    asm.close()
