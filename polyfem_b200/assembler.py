@@ -587,17 +587,21 @@ class ElasticForm:
         return self.assembler.assemble_hessian(x, self.precision, self.project_to_psd)
 
     # weighted (Form.hpp) -----------------------------------------------------
+    def _weighted(self, v):
+        w = self.weight() / self._scale
+        return v if w == 1.0 else v * w  # times one: a copy and, on the device, a launch for nothing
+
     def value(self, x):
-        return (self.weight() / self._scale) * self.value_unweighted(x)
+        return self._weighted(self.value_unweighted(x))
 
     def value_per_element(self, x):
-        return (self.weight() / self._scale) * self.value_per_element_unweighted(x)
+        return self._weighted(self.value_per_element_unweighted(x))
 
     def first_derivative(self, x):
-        return self.first_derivative_unweighted(x) * (self.weight() / self._scale)
+        return self._weighted(self.first_derivative_unweighted(x))
 
     def second_derivative(self, x):
-        return self.second_derivative_unweighted(x) * (self.weight() / self._scale)
+        return self._weighted(self.second_derivative_unweighted(x))
 
     def is_step_valid(self, x0, x1) -> bool:
         """ElasticForm::is_step_valid (ElasticForm.cpp:388-396): reject NaN gradients."""

@@ -8,6 +8,27 @@
 namespace pfg
 {
 
+// Elements of a thread block of the gradient and shape kernels
+constexpr int TILE_E = 128;
+
+// Where a tile of TILE_E consecutive elements leaves its contributions to nodal vectors:
+// summed over the tile in shared memory first, one slot per (tile, node), so most of the
+// traffic to the slots and back disappears (the tile's elements share most of their nodes).
+//  pos      : [E*n] place of (e, a) in the tile's buffer, grouped by node, elements ascending
+//  off      : [tiles+1] first tile node of every tile
+//  start    : [nodes of all tiles + tiles] first place of every tile node, an end entry per tile
+//  slot     : [nodes of all tiles] the slot of the tile node's sum, slots in node order, tiles ascending
+//  node_off : [N+1] slots of every node
+struct TilePlan
+{
+	const unsigned short *pos = nullptr; // NULL: one slot per incidence instead (DevMesh::eb_inc)
+	const int *off = nullptr;
+	const unsigned short *start = nullptr;
+	const int *slot = nullptr;
+	const int *node_off = nullptr;
+	int n_slots = 0;
+};
+
 // Device-resident mesh in the layout the kernels read.
 //  conn     : [n][E] int32 (structure of arrays: local node a of all elements is contiguous)
 //  gconn    : [n_g][E] int32 (aliases conn for isoparametric elements)
@@ -39,6 +60,9 @@ struct DevMesh
 	const int *ginc_off = nullptr;
 	const int *ginc_eb = nullptr;
 	const int *g_eb_inc = nullptr; // [E*n_g] inverse of ginc_eb (aliases eb_inc when isoparametric)
+	TilePlan tile, gtile; // nodal sums of the FE and the geometric nodes
+	const int *sel = nullptr; // MultiModels: only elements with sel[e] == comp contribute to nodal sums
+	int comp = 0;
 	int *err = nullptr; // set to 1 by a kernel whose bounded wait gave up (the context reports it)
 	int *work = nullptr; // element counter of the PSD projection's persistent warps (cleared before each launch)
 };
@@ -85,7 +109,7 @@ struct Scratch
 {
 	double *partials = nullptr;       // per-block energy partial sums
 	unsigned int *ticket = nullptr;   // last-block-done counter (returns to 0 after each launch)
-	unsigned long long *inverted = nullptr;
+	unsigned long long *inverted = nullptr; // [0] the last call's count, [1] the running one (zero between calls)
 	int max_blocks = 0;
 	double *vec_stage = nullptr;      // one 32-byte slot per incidence, in incidence (node) order: element gradient / shape contributions
 	void *hess_stage = nullptr;       // one packed block triangle per element (tri_pad values, FP64 or FP32)
@@ -124,7 +148,7 @@ cudaError_t launch_lump_rows(int n_nodes, const int *outer, const int *inner, co
 cudaError_t launch_fp64_blocks(const DevMesh &m, const double *u, double *stage, cudaStream_t s);
 cudaError_t launch_fp64_finish(const DevMesh &m, const DevPattern &p, double *stage, bool project_psd, cudaStream_t s);
 cudaError_t launch_gradient_stage(const DevMesh &m, const double *u, const Scratch &sc, cudaStream_t s);
-cudaError_t launch_gradient_gather(const DevMesh &m, const double *stage, double *g, cudaStream_t s);
+cudaError_t launch_gradient_gather(const DevMesh &m, const double *stage, double *g, unsigned long long *inverted, cudaStream_t s);
 cudaError_t launch_combine_elements(double *acc, const double *src, long long per, int E, const int *sel, int comp,
 									bool first, cudaStream_t s);
 cudaError_t launch_combine_slots(double *acc, const double *src, long long n_inc, int n, const int *inc_eb, const int *sel,
@@ -153,6 +177,12 @@ cudaError_t launch_ad_blocks(const DevMesh &m, const double *u, double *stage, c
 cudaError_t launch_ad_material_vjp(const DevMesh &m, const double *u, const double *adj, double *out, cudaStream_t s);
 cudaError_t launch_ad_shape_vjp_stage(const DevMesh &m, const double *u, const double *adj, const Scratch &sc,
 									  cudaStream_t s);
+// TilePlan arrays: slots before each node (node_off, N+1) and tile nodes before each tile
+// (off, tiles+1), both counts of the same (tile, node) pairs; then the places and slots
+cudaError_t launch_tile_counts(int E, int n_nodes, int nn, const int *inc_off, const int *inc_eb, int *node_off, int *off,
+							   cudaStream_t s);
+cudaError_t launch_tile_build(int E, int nn, const int *conn, const int *inc_off, const int *inc_eb, const int *off,
+							  const int *node_off, unsigned short *pos, unsigned short *start, int *slot, cudaStream_t s);
 // H p of the NeoHookean Hessian at u without the matrix (FP64); sc.vec_stage as the gradient's
 cudaError_t launch_hessian_vector(const DevMesh &m, const double *u, const double *p, double *out, const Scratch &sc,
 								  cudaStream_t s);

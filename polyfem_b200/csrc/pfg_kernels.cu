@@ -14,6 +14,7 @@
 #include "pfg_device.cuh"
 
 #include <cstdio>
+#include <type_traits>
 #include <cstdlib>
 
 namespace pfg
@@ -121,8 +122,8 @@ __global__ void __launch_bounds__(NT, elem_kernel_min_ctas<EL>()) k_energy(DevMe
 	// grid-stride: a resident grid, each thread summing its elements in order, so the
 	// block reduction and the partials' tail are paid once per resident block
 	double en = 0.0;
-	for (int e = blockIdx.x * NT + threadIdx.x; e < m.E; e += gridDim.x * NT) en += element_energy<EL, T>(m, u, e, inverted);
-	reduce_to_result<NT>(en, partials, result, ticket);
+	for (int e = blockIdx.x * NT + threadIdx.x; e < m.E; e += gridDim.x * NT) en += element_energy<EL, T>(m, u, e, inverted + 1);
+	reduce_to_result<NT>(en, partials, result, ticket, inverted);
 }
 
 template <class EL, class T, int NT>
@@ -136,12 +137,16 @@ __global__ void __launch_bounds__(NT) k_energy_per_element(DevMesh m, const doub
 // ---------------------------------------------------------------------------
 // gradient (NLAssembler::assemble_gradient)
 // ---------------------------------------------------------------------------
-template <class EL, class T, int NT>
-__global__ void __launch_bounds__(NT, EL::ET == 1 ? 8 : 1) k_gradient(DevMesh m, const double *__restrict__ u, double *__restrict__ stage,
+#ifndef PFG_P1_CTAS
+#define PFG_P1_CTAS 6
+#endif
+template <class EL, class T, int NT, bool TILED>
+__global__ void __launch_bounds__(NT, EL::ET == 1 ? (TILED ? PFG_P1_CTAS : 8) : 1) k_gradient(DevMesh m, const double *__restrict__ u, double *__restrict__ stage,
 												 unsigned long long *inverted)
 {
-	const int e = blockIdx.x * NT + threadIdx.x;
-	if (e >= m.E) return;
+	const bool on = blockIdx.x * NT + threadIdx.x < m.E;
+	if (!TILED && !on) return;
+	const int e = on ? blockIdx.x * NT + threadIdx.x : m.E - 1;
 	// The displacement gradient grad u = sum_a u_a (x) grad(phi_a) is formed in FP64
 	// in every mode: it is a difference of nearby nodal values, and rounding u or
 	// J^-T to FP32 first costs ~3x in the FP32 gradient's error on smooth fields.
@@ -235,15 +240,13 @@ __global__ void __launch_bounds__(NT, EL::ET == 1 ? 8 : 1) k_gradient(DevMesh m,
 				}
 			}
 	}
-	if (bad) atomicAdd(inverted, 1ull);
-	// the element's contributions, one 32-byte slot per incidence (e, a) at the
-	// incidence's position in node order: (G0, G1, G2, 0)
+	if (bad && on) atomicAdd(inverted + 1, 1ull);
+	double G[EL::N][3];
 #pragma unroll
 	for (int a = 0; a < EL::N; ++a)
-	{
-		const int k = __ldg(m.eb_inc + (size_t)e * EL::N + a);
-		st_slot(stage + (size_t)k * 4, double(Gacc[a][0]), double(Gacc[a][1]), double(Gacc[a][2]));
-	}
+#pragma unroll
+		for (int d = 0; d < 3; ++d) G[a][d] = double(Gacc[a][d]);
+	put_contributions<EL::N, NT, TILED>(m, m.tile, m.eb_inc, stage, e, on, G);
 }
 
 // Per node: the sum of its incidences' contributions in incidence (element) order
@@ -252,8 +255,9 @@ __global__ void __launch_bounds__(NT, EL::ET == 1 ? 8 : 1) k_gradient(DevMesh m,
 // run; loads are issued eight slots at a time.  Deterministic.
 template <int NT>
 __global__ void __launch_bounds__(NT) k_vec_gather(int n_nodes, const int *__restrict__ off,
-												   const double *__restrict__ stage, double *__restrict__ out)
+												   const double *__restrict__ stage, double *__restrict__ out, unsigned long long *inv)
 {
+	if (blockIdx.x == 0 && threadIdx.x == 0) publish_inverted(inv); // of the element kernel before it
 	constexpr int BATCH = 8;
 	const int B = blockIdx.x * NT + threadIdx.x;
 	if (B >= n_nodes) return;
@@ -292,8 +296,9 @@ __global__ void __launch_bounds__(NT) k_vec_gather(int n_nodes, const int *__res
 // loads per thread.
 template <int G, int NT>
 __global__ void __launch_bounds__(NT) k_vec_gather_group(int n_nodes, const int *__restrict__ off,
-														 const double *__restrict__ stage, double *__restrict__ out)
+														 const double *__restrict__ stage, double *__restrict__ out, unsigned long long *inv)
 {
+	if (blockIdx.x == 0 && threadIdx.x == 0) publish_inverted(inv); // of the element kernel before it
 	static_assert(G == 8 || G == 16 || G == 32, "node groups are aligned parts of a warp");
 	const int t = blockIdx.x * NT + threadIdx.x;
 	const int B = t / G, l = t % G;
@@ -328,20 +333,198 @@ __global__ void __launch_bounds__(NT) k_vec_gather_group(int n_nodes, const int 
 __host__ __device__ constexpr int nodes_of(int et) { return et == 1 ? 4 : et == 2 ? 10 : 8; }
 __host__ __device__ constexpr int geom_nodes_of(int et) { return et == 3 ? 8 : 4; }
 
-// Per-node sums of one 32-byte slot per incidence: a G-lane group per node when
-// nodes average more than 12 incidences, else one thread per node.
-static void launch_vec_gather(int n_nodes, const int *off, long long n_inc, const double *stage, double *out,
-							  cudaStream_t s)
+// Per-node sums of the slots (one per incidence, or per tile and node): a G-lane group per
+// node when nodes average more than 12 slots, else one thread per node.
+static void launch_vec_gather(int n_nodes, const int *off, long long n_inc, const TilePlan &tp, const double *stage, double *out,
+							  unsigned long long *inv, cudaStream_t s)
 {
+	if (tp.pos)
+	{
+		off = tp.node_off;
+		n_inc = tp.n_slots;
+	}
 	if (n_nodes <= 0) return;
 	constexpr int NT = 128;
 	if (n_inc > 12LL * n_nodes)
 	{
 		constexpr int G = 32;
-		k_vec_gather_group<G, NT><<<(int)(((long long)n_nodes * G + NT - 1) / NT), NT, 0, s>>>(n_nodes, off, stage, out);
+		k_vec_gather_group<G, NT><<<(int)(((long long)n_nodes * G + NT - 1) / NT), NT, 0, s>>>(n_nodes, off, stage, out, inv);
 	}
 	else
-		k_vec_gather<NT><<<(n_nodes + NT - 1) / NT, NT, 0, s>>>(n_nodes, off, stage, out);
+		k_vec_gather<NT><<<(n_nodes + NT - 1) / NT, NT, 0, s>>>(n_nodes, off, stage, out, inv);
+}
+
+// ---------------------------------------------------------------------------
+// TilePlan on the device.  A node's incidences are in element order, so those of one tile
+// follow one another: a slot per such run.
+// ---------------------------------------------------------------------------
+__global__ void k_tile_count(int n_nodes, int nn, const int *__restrict__ inc_off, const int *__restrict__ inc_eb,
+							 int *__restrict__ node_cnt, int *__restrict__ tile_cnt)
+{
+	const int B = blockIdx.x * blockDim.x + threadIdx.x;
+	if (B >= n_nodes) return;
+	int last = -1, c = 0;
+	for (int k = __ldg(inc_off + B); k < __ldg(inc_off + B + 1); ++k)
+	{
+		const int t = __ldg(inc_eb + k) / (nn * TILE_E);
+		if (t == last) continue;
+		last = t;
+		++c;
+		atomicAdd(tile_cnt + t, 1);
+	}
+	node_cnt[B] = c;
+}
+
+// exclusive prefix sums of x[0 .. n) in place, the total in x[n]; one block
+__global__ void __launch_bounds__(1024) k_exclusive_scan(int *x, int n)
+{
+	__shared__ int part[32];
+	__shared__ int carry;
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	if (threadIdx.x == 0) carry = 0;
+	__syncthreads();
+	for (int i0 = 0; i0 < n; i0 += 4096)
+	{
+		const int i = i0 + 4 * threadIdx.x;
+		int v[4], s = 0;
+#pragma unroll
+		for (int j = 0; j < 4; ++j)
+		{
+			v[j] = i + j < n ? x[i + j] : 0;
+			s += v[j];
+		}
+		int incl = s;
+#pragma unroll
+		for (int o = 1; o < 32; o *= 2)
+		{
+			const int y = __shfl_up_sync(0xffffffffu, incl, o);
+			if (lane >= o) incl += y;
+		}
+		if (lane == 31) part[warp] = incl;
+		__syncthreads();
+		if (warp == 0)
+		{
+			int p = part[lane];
+#pragma unroll
+			for (int o = 1; o < 32; o *= 2)
+			{
+				const int y = __shfl_up_sync(0xffffffffu, p, o);
+				if (lane >= o) p += y;
+			}
+			part[lane] = p;
+		}
+		__syncthreads();
+		int e = carry + incl - s + (warp ? part[warp - 1] : 0);
+#pragma unroll
+		for (int j = 0; j < 4; ++j)
+		{
+			if (i + j < n) x[i + j] = e;
+			e += v[j];
+		}
+		__syncthreads();
+		if (threadIdx.x == 0) carry += part[31];
+		__syncthreads();
+	}
+	if (threadIdx.x == 0) x[n] = carry;
+}
+
+// A block per tile: its incidences sorted by (node, element, local node), a run per node.
+template <int NN>
+__global__ void __launch_bounds__(TILE_E) k_tile_build(int E, const int *__restrict__ conn, const int *__restrict__ inc_off,
+													   const int *__restrict__ inc_eb, const int *__restrict__ off,
+													   const int *__restrict__ node_off, unsigned short *__restrict__ pos,
+													   unsigned short *__restrict__ start, int *__restrict__ slot)
+{
+	constexpr int P = NN * TILE_E <= 512 ? 512 : NN * TILE_E <= 1024 ? 1024 : 2048, PER = P / TILE_E;
+	__shared__ unsigned long long key[P];
+	__shared__ int warp_runs[TILE_E / 32];
+	const int tile = blockIdx.x, e0 = tile * TILE_E, ne = min(TILE_E, E - e0), tid = threadIdx.x, lane = tid & 31;
+	for (int i = tid; i < P; i += TILE_E)
+	{
+		const int el = i / NN, a = i % NN;
+		key[i] = el < ne ? (unsigned long long)__ldg(conn + (size_t)a * E + e0 + el) << 11 | (unsigned)i : ~0ull;
+	}
+	for (int k = 2; k <= P; k *= 2)
+		for (int j = k / 2; j > 0; j /= 2)
+		{
+			__syncthreads();
+			for (int i = tid; i < P / 2; i += TILE_E)
+			{
+				const int lo = 2 * i - (i & (j - 1)), hi = lo + j; // bit j of lo is clear
+				const unsigned long long x = key[lo], y = key[hi];
+				if ((x > y) == ((lo & k) == 0))
+				{
+					key[lo] = y;
+					key[hi] = x;
+				}
+			}
+		}
+	__syncthreads();
+	int runs = 0;
+	for (int q = 0; q < PER; ++q)
+	{
+		const int i = tid * PER + q;
+		runs += key[i] != ~0ull && (i == 0 || key[i] >> 11 != key[i - 1] >> 11);
+	}
+	int incl = runs;
+#pragma unroll
+	for (int o = 1; o < 32; o *= 2)
+	{
+		const int y = __shfl_up_sync(0xffffffffu, incl, o);
+		if (lane >= o) incl += y;
+	}
+	if (lane == 31) warp_runs[tid >> 5] = incl;
+	__syncthreads();
+	int r = incl - runs;
+	for (int w = 0; w < tid >> 5; ++w) r += warp_runs[w];
+	const int t0 = __ldg(off + tile);
+	for (int q = 0; q < PER; ++q)
+	{
+		const int i = tid * PER + q;
+		if (key[i] == ~0ull) break;
+		const int node = (int)(key[i] >> 11);
+		pos[(size_t)e0 * NN + (unsigned)(key[i] & 2047)] = (unsigned short)i;
+		if (i > 0 && (int)(key[i - 1] >> 11) == node) continue;
+		// the node's slot: its runs in earlier tiles come first
+		int last = -1, s = __ldg(node_off + node);
+		for (int k = __ldg(inc_off + node);; ++k)
+		{
+			const int t = __ldg(inc_eb + k) / (NN * TILE_E);
+			if (t >= tile) break;
+			s += t != last;
+			last = t;
+		}
+		start[t0 + tile + r] = (unsigned short)i;
+		slot[t0 + r] = s;
+		++r;
+	}
+	if (tid == 0) start[__ldg(off + tile + 1) + tile] = (unsigned short)(ne * NN);
+}
+
+cudaError_t launch_tile_counts(int E, int n_nodes, int nn, const int *inc_off, const int *inc_eb, int *node_off, int *off,
+							   cudaStream_t s)
+{
+	const int tiles = (E + TILE_E - 1) / TILE_E;
+	cudaError_t e = cudaMemsetAsync(off, 0, sizeof(int) * (size_t)(tiles + 1), s);
+	if (e != cudaSuccess) return e;
+	if (n_nodes > 0) k_tile_count<<<(n_nodes + 255) / 256, 256, 0, s>>>(n_nodes, nn, inc_off, inc_eb, node_off, off);
+	k_exclusive_scan<<<1, 1024, 0, s>>>(node_off, n_nodes);
+	k_exclusive_scan<<<1, 1024, 0, s>>>(off, tiles);
+	return cudaGetLastError();
+}
+
+cudaError_t launch_tile_build(int E, int nn, const int *conn, const int *inc_off, const int *inc_eb, const int *off,
+							  const int *node_off, unsigned short *pos, unsigned short *start, int *slot, cudaStream_t s)
+{
+	const int tiles = (E + TILE_E - 1) / TILE_E;
+	switch (nn)
+	{
+	case 4: k_tile_build<4><<<tiles, TILE_E, 0, s>>>(E, conn, inc_off, inc_eb, off, node_off, pos, start, slot); break;
+	case 8: k_tile_build<8><<<tiles, TILE_E, 0, s>>>(E, conn, inc_off, inc_eb, off, node_off, pos, start, slot); break;
+	case 10: k_tile_build<10><<<tiles, TILE_E, 0, s>>>(E, conn, inc_off, inc_eb, off, node_off, pos, start, slot); break;
+	default: return cudaErrorInvalidValue;
+	}
+	return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
@@ -1591,12 +1774,13 @@ __global__ void __launch_bounds__(NT) k_gen_energy_per_element(DevMesh m, const 
 
 // element gradient G[a][d] = sum_q da (P J^-1)[d][r] gref(q, a, r), staged per
 // incidence like the NeoHookean gradient
-template <class EL, int MAT, int NT>
+template <class EL, int MAT, int NT, bool TILED>
 __global__ void __launch_bounds__(NT) k_gen_gradient(DevMesh m, const double *__restrict__ u, double *__restrict__ stage,
 													 unsigned long long *inverted)
 {
-	const int e = blockIdx.x * NT + threadIdx.x;
-	if (e >= m.E) return;
+	const bool on = blockIdx.x * NT + threadIdx.x < m.E;
+	if (!TILED && !on) return;
+	const int e = on ? blockIdx.x * NT + threadIdx.x : m.E - 1;
 	double Xg[EL::NG][3], U[EL::N][3], Gacc[EL::N][3];
 	int nodes[EL::N];
 	load_geom<EL, double>(m, e, Xg);
@@ -1632,13 +1816,8 @@ __global__ void __launch_bounds__(NT) k_gen_gradient(DevMesh m, const double *__
 				}
 			}
 	}
-	if (bad) atomicAdd(inverted, 1ull);
-#pragma unroll
-	for (int a = 0; a < EL::N; ++a)
-	{
-		const int k = __ldg(m.eb_inc + (size_t)e * EL::N + a);
-		st_slot(stage + (size_t)k * 4, Gacc[a][0], Gacc[a][1], Gacc[a][2]);
-	}
+	if (bad && on) atomicAdd(inverted + 1, 1ull);
+	put_contributions<EL::N, NT, TILED>(m, m.tile, m.eb_inc, stage, e, on, Gacc);
 }
 
 // Element blocks for the other materials, one warp per element: per point (lanes
@@ -2112,12 +2291,13 @@ cudaError_t launch_hessian(const DevMesh &m, const DevPattern &p, const double *
 // a single product writes and reads the element triangles and the CSC values: P2 32^3
 // 881 -> 72 us.
 // ---------------------------------------------------------------------------
-template <class EL, int NT>
+template <class EL, int NT, bool TILED>
 __global__ void __launch_bounds__(NT) k_hessian_vector(DevMesh m, const double *__restrict__ u, const double *__restrict__ p,
 													   double *__restrict__ stage)
 {
-	const int e = blockIdx.x * NT + threadIdx.x;
-	if (e >= m.E) return;
+	const bool on = blockIdx.x * NT + threadIdx.x < m.E;
+	if (!TILED && !on) return;
+	const int e = on ? blockIdx.x * NT + threadIdx.x : m.E - 1;
 	double Xg[EL::NG][3];
 	double U[EL::N][3], Pn[EL::N][3];
 	int nodes[EL::N];
@@ -2205,12 +2385,7 @@ __global__ void __launch_bounds__(NT) k_hessian_vector(DevMesh m, const double *
 				}
 			}
 	}
-#pragma unroll
-	for (int a = 0; a < EL::N; ++a)
-	{
-		const int k = __ldg(m.eb_inc + (size_t)e * EL::N + a);
-		st_slot(stage + (size_t)k * 4, Gacc[a][0], Gacc[a][1], Gacc[a][2]);
-	}
+	put_contributions<EL::N, NT, TILED>(m, m.tile, m.eb_inc, stage, e, on, Gacc);
 }
 
 // (lambda, mu) pairs of the elements from two arrays (strided copies of 8 bytes a row took
@@ -2280,12 +2455,13 @@ __global__ void __launch_bounds__(NT) k_material_vjp(DevMesh m, const double *__
 //   R:grad p  = mu a.(Gp g) + (mu - lambda lnJ)(F^-T g).(Gp F^-1 a) + lambda (a.F^-T g)(F^-T:Gp)
 //   (P V^T - tr(V) P):grad p = (P g).Gp[:,d] - g_d (P:Gp),     a = Gu[:,d]
 // ---------------------------------------------------------------------------
-template <class EL, class T, int NT>
+template <class EL, class T, int NT, bool TILED>
 __global__ void __launch_bounds__(NT) k_shape_vjp(DevMesh m, const double *__restrict__ u,
 												  const double *__restrict__ adj, double *__restrict__ stage)
 {
-	const int e = blockIdx.x * NT + threadIdx.x;
-	if (e >= m.E) return;
+	const bool on = blockIdx.x * NT + threadIdx.x < m.E;
+	if (!TILED && !on) return;
+	const int e = on ? blockIdx.x * NT + threadIdx.x : m.E - 1;
 	T Xg[EL::NG][3];
 	T U[EL::N][3], Pn[EL::N][3];
 	int nodes[EL::N];
@@ -2388,12 +2564,12 @@ __global__ void __launch_bounds__(NT) k_shape_vjp(DevMesh m, const double *__res
 			}
 		}
 	}
+	double G[EL::NG][3];
 #pragma unroll
-	for (int v = 0; v < EL::NG; ++v)
-	{
-		const int k = __ldg(m.g_eb_inc + (size_t)e * EL::NG + v);
-		st_slot(stage + (size_t)k * 4, double(acc[v][0]), double(acc[v][1]), double(acc[v][2]));
-	}
+	for (int a = 0; a < EL::NG; ++a)
+#pragma unroll
+		for (int d = 0; d < 3; ++d) G[a][d] = double(acc[a][d]);
+	put_contributions<EL::NG, NT, TILED>(m, m.gtile, m.g_eb_inc, stage, e, on, G);
 }
 
 // ---------------------------------------------------------------------------
@@ -2449,11 +2625,17 @@ static void gen_energy_mat(const DevMesh &m, const double *u, bool per_element, 
 template <class EL>
 static void gen_gradient_mat(const DevMesh &m, const double *u, const Scratch &sc, cudaStream_t s)
 {
-	constexpr int NT = 128;
+	constexpr int NT = TILE_E;
+	const auto launch = [&](auto mat) {
+		if (m.tile.pos)
+			k_gen_gradient<EL, decltype(mat)::value, NT, true><<<blocks_for(m.E, NT), NT, 0, s>>>(m, u, sc.vec_stage, sc.inverted);
+		else
+			k_gen_gradient<EL, decltype(mat)::value, NT, false><<<blocks_for(m.E, NT), NT, 0, s>>>(m, u, sc.vec_stage, sc.inverted);
+	};
 	if (m.mat == MAT_ISO_NEOHOOKEAN)
-		k_gen_gradient<EL, MAT_ISO_NEOHOOKEAN, NT><<<blocks_for(m.E, NT), NT, 0, s>>>(m, u, sc.vec_stage, sc.inverted);
+		launch(std::integral_constant<int, MAT_ISO_NEOHOOKEAN>{});
 	else
-		k_gen_gradient<EL, MAT_SAINT_VENANT, NT><<<blocks_for(m.E, NT), NT, 0, s>>>(m, u, sc.vec_stage, sc.inverted);
+		launch(std::integral_constant<int, MAT_SAINT_VENANT>{});
 }
 
 int energy_elems_per_block(int) { return 256; }
@@ -2490,7 +2672,10 @@ template <class EL, class T>
 static void gradient_t(const DevMesh &m, const double *u, const Scratch &sc, cudaStream_t s)
 {
 	constexpr int NT = 128;
-	k_gradient<EL, T, NT><<<blocks_for(m.E, NT), NT, 0, s>>>(m, u, sc.vec_stage, sc.inverted);
+	if (m.tile.pos)
+		k_gradient<EL, T, NT, true><<<blocks_for(m.E, NT), NT, 0, s>>>(m, u, sc.vec_stage, sc.inverted);
+	else
+		k_gradient<EL, T, NT, false><<<blocks_for(m.E, NT), NT, 0, s>>>(m, u, sc.vec_stage, sc.inverted);
 }
 
 cudaError_t launch_gradient(const DevMesh &m, const double *u, int prec, double *g, const Scratch &sc, cudaStream_t s)
@@ -2518,7 +2703,7 @@ cudaError_t launch_gradient(const DevMesh &m, const double *u, int prec, double 
 		case 3: f32 ? gradient_t<Q1Hex, float>(m, u, sc, s) : gradient_t<Q1Hex, double>(m, u, sc, s); break;
 		default: return cudaErrorInvalidValue;
 		}
-	launch_vec_gather(m.N, m.inc_off, (long long)m.E * nodes_of(m.et), sc.vec_stage, g, s);
+	launch_vec_gather(m.N, m.inc_off, (long long)m.E * nodes_of(m.et), m.tile, sc.vec_stage, g, sc.inverted, s);
 	return cudaGetLastError();
 }
 
@@ -2526,16 +2711,22 @@ cudaError_t launch_hessian_vector(const DevMesh &m, const double *u, const doubl
 								  cudaStream_t s)
 {
 	if (m.E == 0) return cudaMemsetAsync(out, 0, sizeof(double) * 3 * (size_t)m.N, s);
-	constexpr int NT = 128;
+	constexpr int NT = TILE_E;
 	const int nb = blocks_for(m.E, NT);
+	const auto launch = [&](auto el) {
+		if (m.tile.pos)
+			k_hessian_vector<decltype(el), NT, true><<<nb, NT, 0, s>>>(m, u, p, sc.vec_stage);
+		else
+			k_hessian_vector<decltype(el), NT, false><<<nb, NT, 0, s>>>(m, u, p, sc.vec_stage);
+	};
 	switch (m.et)
 	{
-	case 1: k_hessian_vector<P1Tet, NT><<<nb, NT, 0, s>>>(m, u, p, sc.vec_stage); break;
-	case 2: k_hessian_vector<P2Tet, NT><<<nb, NT, 0, s>>>(m, u, p, sc.vec_stage); break;
-	case 3: k_hessian_vector<Q1Hex, NT><<<nb, NT, 0, s>>>(m, u, p, sc.vec_stage); break;
+	case 1: launch(P1Tet{}); break;
+	case 2: launch(P2Tet{}); break;
+	case 3: launch(Q1Hex{}); break;
 	default: return cudaErrorInvalidValue;
 	}
-	launch_vec_gather(m.N, m.inc_off, (long long)m.E * nodes_of(m.et), sc.vec_stage, out, s);
+	launch_vec_gather(m.N, m.inc_off, (long long)m.E * nodes_of(m.et), m.tile, sc.vec_stage, out, nullptr, s);
 	return cudaGetLastError();
 }
 
@@ -2569,6 +2760,9 @@ cudaError_t launch_shape_vjp(const DevMesh &m, const double *u, const double *ad
 	const int nb = blocks_for(m.E, NT);
 	const bool f32 = prec != PREC_FP64;
 	double *st = sc.vec_stage;
+	// tiles for P1 NeoHookean only (48^3: 81 -> 64 us): P2 and Q1 have few geometric slots for
+	// their arithmetic, and lose 1-4% to the pass through shared memory
+	const TilePlan plan = m.et == 1 && m.mat == 0 ? m.gtile : TilePlan();
 	if (m.mat != 0)
 	{
 		cudaError_t e = launch_ad_shape_vjp_stage(m, u, adj, sc, s);
@@ -2577,12 +2771,17 @@ cudaError_t launch_shape_vjp(const DevMesh &m, const double *u, const double *ad
 	else
 		switch (m.et)
 		{
-		case 1: f32 ? k_shape_vjp<P1Tet, float, NT><<<nb, NT, 0, s>>>(m, u, adj, st) : k_shape_vjp<P1Tet, double, NT><<<nb, NT, 0, s>>>(m, u, adj, st); break;
-		case 2: f32 ? k_shape_vjp<P2Tet, float, NT><<<nb, NT, 0, s>>>(m, u, adj, st) : k_shape_vjp<P2Tet, double, NT><<<nb, NT, 0, s>>>(m, u, adj, st); break;
-		case 3: f32 ? k_shape_vjp<Q1Hex, float, NT><<<nb, NT, 0, s>>>(m, u, adj, st) : k_shape_vjp<Q1Hex, double, NT><<<nb, NT, 0, s>>>(m, u, adj, st); break;
+		case 1:
+			if (plan.pos)
+				f32 ? k_shape_vjp<P1Tet, float, NT, true><<<nb, NT, 0, s>>>(m, u, adj, st) : k_shape_vjp<P1Tet, double, NT, true><<<nb, NT, 0, s>>>(m, u, adj, st);
+			else
+				f32 ? k_shape_vjp<P1Tet, float, NT, false><<<nb, NT, 0, s>>>(m, u, adj, st) : k_shape_vjp<P1Tet, double, NT, false><<<nb, NT, 0, s>>>(m, u, adj, st);
+			break;
+		case 2: f32 ? k_shape_vjp<P2Tet, float, NT, false><<<nb, NT, 0, s>>>(m, u, adj, st) : k_shape_vjp<P2Tet, double, NT, false><<<nb, NT, 0, s>>>(m, u, adj, st); break;
+		case 3: f32 ? k_shape_vjp<Q1Hex, float, NT, false><<<nb, NT, 0, s>>>(m, u, adj, st) : k_shape_vjp<Q1Hex, double, NT, false><<<nb, NT, 0, s>>>(m, u, adj, st); break;
 		default: return cudaErrorInvalidValue;
 		}
-	launch_vec_gather(m.Ng, m.ginc_off, (long long)m.E * geom_nodes_of(m.et), st, out, s);
+	launch_vec_gather(m.Ng, m.ginc_off, (long long)m.E * geom_nodes_of(m.et), plan, st, out, nullptr, s);
 	return cudaGetLastError();
 }
 
@@ -2815,10 +3014,10 @@ cudaError_t launch_gradient_stage(const DevMesh &m, const double *u, const Scrat
 	return cudaGetLastError();
 }
 
-cudaError_t launch_gradient_gather(const DevMesh &m, const double *stage, double *g, cudaStream_t s)
+cudaError_t launch_gradient_gather(const DevMesh &m, const double *stage, double *g, unsigned long long *inverted, cudaStream_t s)
 {
 	if (m.E == 0) return cudaMemsetAsync(g, 0, sizeof(double) * 3 * (size_t)m.N, s);
-	launch_vec_gather(m.N, m.inc_off, (long long)m.E * nodes_of(m.et), stage, g, s);
+	launch_vec_gather(m.N, m.inc_off, (long long)m.E * nodes_of(m.et), m.tile, stage, g, inverted, s);
 	return cudaGetLastError();
 }
 

@@ -617,12 +617,13 @@ __global__ void __launch_bounds__(NT) k_ad_energy_per_element(DevMesh m, const d
 
 // element gradient G[a][d] = sum_q da sum_c P[d][c] g_a[c], g_a = J^-T gref_a, one
 // slot per incidence as the other gradient kernels stage it
-template <class EL, int MAT, int NT>
+template <class EL, int MAT, int NT, bool TILED>
 __global__ void __launch_bounds__(NT) k_ad_gradient(DevMesh m, const double *__restrict__ u, double *__restrict__ stage,
 													unsigned long long *inverted)
 {
-	const int e = blockIdx.x * NT + threadIdx.x;
-	if (e >= m.E) return;
+	const bool on = blockIdx.x * NT + threadIdx.x < m.E;
+	if (!TILED && !on) return;
+	const int e = on ? blockIdx.x * NT + threadIdx.x : m.E - 1;
 	double Xg[EL::NG][3], U[EL::N][3], Gacc[EL::N][3];
 	int nodes[EL::N];
 	load_geom<EL, double>(m, e, Xg);
@@ -659,13 +660,8 @@ __global__ void __launch_bounds__(NT) k_ad_gradient(DevMesh m, const double *__r
 				}
 			}
 	}
-	if (bad) atomicAdd(inverted, 1ull);
-#pragma unroll
-	for (int a = 0; a < EL::N; ++a)
-	{
-		const int k = __ldg(m.eb_inc + (size_t)e * EL::N + a);
-		st_slot(stage + (size_t)k * 4, Gacc[a][0], Gacc[a][1], Gacc[a][2]);
-	}
+	if (bad && on) atomicAdd(inverted + 1, 1ull);
+	put_contributions<EL::N, NT, TILED>(m, m.tile, m.eb_inc, stage, e, on, Gacc);
 }
 
 // ---------------------------------------------------------------------------
@@ -1056,12 +1052,13 @@ __global__ void __launch_bounds__(NT) k_le_material_vjp(DevMesh m, const double 
 //   (C:M + P V^T - tr(V) P) : grad p = a.(Q g) + (P g).grad p[:, d] - g_d (P : grad p),
 // with a = grad u[:, d] and Q = C : grad p (C is symmetric in its index pairs).
 // Element contributions into one slot per geometric incidence.
-template <class EL, int MAT, int NT>
+template <class EL, int MAT, int NT, bool TILED>
 __global__ void __launch_bounds__(NT) k_ad_shape_vjp(DevMesh m, const double *__restrict__ u,
 													 const double *__restrict__ adj, double *__restrict__ stage)
 {
-	const int e = blockIdx.x * NT + threadIdx.x;
-	if (e >= m.E) return;
+	const bool on = blockIdx.x * NT + threadIdx.x < m.E;
+	if (!TILED && !on) return;
+	const int e = on ? blockIdx.x * NT + threadIdx.x : m.E - 1;
 	double Xg[EL::NG][3], U[EL::N][3], Pn[EL::N][3], acc[EL::NG][3];
 	int nodes[EL::N];
 	load_geom<EL, double>(m, e, Xg);
@@ -1112,12 +1109,7 @@ __global__ void __launch_bounds__(NT) k_ad_shape_vjp(DevMesh m, const double *__
 			}
 		}
 	}
-#pragma unroll
-	for (int v = 0; v < EL::NG; ++v)
-	{
-		const int k = __ldg(m.g_eb_inc + (size_t)e * EL::NG + v);
-		st_slot(stage + (size_t)k * 4, acc[v][0], acc[v][1], acc[v][2]);
-	}
+	put_contributions<EL::NG, NT, TILED>(m, m.gtile, m.g_eb_inc, stage, e, on, acc);
 }
 
 // ---------------------------------------------------------------------------
@@ -1178,7 +1170,10 @@ cudaError_t launch_ad_gradient_stage(const DevMesh &m, const double *u, const Sc
 	return with_ad_material(m, [&](auto el, auto mat) {
 		using EL = decltype(el);
 		constexpr int MAT = decltype(mat)::value, NT = 128;
-		k_ad_gradient<EL, MAT, NT><<<ad_blocks_for(m.E, NT), NT, 0, s>>>(m, u, sc.vec_stage, sc.inverted);
+		if (m.tile.pos)
+			k_ad_gradient<EL, MAT, NT, true><<<ad_blocks_for(m.E, NT), NT, 0, s>>>(m, u, sc.vec_stage, sc.inverted);
+		else
+			k_ad_gradient<EL, MAT, NT, false><<<ad_blocks_for(m.E, NT), NT, 0, s>>>(m, u, sc.vec_stage, sc.inverted);
 	});
 }
 
@@ -1223,7 +1218,7 @@ cudaError_t launch_ad_shape_vjp_stage(const DevMesh &m, const double *u, const d
 	const int nb = ad_blocks_for(m.E, NT);
 	auto launch = [&](auto el, auto mat) {
 		using EL = decltype(el);
-		k_ad_shape_vjp<EL, decltype(mat)::value, NT><<<nb, NT, 0, s>>>(m, u, adj, sc.vec_stage);
+		k_ad_shape_vjp<EL, decltype(mat)::value, NT, false><<<nb, NT, 0, s>>>(m, u, adj, sc.vec_stage);
 	};
 	auto by_el = [&](auto mat) -> cudaError_t {
 		switch (m.et)

@@ -37,7 +37,7 @@ struct NoallocScratch
 	double partials[PFG_NOALLOC_MAX_BLOCKS];
 	unsigned int ticket;
 	unsigned int pad;
-	unsigned long long inverted;
+	unsigned long long inverted[2];
 };
 static __device__ __align__(256) NoallocScratch g_noalloc_scratch;
 
@@ -118,8 +118,8 @@ extern "C" int pfg_energy_noalloc(int elem_type, int n_elements, int n_nodes, in
 	if (st != PFG_OK) return st;
 
 	cudaStream_t cs = static_cast<cudaStream_t>(stream);
-	// the ticket and the inverted counter must start at zero
-	ce = cudaMemsetAsync(&s->ticket, 0, sizeof(unsigned int) * 2 + sizeof(unsigned long long), cs);
+	// the ticket and the inverted counters must start at zero
+	ce = cudaMemsetAsync(&s->ticket, 0, sizeof(unsigned int) * 2 + 2 * sizeof(unsigned long long), cs);
 	if (ce != cudaSuccess) return noalloc_fail(PFG_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(ce));
 
 	pfg::DevMesh m;
@@ -134,7 +134,7 @@ extern "C" int pfg_energy_noalloc(int elem_type, int n_elements, int n_nodes, in
 	pfg::Scratch sc;
 	sc.partials = s->partials;
 	sc.ticket = &s->ticket;
-	sc.inverted = &s->inverted;
+	sc.inverted = s->inverted;
 	sc.max_blocks = PFG_NOALLOC_MAX_BLOCKS;
 	ce = pfg::launch_energy(m, u, prec, false, out, sc, cs);
 	if (ce != cudaSuccess) return noalloc_fail(PFG_ERR_CUDA, std::string("energy kernel: ") + cudaGetErrorString(ce));

@@ -266,3 +266,39 @@ def test_medium_mesh_hessian_against_oracle(require_gpu, et, g):
         assert rel_err(hs, v) <= 1e-6, prec
         assert np.array_equal(hs, asm.assemble_hessian_values(u, prec)), prec
     asm.close()
+
+
+@pytest.mark.parametrize("et", [M.P1_TET, M.P2_TET, M.Q1_HEX], ids=["P1", "P2", "Q1"])
+@pytest.mark.parametrize("E", [1, 127, 128, 129, 384])
+def test_gradient_tiles_at_block_edges(require_gpu, et, E):
+    """The nodal sums taken per tile of 128 elements: element counts on and beside the tile,
+    and the same elements shuffled (which leaves the per-tile sums unused), against the
+    oracle; repeated calls agree bitwise, and the inverted count is the last call's."""
+    import copy
+
+    from oracle.binding import Oracle
+    mesh, lam, mu, u, p = make_case(et, 8 if et == M.Q1_HEX else 4, seed=12)
+    sub = copy.copy(mesh)
+    sub.conn = np.ascontiguousarray(mesh.conn[:E])
+    sub.gconn = sub.conn if mesh.gconn is mesh.conn else np.ascontiguousarray(mesh.gconn[:E])
+    rng = np.random.default_rng(E)
+    order = rng.permutation(E)
+    shuf = copy.copy(sub)
+    shuf.conn = np.ascontiguousarray(sub.conn[order])
+    shuf.gconn = shuf.conn if mesh.gconn is mesh.conn else np.ascontiguousarray(sub.gconn[order])
+    for m_, l_, k_ in ((sub, lam[:E], mu[:E]), (shuf, lam[:E][order], mu[:E][order])):
+        orc = Oracle(m_, l_, k_)
+        asm = NeoHookeanAssembler.from_mesh(m_, l_, k_)
+        g = asm.assemble_gradient(u)
+        assert rel_err(g, orc.gradient(u)) <= 1e-12
+        assert asm.inverted_count() == 0
+        flipped = u.copy()
+        flipped.reshape(-1, 3)[m_.conn[0, 0]] += 10 * mesh.h
+        asm.assemble_energy(flipped)
+        n_bad = asm.inverted_count()
+        assert n_bad >= 1
+        asm.assemble_gradient(flipped)
+        assert asm.inverted_count() == n_bad
+        assert np.array_equal(asm.assemble_gradient(u), g) and asm.inverted_count() == 0
+        assert rel_err(asm.force_shape_derivative(u, p), orc.shape_vjp(u, p)) <= 1e-12
+        asm.close()
