@@ -665,7 +665,7 @@ __global__ void __launch_bounds__(NT) k_ad_gradient(DevMesh m, const double *__r
 }
 
 // ---------------------------------------------------------------------------
-// element blocks: one warp per element
+// element blocks
 // ---------------------------------------------------------------------------
 // Entry k (i <= j, tri_index(9, i, j) order) of the 9 x 9 table C, with i = 3a + A,
 // j = 3b + B: the flat indices and 0/1 factors of its terms, so that the lanes of a
@@ -714,23 +714,34 @@ constexpr CEntryTable make_centries()
 	return t;
 }
 __constant__ CEntryTable c_ad_centries = make_centries();
-// the pairs (x, y), x <= y, of the three invariants; the node pairs of the element
-// block triangle (P1, P2, Q1)
+// the pairs (x, y), x <= y, of the three invariants
 __constant__ PairTable c_ad_x3 = make_pairs(3);
-__constant__ PairTable c_ad_pairs[3] = {make_pairs(4), make_pairs(10), make_pairs(8)};
 
+// One element's workspace; the triangle takes the place of the point data at the end.
 template <class EL>
-struct AdWarp
+struct AdElem
 {
 	static constexpr int N = EL::N, NG = EL::NG, NQ = EL::NQ, TP = tri_pad(EL::N);
 	double U[N][3], X[NG][3];
 	double Jit[NQ][9], da[NQ];
-	Invariants inv[NQ];
-	double psi[NQ][9];              // psi_x (x = I1, I2, J), then psi_xy (x <= y) in tri_index(3, x, y) order
-	double C[NQ][45];               // da d2psi/dF2 at point q, entry (i <= j) at tri_index(9, i, j)
-	alignas(16) double g[NQ][N][4]; // physical basis gradients (x, y, z, 0): two 16-byte loads
-	alignas(16) double tri[TP];     // the element's packed block triangle, copied out as double2
+	double psi[NQ][9]; // psi_x (x = I1, I2, J), then psi_xy (x <= y) in tri_index(3, x, y) order
+	struct Point
+	{
+		Invariants inv[NQ];
+		double C[NQ][45];   // da d2psi/dF2 at point q, entry (i <= j) at tri_index(9, i, j)
+		double g[NQ][N][3]; // physical basis gradients
+	};
+	static constexpr size_t BODY = sizeof(Point) > TP * sizeof(double) ? sizeof(Point) : TP * sizeof(double);
+	static constexpr size_t HEAD = 16 * ((sizeof(double) * (3 * N + 3 * NG + 19 * NQ) + 15) / 16);
+	// elements 4 doubles apart mod 16: what the warp's elements read at one place falls on
+	// distinct banks; whole 16-byte vectors for the triangle
+	static constexpr size_t WORDS = (HEAD + BODY) / 8, SIZE = 8 * (WORDS + (20 - WORDS % 16) % 16);
 };
+// elements a warp takes at once (a lane per element and local node), warps per CTA
+template <class EL>
+__host__ __device__ constexpr int ad_elems() { return 32 / EL::N; }
+template <class EL>
+__host__ __device__ constexpr int ad_warps() { return EL::ET == 3 ? 2 : 4; }
 
 __host__ __device__ constexpr int c9(int i, int j) { return i <= j ? tri_index(9, i, j) : tri_index(9, j, i); }
 
@@ -770,41 +781,71 @@ __device__ __forceinline__ double inv_hessian_entry(const Invariants &v, const d
 	return h;
 }
 
+// A warp takes `per` <= 32 / N elements at once through the lane phases (points; (point, node);
+// (point, invariant pair); (point, entry of C)), then a lane per (element, row node a): at
+// every point it contracts its g_a with C once, T[k][d] = sum_c g_a[c] C[(r,c),(k,d)] row by
+// row, and uses it for the blocks (a, a + d mod N), d = 0 .. N/2 (every pair once; d = N/2
+// from the lower half only): 243 multiply-adds and 63 shared loads for 5.5 blocks (P2).  A
+// lane per node pair of one element at a time contracted C anew for each, 108 multiply-adds
+// and 49 loads a block, and left most lanes idle in the point phases.
+// MooneyRivlin P2 21^3: 331 -> 208 us, P1 36^3: 463 -> 200, Q1 40^3: 640 -> 470.
 template <class EL, int MAT, int WPB>
-__global__ void __launch_bounds__(WPB * 32) k_ad_blocks(DevMesh m, const double *__restrict__ u, double *__restrict__ stage)
+__global__ void __launch_bounds__(WPB * 32, EL::ET == 2 ? 3 : 1) k_ad_blocks(DevMesh m, const double *__restrict__ u, double *__restrict__ stage, int per)
 {
-	using W = AdWarp<EL>;
-	constexpr int N = EL::N, NG = EL::NG, NQ = EL::NQ, NP = N * (N + 1) / 2, TP = W::TP;
+	using W = AdElem<EL>;
+	constexpr int N = EL::N, NG = EL::NG, NQ = EL::NQ, TP = W::TP, EPW = ad_elems<EL>(), ND = N / 2 + 1;
 	extern __shared__ __align__(16) unsigned char smem_raw[];
-	W &S = reinterpret_cast<W *>(smem_raw)[threadIdx.x >> 5];
+	unsigned char *warp_mem = smem_raw + (size_t)(threadIdx.x >> 5) * EPW * W::SIZE;
+	const auto elem = [&](int k) -> W & { return *reinterpret_cast<W *>(warp_mem + (size_t)k * W::SIZE); };
+	const auto body = [&](int k) { return reinterpret_cast<typename W::Point *>(warp_mem + (size_t)k * W::SIZE + W::HEAD); };
 	const int lane = threadIdx.x & 31;
 	// the lookup tables in shared memory: lanes at different entries read them without
 	// the serialisation of divergent constant-memory reads
 	__shared__ CEntry s_ce[45];
-	__shared__ unsigned char s_pa[NP], s_pb[NP], s_xa[6], s_xb[6];
+	__shared__ unsigned char s_xa[6], s_xb[6];
+	__shared__ double s_g[NQ][N][3]; // reference gradients (evaluated per lane they diverge: a third of the kernel's time)
 	for (int t = threadIdx.x; t < 45; t += WPB * 32) s_ce[t] = c_ad_centries.e[t];
-	for (int t = threadIdx.x; t < NP; t += WPB * 32)
-	{
-		s_pa[t] = c_ad_pairs[EL::ET - 1].a[t];
-		s_pb[t] = c_ad_pairs[EL::ET - 1].b[t];
-	}
 	for (int t = threadIdx.x; t < 6; t += WPB * 32)
 	{
 		s_xa[t] = c_ad_x3.a[t];
 		s_xb[t] = c_ad_x3.b[t];
 	}
+	if (threadIdx.x < NQ)
+#pragma unroll
+		for (int q = 0; q < NQ; ++q)
+			if (q == threadIdx.x)
+#pragma unroll
+				for (int n = 0; n < N; ++n)
+#pragma unroll
+					for (int r = 0; r < 3; ++r) s_g[q][n][r] = gref<EL>(q, n, r);
 	__syncthreads();
-	for (int e = blockIdx.x * WPB + (threadIdx.x >> 5); e < m.E; e += gridDim.x * WPB)
+	const int el = lane / N, a = lane % N; // of the contraction; el >= ne: no element
+	for (int e0 = (blockIdx.x * WPB + (threadIdx.x >> 5)) * per; e0 < m.E; e0 += gridDim.x * WPB * per)
 	{
-		for (int i = lane; i < N * 3; i += 32)
-			S.U[i / 3][i % 3] = __ldg(u + (size_t)__ldg(m.conn + (size_t)(i / 3) * m.E + e) * 3 + i % 3);
-		for (int i = lane; i < NG * 3; i += 32)
-			S.X[i / 3][i % 3] = __ldg(m.X + (size_t)__ldg(m.gconn + (size_t)(i / 3) * m.E + e) * 3 + i % 3);
-		__syncwarp();
-		const MatP prm = ad_params<MAT>(m, e);
-		if (lane < NQ)
+		const int ne = min(per, m.E - e0);
+		if (el < ne)
 		{
-			const int q = lane;
+			const double *uu = u + (size_t)__ldg(m.conn + (size_t)a * m.E + e0 + el) * 3;
+			const double *xx = m.X + (size_t)(a < NG ? __ldg(m.gconn + (size_t)a * m.E + e0 + el) : 0) * 3;
+			double v[3], y[3];
+#pragma unroll
+			for (int d = 0; d < 3; ++d)
+			{
+				v[d] = __ldg(uu + d);
+				y[d] = a < NG ? __ldg(xx + d) : 0.0;
+			}
+#pragma unroll
+			for (int d = 0; d < 3; ++d)
+			{
+				elem(el).U[a][d] = v[d];
+				if (a < NG) elem(el).X[a][d] = y[d];
+			}
+		}
+		__syncwarp();
+		for (int t = lane; t < ne * NQ; t += 32)
+		{
+			const int k = t / NQ, q = t % NQ;
+			W &S = elem(k);
 			double Jit[3][3], detJ, F[3][3];
 			geometry<EL, double>(q, S.X, Jit, detJ);
 			gen_def_grad<EL>(q, S.U, Jit, F);
@@ -813,52 +854,58 @@ __global__ void __launch_bounds__(WPB * 32) k_ad_blocks(DevMesh m, const double 
 #pragma unroll
 				for (int c = 0; c < 3; ++c) S.Jit[q][3 * r + c] = Jit[r][c];
 			S.da[q] = detJ * qweight<EL>(q);
-			if constexpr (!quadratic_mat<MAT>()) invariants(F, S.inv[q]); // entry_mat: F = dI1/dF / 2
+			if constexpr (!quadratic_mat<MAT>()) invariants(F, body(k)->inv[q]); // entry_mat: F = dI1/dF / 2
 			if constexpr (MAT == MAT_SAINT_VENANT_TENSOR)
 			{
 				// the point's Voigt stress, shared by its 45 tangent entries (psi is unused here)
-				double e[6];
-				green_voigt_stress(S.inv[q].Cr, m.hooke, e, S.psi[q]);
+				double ev[6];
+				green_voigt_stress(body(k)->inv[q].Cr, m.hooke, ev, S.psi[q]);
 			}
 		}
 		__syncwarp();
 		// lanes over (point, node): g = J^-T gref
-		for (int t = lane; t < NQ * N; t += 32)
+		for (int t = lane; t < ne * NQ * N; t += 32)
 		{
-			const int q = t / N, a = t - q * N;
-			double *g = S.g[q][a];
+			const int k = t / (NQ * N), q = t / N % NQ, b = t % N;
+			const W &S = elem(k);
+			double *g = body(k)->g[q][b];
 #pragma unroll
 			for (int c = 0; c < 3; ++c)
-				g[c] = gref<EL>(q, a, 0) * S.Jit[q][c] + gref<EL>(q, a, 1) * S.Jit[q][3 + c] + gref<EL>(q, a, 2) * S.Jit[q][6 + c];
-			g[3] = 0.0;
+				g[c] = s_g[q][b][0] * S.Jit[q][c] + s_g[q][b][1] * S.Jit[q][3 + c] + s_g[q][b][2] * S.Jit[q][6 + c];
 		}
 		if constexpr (invariant_mat<MAT>())
 		{
 			// lanes over (point, invariant pair x <= y): one hyper-dual evaluation each
-			for (int t = lane; t < NQ * 6; t += 32)
+			for (int t = lane; t < ne * NQ * 6; t += 32)
 			{
-				const int q = t / 6, k = t - q * 6, x = s_xa[k], y = s_xb[k];
-				const Invariants &v = S.inv[q];
+				const int k = t / (NQ * 6), q = t / 6 % NQ, i = t % 6, x = s_xa[i], y = s_xb[i];
+				W &S = elem(k);
+				const Invariants &v = body(k)->inv[q];
 				const HDual h = inv_psi<MAT, HDual>({v.I1, x == 0 ? 1.0 : 0.0, y == 0 ? 1.0 : 0.0, 0.0},
 													{v.I2, x == 1 ? 1.0 : 0.0, y == 1 ? 1.0 : 0.0, 0.0},
-													{v.J, x == 2 ? 1.0 : 0.0, y == 2 ? 1.0 : 0.0, 0.0}, prm);
-				S.psi[q][3 + k] = h.ab;
+													{v.J, x == 2 ? 1.0 : 0.0, y == 2 ? 1.0 : 0.0, 0.0}, ad_params<MAT>(m, e0 + k));
+				S.psi[q][3 + i] = h.ab;
 				if (x == y) S.psi[q][x] = h.a;
 			}
 			__syncwarp();
 		}
 		// lanes over (point, entry i <= j of C)
-		for (int t = lane; t < NQ * 45; t += 32)
+		for (int t = lane; t < ne * NQ * 45; t += 32)
 		{
-			const int q = t / 45, k = t - q * 45;
-			const CEntry ce = s_ce[k];
+			const int k = t / (NQ * 45), q = t / 45 % NQ, i = t % 45;
+			const W &S = elem(k);
+			typename W::Point *B = body(k);
+			const CEntry ce = s_ce[i];
 			double h;
 			if constexpr (MAT == MAT_SAINT_VENANT_TENSOR)
-				h = svt_hessian_entry(S.inv[q], S.psi[q], m.hooke, ce);
+				h = svt_hessian_entry(B->inv[q], S.psi[q], m.hooke, ce);
 			else if constexpr (MAT == MAT_HOOKE)
 				h = __ldg(m.hooke + 6 * voigt(ce.i / 3, ce.i % 3) + voigt(ce.j / 3, ce.j % 3));
 			else if constexpr (MAT == MAT_LINEAR_ELASTICITY)
+			{
+				const MatP prm = ad_params<MAT>(m, e0 + k);
 				h = prm.y * (ce.dab * ce.dAB + ce.le_aBbA) + prm.x * ce.le_aAbB;
+			}
 			else if constexpr (entry_mat<MAT>())
 			{
 				// one hyper-dual evaluation over the entries (i, j) of F
@@ -866,54 +913,80 @@ __global__ void __launch_bounds__(WPB * 32) k_ad_blocks(DevMesh m, const double 
 #pragma unroll
 				for (int r = 0; r < 3; ++r)
 #pragma unroll
-					for (int c = 0; c < 3; ++c) F[r][c] = 0.5 * S.inv[q].dx[0][3 * r + c];
+					for (int c = 0; c < 3; ++c) F[r][c] = 0.5 * B->inv[q].dx[0][3 * r + c];
 #pragma unroll
 				for (int l = 0; l < 9; ++l) ej[l] = l == ce.j ? 1.0 : 0.0;
 				HDual Fh[3][3];
 				hd_def_grad(F, ce.i, ej, Fh);
-				h = ogden_psi<MAT, HDual>(Fh, prm).ab;
+				h = ogden_psi<MAT, HDual>(Fh, ad_params<MAT>(m, e0 + k)).ab;
 			}
 			else
-				h = inv_hessian_entry(S.inv[q], S.psi[q], ce);
-			S.C[q][k] = S.da[q] * h;
+				h = inv_hessian_entry(B->inv[q], S.psi[q], ce);
+			B->C[q][i] = S.da[q] * h;
 		}
 		__syncwarp();
-		// lanes over node pairs (a <= b): H_ab[r][k] = sum_q sum_{c,d} g_a[c] C[(r,c),(k,d)] g_b[d]
-		for (int p = lane; p < NP; p += 32)
+		double h[ND][3][3];
+#pragma unroll
+		for (int d = 0; d < ND; ++d)
+#pragma unroll
+			for (int r = 0; r < 3; ++r) h[d][r][0] = h[d][r][1] = h[d][r][2] = 0.0;
+		if (el < ne)
 		{
-			const int a = s_pa[p], b = s_pb[p];
-			double h[3][3] = {};
+			const typename W::Point *B = body(el);
+#pragma unroll 1
 			for (int q = 0; q < NQ; ++q)
 			{
-				const double2 a01 = reinterpret_cast<const double2 *>(S.g[q][a])[0], a2 = reinterpret_cast<const double2 *>(S.g[q][a])[1];
-				const double2 b01 = reinterpret_cast<const double2 *>(S.g[q][b])[0], b2 = reinterpret_cast<const double2 *>(S.g[q][b])[1];
-				const double ga[3] = {a01.x, a01.y, a2.x}, gb[3] = {b01.x, b01.y, b2.x};
-				const double *Cq = S.C[q];
+				const double *Cq = B->C[q];
+				double g[ND][3];
+#pragma unroll
+				for (int d = 0; d < ND; ++d)
+				{
+					const int b = a + d < N ? a + d : a + d - N;
+#pragma unroll
+					for (int c = 0; c < 3; ++c) g[d][c] = B->g[q][b][c];
+				}
+#pragma unroll
+				for (int r = 0; r < 3; ++r)
+				{
+					double T[3][3];
+#pragma unroll
+					for (int k = 0; k < 3; ++k)
+#pragma unroll
+						for (int c = 0; c < 3; ++c)
+							T[k][c] = g[0][0] * Cq[c9(3 * r, 3 * k + c)] + g[0][1] * Cq[c9(3 * r + 1, 3 * k + c)] +
+									  g[0][2] * Cq[c9(3 * r + 2, 3 * k + c)];
+#pragma unroll
+					for (int d = 0; d < ND; ++d)
+#pragma unroll
+						for (int k = 0; k < 3; ++k)
+							h[d][r][k] = fma(T[k][2], g[d][2], fma(T[k][1], g[d][1], fma(T[k][0], g[d][0], h[d][r][k])));
+				}
+			}
+		}
+		__syncwarp();
+		if (el < ne)
+		{
+			double *R = reinterpret_cast<double *>(body(el));
+#pragma unroll
+			for (int d = 0; d < ND; ++d)
+			{
+				const int b = a + d < N ? a + d : a + d - N;
+				if (d == ND - 1 && a >= N / 2) continue; // the pair belongs to lane b
+				const bool up = a <= b; // else stored transposed as (b, a)
+				double *H = R + 9 * (up ? tri_index(N, a, b) : tri_index(N, b, a));
 #pragma unroll
 				for (int r = 0; r < 3; ++r)
 #pragma unroll
-					for (int k = 0; k < 3; ++k)
-					{
-						double s_ = 0.0;
-#pragma unroll
-						for (int c = 0; c < 3; ++c)
-						{
-							const double w = Cq[c9(3 * r + c, 3 * k)] * gb[0] + Cq[c9(3 * r + c, 3 * k + 1)] * gb[1] +
-											 Cq[c9(3 * r + c, 3 * k + 2)] * gb[2];
-							s_ += ga[c] * w;
-						}
-						h[r][k] += s_;
-					}
+					for (int k = 0; k < 3; ++k) H[up ? 3 * k + r : 3 * r + k] = h[d][r][k];
 			}
-#pragma unroll
-			for (int r = 0; r < 3; ++r)
-#pragma unroll
-				for (int k = 0; k < 3; ++k) S.tri[9 * p + 3 * k + r] = h[r][k];
 		}
 		__syncwarp();
-		double2 *dst = reinterpret_cast<double2 *>(stage + (size_t)e * TP);
-		const double2 *src = reinterpret_cast<const double2 *>(S.tri);
-		for (int i = lane; i < TP / 2; i += 32) dst[i] = src[i];
+		for (int k = 0; k < ne; ++k)
+		{
+			double2 *dst = reinterpret_cast<double2 *>(stage + (size_t)(e0 + k) * TP);
+			const double2 *src = reinterpret_cast<const double2 *>(body(k));
+			for (int i = lane; i < TP / 2; i += 32) dst[i] = src[i];
+		}
 		__syncwarp();
 	}
 }
@@ -1183,12 +1256,15 @@ cudaError_t launch_ad_blocks(const DevMesh &m, const double *u, double *stage, c
 	cudaError_t err = cudaSuccess;
 	cudaError_t st = with_ad_material(m, [&](auto el, auto mat) {
 		using EL = decltype(el);
-		constexpr int MAT = decltype(mat)::value, WPB = 4;
-		const size_t bytes = WPB * sizeof(AdWarp<EL>);
+		constexpr int MAT = decltype(mat)::value, WPB = ad_warps<EL>();
+		const size_t bytes = WPB * ad_elems<EL>() * AdElem<EL>::SIZE;
 		err = cudaFuncSetAttribute(k_ad_blocks<EL, MAT, WPB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 		if (err != cudaSuccess) return;
-		const int nb = std::min((m.E + WPB - 1) / WPB, 148 * 32);
-		k_ad_blocks<EL, MAT, WPB><<<nb, WPB * 32, bytes, s>>>(m, u, stage);
+		// an element for every warp of a resident grid before a warp takes several:
+		// Q1 6^3 (216 elements) 21 us with four elements a warp, 11.5 with one
+		const int per = std::min(ad_elems<EL>(), (m.E + 148 * 3 * WPB - 1) / (148 * 3 * WPB));
+		const int nb = std::min((m.E + per * WPB - 1) / (per * WPB), 148 * 6);
+		k_ad_blocks<EL, MAT, WPB><<<nb, WPB * 32, bytes, s>>>(m, u, stage, per);
 	});
 	return err != cudaSuccess ? err : st;
 }

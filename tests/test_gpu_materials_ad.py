@@ -190,3 +190,23 @@ def test_adjoint_terms_the_reference_lacks(require_gpu):
         asm.force_shape_derivative(u, p, "fp32")
     assert ei.value.status == 4
     asm.close()
+
+
+@pytest.mark.parametrize("et,g,E", [(M.P1_TET, 9, 4374), (M.P2_TET, 8, 2500), (M.Q1_HEX, 13, 2197)]
+                         + [(M.Q1_HEX, 4, n) for n in (1, 3, 4, 5, 15, 16, 17)], ids=str)
+def test_blocks_of_several_elements_per_warp(require_gpu, et, g, E):
+    """Element counts that leave a warp's last group, a block's last warp or a last block
+    part filled, in the kernels that give a warp several elements: MooneyRivlin, and the
+    FP64 NeoHookean blocks of Q1, against the oracle."""
+    import copy
+    mesh, lam, mu, u, _ = make_case(et, g, seed=19)
+    sub = copy.copy(mesh)
+    sub.conn = np.ascontiguousarray(mesh.conn[:E])
+    sub.gconn = sub.conn if mesh.gconn is mesh.conn else np.ascontiguousarray(mesh.gconn[:E])
+    prm = material_params("MooneyRivlin", E, seed=4)
+    asm = NeoHookeanAssembler.from_mesh(sub, lam[:E], mu[:E])
+    for mat in ("MooneyRivlin", "NeoHookean") if et == M.Q1_HEX else ("MooneyRivlin",):
+        asm.set_material(mat, **(prm if mat == "MooneyRivlin" else {}))
+        orc = Oracle(sub, lam[:E], mu[:E], n_threads=4, material=mat, params=prm if mat == "MooneyRivlin" else None)
+        assert rel_err(asm.assemble_hessian_values(u), orc.hessian(u)[2]) <= 1e-12
+    asm.close()
