@@ -1217,7 +1217,7 @@ static cudaError_t launch_blocks_fp64(const DevMesh &m, const double *u, double 
 // values c, c+3, c+6), and writes them once.  No shared memory, no atomics: the
 // sum order of every entry is fixed.
 template <class EL, class T, int WARPS>
-__global__ void __launch_bounds__(WARPS * 32, 8)
+__global__ void __launch_bounds__(WARPS * 32, 64 / WARPS)
 	k_hessian_reduce(DevMesh m, DevPattern pat, const T *__restrict__ stage)
 {
 	constexpr int N = EL::N;
@@ -1296,12 +1296,14 @@ __global__ void __launch_bounds__(WARPS * 32, 8)
 	}
 }
 
-// Pass 2 of every Hessian-pattern assembly.
+// Pass 2 of every Hessian-pattern assembly, four nodes per block: a block leaves when its
+// longest column is done (P2 32^3 FP64: 16 warps 511 us, 8 400, 4 387, 2 429; Q1 64^3: 344,
+// 335, 324, 324; P1 48^3: 206, 199, 195, 195).
 template <class EL, class T>
 static cudaError_t launch_reduce(const DevMesh &m, const DevPattern &p, const T *stage, cudaStream_t s)
 {
 	if (m.N <= 0) return cudaSuccess;
-	constexpr int WARPS = 8;
+	constexpr int WARPS = 4;
 	k_hessian_reduce<EL, T, WARPS><<<(m.N + WARPS - 1) / WARPS, WARPS * 32, 0, s>>>(m, p, stage);
 	return cudaGetLastError();
 }
@@ -1393,8 +1395,9 @@ __device__ __forceinline__ double rcp_nr(double q)
 // (p_i, p_{i-1}) is rescaled by 2^500 every fourth step once |p_i| < 2^-500, so
 // no minor underflows (|d_i - x| <= 2.001 and e_i^2 <= 1 bound the growth by
 // (1 + sqrt 2)^30 < 2^40 between rescalings).
-template <int M>
-__device__ __forceinline__ int sturm_count(const double2 *__restrict__ de2, double x)
+// RATIO: ratio = p_M / p_{M-1}, zero at an eigenvalue and falling through it.
+template <int M, bool RATIO>
+__device__ __forceinline__ int sturm_count(const double2 *__restrict__ de2, double x, double &ratio)
 {
 	double pm = 1.0, p = de2[0].x - x;
 	if (p == 0.0) p = -PSD_PIVMIN;
@@ -1415,6 +1418,7 @@ __device__ __forceinline__ int sturm_count(const double2 *__restrict__ de2, doub
 		pm = p;
 		p = pn;
 	}
+	if constexpr (RATIO) ratio = p / pm;
 	return c;
 }
 
@@ -1524,6 +1528,43 @@ __device__ __forceinline__ void psd_reflect(const PW &S, double (&y)[M], int i)
 	}
 }
 
+// All steps in bands: step i runs over the first W >= i columns, W = M, then M minus one
+// band, ... (the columns beyond hold zeros of u and q: the same bits with fewer multiply-adds).
+// Three bands for P2 and Q1, two for P1's 12 rows; more are more code, and the kernel is
+// bound by fetching it (see psd_phase): P2 24^3 with five bands 2,824 us, three 2,799.
+template <int M>
+__host__ __device__ constexpr int psd_band() { return M > 12 ? (M / 3 + 1) / 2 * 2 : M / 2; }
+// The warps of a block enter each phase together: the unrolled phases are larger than the
+// instruction caches, and warps that drift apart fetch each one's code anew (P2 24^3
+// 3,260 us without the barriers, 2,842 with, 2,799 with one per band too).  P1's warps take
+// elements from a counter and cannot wait for one another.  A warp that has left (a
+// projected or positive element) does not hold the others.
+template <int M>
+__device__ __forceinline__ void psd_phase()
+{
+	if constexpr (M > 12) __syncthreads();
+}
+template <int M, int W, class PW>
+__device__ __forceinline__ void psd_tridiagonalise(PW &S, double (&a)[M], int lane)
+{
+	constexpr int NEXT = W - psd_band<M>();
+#pragma unroll 1
+	for (int i = W == M ? M - 1 : W; i > (NEXT > 0 ? NEXT : 1); --i) psd_tred2_step<M, W>(S, a, i, lane);
+	if constexpr (NEXT > 0)
+	{
+		psd_phase<M>();
+		psd_tridiagonalise<M, NEXT>(S, a, lane);
+	}
+}
+template <int M, int W, class PW>
+__device__ __forceinline__ void psd_back_transform(const PW &S, double (&y)[M])
+{
+	constexpr int NEXT = W - psd_band<M>();
+	if constexpr (NEXT > 0) psd_back_transform<M, NEXT>(S, y);
+#pragma unroll 1
+	for (int i = (NEXT > 0 ? NEXT : 1) + 1; i <= (W == M ? M - 1 : W); ++i) psd_reflect<M, W>(S, y, i);
+}
+
 // The projection of element e by one warp (all 32 lanes, converged on entry and
 // on every return; S is the warp's shared workspace)
 template <class EL, class T>
@@ -1555,13 +1596,8 @@ __device__ __forceinline__ void psd_element(PsdWarp<EL> &S, T *__restrict__ stag
 	for (int t = 0; t < M; ++t) nan_in |= isnan(a[t]);
 	if (__any_sync(FULL, nan_in)) return; // NaN propagates unchanged
 
-	// --- 1. tridiagonalisation ------------------------------------------------
-	// steps M-1 .. H+1 touch all columns, steps H .. 2 only columns < H
-	constexpr int H = ((M / 2) + 1) & ~1;
-#pragma unroll 1
-	for (int i = M - 1; i > H; --i) psd_tred2_step<M, M>(S, a, i, lane);
-#pragma unroll 1
-	for (int i = H; i >= 2; --i) psd_tred2_step<M, H>(S, a, i, lane);
+	// --- 1. tridiagonalisation: step i touches the columns below i only ----------
+	psd_tridiagonalise<M, M>(S, a, lane);
 	double *V = S.V;
 	double dj = 0.0;
 #pragma unroll
@@ -1576,6 +1612,7 @@ __device__ __forceinline__ void psd_element(PsdWarp<EL> &S, T *__restrict__ stag
 	}
 	__syncwarp();
 
+	psd_phase<M>();
 	// --- 2./3. scale; count below -tau, then multisection ------------------------
 	const double ej = lane < M ? S.en[lane] : 0.0;
 	const double ej1 = lane + 1 < M ? S.en[lane + 1] : 0.0;
@@ -1592,22 +1629,33 @@ __device__ __forceinline__ void psd_element(PsdWarp<EL> &S, T *__restrict__ stag
 	__syncwarp();
 	// iteration -1 counts the eigenvalues below -tau on every lane; later
 	// iterations: 32 / k lanes per eigenvalue j < k, each at an interior point of
-	// the eigenvalue's interval [lo, hi) (count(lo) <= j < count(hi))
+	// the eigenvalue's interval [lo, hi) (count(lo) <= j < count(hi)).  The points are
+	// evenly spread until the last minors' ratio is known at both ends and changes sign;
+	// then they close in on its secant's root r from both sides, r -+ w 2^-e with e from 3
+	// outside to 17 inside, as long as a round gains more than the even points would.
 	int k = 0, G = 1, jg = 0;
-	bool act = false;
+	bool act = false, secant = true;
+	constexpr bool SECANT = M > 12; // P2 24^3 2,865 -> 2,794 us; P1 36^3 loses, 1,942 -> 1,958
 	unsigned gmask = 0u;
-	double frac = 0.0, lo = -1.0 - 1e-3, hi = -psd_tau<T>(), x = hi;
+	double even = 0.0, near = 0.0, lo = -1.0 - 1e-3, hi = -psd_tau<T>(), flo = 0.0, fhi = 0.0, x = hi;
 #pragma unroll 1
 	for (int it = -1; it < PSD_MAX_BISECT; ++it)
 	{
-		bool done = true;
+		bool done = true, pred = false;
 		if (it >= 0)
 		{
 			done = !act || hi - lo <= PSD_WIDTH;
 			if (__all_sync(FULL, done)) break;
-			x = fma(hi - lo, frac, lo);
+			x = fma(hi - lo, even, lo);
+			pred = SECANT && secant && G >= 4 && flo > 0.0 && fhi < 0.0;
+			if (SECANT && pred)
+			{
+				const double r = lo + (hi - lo) * (flo / (flo - fhi));
+				x = fmin(fmax(fma(hi - lo, near, r), lo), hi);
+			}
 		}
-		const int c = sturm_count<M>(S.de2, x);
+		double f = 0.0;
+		const int c = sturm_count<M, SECANT>(S.de2, x, f);
 		if (it < 0)
 		{
 			k = c;
@@ -1616,24 +1664,43 @@ __device__ __forceinline__ void psd_element(PsdWarp<EL> &S, T *__restrict__ stag
 			jg = lane / G;
 			act = jg < k;
 			gmask = G == 32 ? FULL : ((1u << G) - 1u);
-			frac = double(lane - jg * G + 1) / double(G + 1);
+			const int t = lane - jg * G, half = G / 2;
+			even = double(t + 1) / double(G + 1);
+			// lanes outside in: exponents 3 .. 17; the middle lane of an odd group at r itself
+			const int out = t < half ? t : G - 1 - t;
+			near = out >= half ? 0.0 : exp2(-3.0 - 14.0 * double(out) / double(half > 1 ? half - 1 : 1));
+			if (t < half) near = -near;
+			fhi = f; // the ratio at -tau: every interval's right end
 			continue;
 		}
 		const unsigned bal = __ballot_sync(FULL, c <= jg);
 		const unsigned mg = act ? (bal >> (jg * G)) & gmask : 0u;
 		// first point of the group with more than jg eigenvalues below it
 		const int tf = mg == gmask ? G : __ffs(~mg) - 1;
-		const double xlo = __shfl_sync(FULL, x, (jg * G + tf - 1) & 31);
-		const double xhi = __shfl_sync(FULL, x, (jg * G + tf) & 31);
+		const int la = (jg * G + tf - 1) & 31, lb = (jg * G + tf) & 31;
+		const double xlo = __shfl_sync(FULL, x, la), xhi = __shfl_sync(FULL, x, lb);
+		const double glo = SECANT ? __shfl_sync(FULL, f, la) : 0.0, ghi = SECANT ? __shfl_sync(FULL, f, lb) : 0.0;
 		if (!done)
 		{
-			if (tf > 0) lo = xlo;
-			if (tf < G) hi = xhi;
+			const double w = hi - lo;
+			if (tf > 0)
+			{
+				lo = xlo;
+				flo = glo;
+			}
+			if (tf < G)
+			{
+				hi = xhi;
+				fhi = ghi;
+			}
+			// a secant round that kept more than an even one would: even points next
+			secant = !pred || (hi - lo) * double(G + 1) <= w;
 		}
 	}
 	const bool vec = lane < k;
 	const double sig = __shfl_sync(FULL, 0.5 * (lo + hi), (lane * G) & 31);
 
+	psd_phase<M>();
 	// --- 4. inverse iteration, lane j -> eigenvector j ---------------------------
 	double y[M];
 #pragma unroll
@@ -1728,11 +1795,9 @@ __device__ __forceinline__ void psd_element(PsdWarp<EL> &S, T *__restrict__ stag
 	}
 	if (__any_sync(FULL, bad)) return;
 
+	psd_phase<M>();
 	// --- 5. back-transform x = P_2 ... P_{M-1} y (reflector 2 first), w = sqrt|l| x
-#pragma unroll 1
-	for (int i = 2; i <= H; ++i) psd_reflect<M, H>(S, y, i);
-#pragma unroll 1
-	for (int i = H + 1; i < M; ++i) psd_reflect<M, M>(S, y, i);
+	psd_back_transform<M, M>(S, y);
 	__syncwarp();
 	if (vec)
 	{
@@ -1778,8 +1843,8 @@ __device__ __forceinline__ void psd_element(PsdWarp<EL> &S, T *__restrict__ stag
 // is left, so a warp whose element is already PSD, or has few negative eigenvalues,
 // goes on to the next one instead of idling until the other warps of its CTA
 // finish (P1 48^3: 5.51 -> 4.97 ms).  The larger P2 and Q1 kernels run one element
-// per warp: persistent warps drift apart in phase and were slower there (P2 40^3
-// 16.3 -> 17.6 ms).  Each element's arithmetic does not depend on which warp
+// per warp: persistent warps drift apart in phase, which costs them instruction fetches
+// (psd_phase; P2 40^3 16.3 -> 17.6 ms).  Each element's arithmetic does not depend on which warp
 // projects it.
 template <class EL>
 __host__ __device__ constexpr bool psd_persistent() { return EL::ET == 1; }
