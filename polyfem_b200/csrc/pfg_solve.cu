@@ -18,10 +18,10 @@
 //   iterations = i, relative residual = sqrt(|r|^2 / rhs2)
 // with D^-1 = 1 / diag(H) where the diagonal is non-zero, else 1.
 // One persistent cooperative kernel (k_cg) runs the iterations: the matrix streams
-// through a ring of shared-memory stages filled by bulk copies, the vectors live in
-// 32-byte slots of one node each (its up to three free dofs, zero-padded), and three
-// grid barriers per iteration separate H p with p.q, the step with r.r and r.z, and the
-// new direction.  Every CTA forms the scalars from the same partials in the same order,
+// through each warp's shared-memory stages, filled by bulk copies, the vectors live in
+// 32-byte slots of one node each (its up to three free dofs, zero-padded), and two or
+// three grid-wide exchanges per iteration separate H p with p.q, the step with r.r and
+// r.z, and the new direction.  Every CTA forms the scalars from the same partials in the same order,
 // so the stop test needs no host; the host reads the state once per batch.
 //
 // H is structurally and numerically symmetric (the reduction sums both triangles of

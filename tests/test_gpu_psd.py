@@ -90,3 +90,21 @@ def test_projection_keeps_nan_of_inverted_elements(require_gpu):
     assert np.isnan(plain).any()
     assert np.array_equal(np.isnan(plain), np.isnan(proj))
     asm.close()
+
+
+@pytest.mark.parametrize("count", [1, 3, 5, 130])
+@pytest.mark.parametrize("et,g", [(M.P2_TET, 3), (M.Q1_HEX, 6)], ids=["P2", "Q1"])
+def test_projection_of_mixed_blocks(require_gpu, et, g, count):
+    """The element matrices of a block go through the projection's phases together: elements
+    at rest beside ones of several negative eigenvalues, and element counts that leave the
+    last block's warps without an element.  Bound: the projection's own, 1e-11."""
+    mesh, lam, mu, _, _ = make_case(et, g, seed=3, jitter=0.1)
+    mesh.conn = np.ascontiguousarray(mesh.conn[:count])
+    mesh.gconn = mesh.conn if et == M.Q1_HEX else np.ascontiguousarray(mesh.gconn[:count])
+    rng = np.random.default_rng(17)
+    stretch = 0.3 * (mesh.node_pos[:, 0] < 0.5)[:, None]
+    u = (-stretch * mesh.node_pos + 0.1 * stretch * mesh.h * rng.standard_normal(mesh.node_pos.shape)).ravel()
+    _, _, v_psd = Oracle(mesh, lam[:count], mu[:count]).hessian(u, project_psd=True)
+    asm = NeoHookeanAssembler.from_mesh(mesh, lam[:count], mu[:count])
+    assert rel_err(asm.assemble_hessian_values(u, "fp64", project_to_psd=True), v_psd) <= 1e-11
+    asm.close()
