@@ -264,8 +264,11 @@ __global__ void __launch_bounds__(CG_NT) k_cg_unpack(int ngroups, const int *__r
 // P2 24^3 is 41 us of streaming (240 MB, half of it from L2), the products that do not
 // overlap it, and 4 us an exchange; at P1 13^3 two exchanges and the chains behind them.
 constexpr int CG_W = 16, CG_CTA = 32 * CG_W;
-constexpr int CG_COST = 640;              // doubles of values a stage holds
-constexpr int CG_BLOB = 300;              // ints of a chunk's descriptors and codes
+// doubles of values a stage holds: three whole groups of 27 3 x 3 blocks, an inner node of a
+// hexahedral mesh (640 values, two of them: Q1 64^3 / 96^3 181 / 622 us an iteration, 169 / 543
+// with three; P2 24^3 80.4, 78.9)
+constexpr int CG_COST = 736;
+constexpr int CG_BLOB = 180;              // ints of a chunk's descriptors and codes
 constexpr int CG_SPIN = 1 << 22;          // bound of every wait
 constexpr int CG_PK = 5, CG_MAX_CTAS = 32 * CG_PK; // packets per lane of an exchange; CTAs
 constexpr int CG_OWN = 256;               // own groups whose q (and, FUSED, p) stay in shared memory
@@ -277,7 +280,7 @@ struct __align__(16) CgStage
 	double v[CG_COST + 2]; // + 2: the copy starts on the 16-byte boundary below
 	int4 blob[CG_BLOB / 4];
 };
-struct CgSmem // 220 KB
+struct CgSmem // 224 KB
 {
 	CgStage st[CG_W][2];
 	unsigned long long full[CG_W][2];
