@@ -473,7 +473,7 @@ int build_pattern(pfg_context *c)
 
 	PFG_CUDA(c, cudaMalloc(&c->d_outer, sizeof(int) * (ndof + 1)));
 	PFG_CUDA(c, cudaMalloc(&c->d_inner, sizeof(int) * std::max<long long>(nnz, 1)));
-	PFG_CUDA(c, cudaMalloc(&c->d_values, sizeof(double) * std::max<long long>(nnz, 1)));
+	PFG_CUDA(c, cudaMalloc(&c->d_values, sizeof(double) * (nnz + 1))); // + 1: pfg_cg_solve reads whole 16-byte units
 	PFG_CUDA(c, cudaMalloc(&c->d_contrib, sizeof(unsigned int) * std::max<size_t>(contrib.size(), 1)));
 	PFG_CUDA(c, cudaMalloc(&c->d_blk_rel, sizeof(unsigned short) * std::max<size_t>(blk_rel.size(), 1)));
 	PFG_CUDA(c, cudaMemcpy(c->d_outer, outer.data(), sizeof(int) * (ndof + 1), cudaMemcpyHostToDevice));
@@ -620,7 +620,7 @@ int build_dirichlet(pfg_context *c)
 	PFG_CUDA(c, cudaMalloc(&c->d_red_outer, sizeof(int) * (n_free + 1)));
 	PFG_CUDA(c, cudaMalloc(&c->d_red_inner, sizeof(int) * std::max<long long>(pos, 1)));
 	PFG_CUDA(c, cudaMalloc(&c->d_red_row_off, sizeof(unsigned short) * std::max<size_t>(row_off.size(), 1)));
-	PFG_CUDA(c, cudaMalloc(&c->d_red_values, sizeof(double) * std::max<long long>(pos, 1)));
+	PFG_CUDA(c, cudaMalloc(&c->d_red_values, sizeof(double) * (pos + 1))); // + 1: as d_values
 	PFG_CUDA(c, cudaMemcpy(c->d_old_to_new, old_to_new.data(), sizeof(int) * ndof, cudaMemcpyHostToDevice));
 	if (n_free) PFG_CUDA(c, cudaMemcpy(c->d_free, freev.data(), sizeof(int) * n_free, cudaMemcpyHostToDevice));
 	PFG_CUDA(c, cudaMemcpy(c->d_red_col_start, col_start.data(), sizeof(int) * ndof, cudaMemcpyHostToDevice));
@@ -1605,7 +1605,7 @@ int pfg_cg_solve(pfg_context *c, int system, const double *values, const double 
 		for (;;)
 		{
 			const int k = std::min(CG_BATCH, max_iter - queued);
-			if (k > 0) PFG_CUDA(c, launch_cg_iterations(k, plan, vals, w, c->d_err, c->stream));
+			if (k > 0) PFG_CUDA(c, launch_cg_iterations(k, plan, vals, values == nullptr, w, c->d_err, c->stream));
 			queued += std::max(k, 0);
 			if ((st = read_scalars())) return st;
 			if (c->h_cg_sc[CG_DONE] != 0.0 || queued >= max_iter) break;

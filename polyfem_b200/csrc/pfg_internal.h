@@ -222,14 +222,14 @@ struct CgWork
 // of k_cg holds (chunk: blob, its size, first value, values or 0 for one group too large to
 // stage; blob: descriptors and neighbour codes; big: the codes of those large groups), every
 // warp's run of chunks with its first group, and the count of grid exchanges (16 bytes)
-// followed by three arrays of 32-byte packets per CTA
+// followed by three arrays of 32-byte packets per CTA; the counts of values and chunks
 struct CgPlan
 {
 	int2 *run = nullptr;
 	int4 *chunk = nullptr, *blob = nullptr;
 	const int *big = nullptr;
 	unsigned *bar = nullptr;
-	int ctas = 0;
+	int ctas = 0, nnz = 0, chunks = 0;
 	bool resident = false; // every run is at most two chunks
 };
 cudaError_t build_cg_plan(int n, int ngroups, const int *groups, const int *outer, const int *inner, CgPlan *pl, cudaStream_t s);
@@ -251,8 +251,10 @@ cudaError_t launch_cg_start(int n, int ngroups, const int *groups, const int *ou
 							const double *vals, const double *b, bool guess, double tol, const double *x, const CgWork &w,
 							cudaStream_t s);
 // `count` iterations unless done: q = H p, alpha, x += alpha p, r -= alpha q, stop
-// test, z = D^-1 r, beta, p = z + beta p, iteration count + 1; *err: a wait gave up
-cudaError_t launch_cg_iterations(int count, const CgPlan &pl, const double *vals, const CgWork &w, int *err, cudaStream_t s);
+// test, z = D^-1 r, beta, p = z + beta p, iteration count + 1; *err: a wait gave up.
+// padded: an odd count of values has one readable double behind it
+cudaError_t launch_cg_iterations(int count, const CgPlan &pl, const double *vals, bool padded, const CgWork &w, int *err,
+								 cudaStream_t s);
 // the slots of x -> the dense x
 cudaError_t launch_cg_unpack(int ngroups, const int *groups, const CgWork &w, double *x, cudaStream_t s);
 

@@ -29,6 +29,7 @@
 // q = H p is a gather: one warp per node's columns, no atomics.  Every dot product is a
 // fixed-order reduction (warp butterfly, warps in order, CTAs in order), so the
 // iterates are bitwise deterministic.
+#include "pfg_bulk_span.h"
 #include "pfg_internal.h"
 
 #include <algorithm>
@@ -277,7 +278,7 @@ constexpr int CG_OWN = 256;               // own groups whose q (and, FUSED, p) 
 // with an end entry, the codes (neighbour group * 4 + its dofs)
 struct __align__(16) CgStage
 {
-	double v[CG_COST + 2]; // + 2: the copy starts on the 16-byte boundary below
+	double v[CG_COST + 2]; // + 2: the copies move whole 16-byte units (bulk_span)
 	int4 blob[CG_BLOB / 4];
 };
 struct CgSmem // 224 KB
@@ -513,9 +514,12 @@ __device__ __forceinline__ void group_products(const double *sv, const int *blob
 	}
 }
 
+// EDGE: the array of values does not end on 16-byte units; the warps that own its first and
+// last chunk clip their copies.  A variant, because the test alone costs the streaming kernel
+// 0.7% (P2 24^3 79.3 -> 79.9 us an iteration); a resident run copies once, and always tests.
 // FUSED (all runs resident): the new direction z + beta p_old is formed where H p gathers
 // it, which reads two slots per block but saves the third exchange of an iteration.
-template <bool FUSED>
+template <bool FUSED, bool EDGE>
 __global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals, CgWork w, int iters, int *err)
 {
 	extern __shared__ __align__(16) unsigned char cg_raw[];
@@ -537,6 +541,7 @@ __global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals,
 	const int ch0 = run[warp].x, nch = run[warp + 1].x - ch0;
 	const int g0 = run[0].y, nown = run[CG_W].y - g0;
 	const bool resident = nch <= 2;
+	const bool edge = EDGE && ((blockIdx.x == 0 && warp == 0) || ch0 + nch == pl.chunks);
 	__syncthreads();
 	// the chunks' entries (blob in 16-byte units, its size in them, first value, values; no
 	// values: too large to stage), 32 at a time, a lane each
@@ -559,11 +564,22 @@ __global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals,
 			unsigned long long *full = &S.full[warp][st];
 			const double *v = vals + v0;
 			const int mv = (int)(((size_t)v >> 3) & 1);
-			const unsigned bv = nv ? (unsigned)((nv + mv + 1) / 2) * 16u : 0u;
+			unsigned bv = nv ? (unsigned)((nv + mv + 1) / 2) * 16u : 0u;
+			const double *src = v - mv;
+			double *dst = T.v;
+			if (EDGE && edge) // see bulk_span
+			{
+				const BulkSpan sp = bulk_span(v0, nv, pl.nnz, mv);
+				if (sp.lo) T.v[mv] = __ldg(v);
+				if (sp.hi) T.v[mv + nv - 1] = __ldg(v + nv - 1);
+				bv = (unsigned)(sp.end - sp.begin) * 8u;
+				src = v + sp.begin;
+				dst = T.v + mv + sp.begin;
+			}
 			asm volatile("mbarrier.arrive.expect_tx.release.cta.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(full)),
 						 "r"(bv + (unsigned)bn * 16u)
 						 : "memory");
-			if (bv) bulk_load(T.v, v - mv, bv, full);
+			if (bv) bulk_load(dst, src, bv, full);
 			bulk_load(T.blob, pl.blob + b0, (unsigned)bn * 16u, full);
 		}
 		return make_int2(v0, nv);
@@ -861,6 +877,8 @@ cudaError_t build_cg_plan(int n, int ngroups, const int *groups, const int *oute
 		close();
 		while ((int)run.size() <= warps) run.push_back(make_int2((int)chunk.size(), ngroups));
 		pl->ctas = ctas;
+		pl->nnz = ho[n];
+		pl->chunks = (int)chunk.size();
 		pl->resident = true;
 		for (int i = 0; i < warps; ++i) pl->resident = pl->resident && run[i + 1].x - run[i].x <= 2;
 		// the overflow codes sit behind the blobs
@@ -914,10 +932,12 @@ cudaError_t launch_cg_start(int n, int ngroups, const int *groups, const int *ou
 	return cudaGetLastError();
 }
 
-cudaError_t launch_cg_iterations(int count, const CgPlan &pl, const double *vals, const CgWork &w, int *err, cudaStream_t s)
+cudaError_t launch_cg_iterations(int count, const CgPlan &pl, const double *vals, bool padded, const CgWork &w, int *err,
+								 cudaStream_t s)
 {
+	const bool edge = ((size_t)vals & 15) || ((pl.nnz & 1) && !padded);
 	// resident runs: the matrix's latency is gone and the exchanges are the cost
-	const void *kernel = pl.resident ? (const void *)k_cg<true> : (const void *)k_cg<false>;
+	const void *kernel = pl.resident ? (const void *)k_cg<true, true> : edge ? (const void *)k_cg<false, true> : (const void *)k_cg<false, false>;
 	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CgSmem));
 	if (e != cudaSuccess) return e;
 	CgPlan p = pl;

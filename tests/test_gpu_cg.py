@@ -199,3 +199,26 @@ def test_group_sizes_and_partly_fixed_nodes(require_gpu, case):
     assert abs(cg.get_info()["solver_iter"] - it_o) <= max(2, it_o // 20)
     assert np.array_equal(cg.solve(b), x)
     asm.close()
+
+
+@pytest.mark.parametrize("et,g", [(M.P1_TET, 1), (M.P1_TET, 4), (M.P2_TET, 13)], ids=["one chunk", "resident", "streaming"])
+@pytest.mark.parametrize("n_fixed", [9, 10])
+def test_values_at_any_alignment(require_gpu, et, g, n_fixed):
+    """Values that begin on 8 bytes, with even and odd counts (the bulk copies move 16-byte
+    units): the same bits as from an aligned array."""
+    import torch
+    mesh, lam, mu, u, _ = make_case(et, g, seed=5)
+    asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
+    asm.set_dirichlet(np.arange(n_fixed))
+    v = asm.assemble_hessian_reduced_values(torch.tensor(u, device="cuda"), project_to_psd=True)
+    b = torch.tensor(np.random.default_rng(2).standard_normal(asm.n_free), device="cuda")
+    cg = ConjugateGradient(asm, "reduced")
+    cg.set_parameters({"tolerance": 1e-10, "max_iter": 300})
+    cg.factorize(v)
+    x = cg.solve(b)
+    assert torch.isfinite(x).all() and bool(x.abs().max() > 0)
+    shifted = torch.full((v.numel() + 1,), float("nan"), dtype=torch.float64, device="cuda")
+    shifted[1:] = v
+    cg.factorize(shifted[1:])
+    assert torch.equal(cg.solve(b), x)
+    asm.close()
