@@ -18,6 +18,7 @@ ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 PFG_OK = 0
 PFG_ERR_INVALID = 1
+PFG_ERR_CUDA = 2
 PFG_ERR_OOM = 3
 PFG_ERR_STATE = 5
 PFG_ERR_NUMERIC = 6

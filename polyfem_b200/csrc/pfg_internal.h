@@ -209,7 +209,8 @@ enum
 	CG_THR = 5,   // stopping threshold on |r|^2
 	CG_DONE = 6,  // 1 once |r|^2 < threshold, 2 when a bounded wait gave up: later launches return at once
 	CG_ITER = 7,  // iterations counted as Eigen counts them (not the one that stopped)
-	CG_NSC = 8
+	CG_ERR = 8,   // an int: set by any CTA whose bounded wait gave up (CTA 0, which writes the others, need not be it)
+	CG_NSC = 9
 };
 // Vectors in slots of four doubles per column group (the group's up to three dofs, zeros
 // behind); dense: 2 n doubles of set-up scratch
@@ -221,14 +222,15 @@ struct CgWork
 // Static plan of a system's pattern, built once: the groups in chunks that a warp's stage
 // of k_cg holds (chunk: blob, its size, first value, values or 0 for one group too large to
 // stage; blob: descriptors and neighbour codes; big: the codes of those large groups), every
-// warp's run of chunks with its first group, and the count of grid exchanges (16 bytes)
-// followed by three arrays of 32-byte packets per CTA; the counts of values and chunks
+// warp's run of chunks with its first group, three arrays of 32-byte packets per CTA, the
+// exchange numbers handed out so far; the counts of values and chunks
 struct CgPlan
 {
 	int2 *run = nullptr;
 	int4 *chunk = nullptr, *blob = nullptr;
 	const int *big = nullptr;
-	unsigned *bar = nullptr;
+	uint4 *packets = nullptr;
+	unsigned gen = 0;
 	int ctas = 0, nnz = 0, chunks = 0;
 	bool resident = false; // every run is at most two chunks
 };
@@ -251,10 +253,11 @@ cudaError_t launch_cg_start(int n, int ngroups, const int *groups, const int *ou
 							const double *vals, const double *b, bool guess, double tol, const double *x, const CgWork &w,
 							cudaStream_t s);
 // `count` iterations unless done: q = H p, alpha, x += alpha p, r -= alpha q, stop
-// test, z = D^-1 r, beta, p = z + beta p, iteration count + 1; *err: a wait gave up.
-// padded: an odd count of values has one readable double behind it
-cudaError_t launch_cg_iterations(int count, const CgPlan &pl, const double *vals, bool padded, const CgWork &w, int *err,
-								 cudaStream_t s);
+// test, z = D^-1 r, beta, p = z + beta p, iteration count + 1.
+// padded: an odd count of values has one readable double behind it; missing: CTAs left out of
+// the launch (the give-up test's way to have a wait run out)
+cudaError_t launch_cg_iterations(int count, CgPlan &pl, const double *vals, bool padded, const CgWork &w, cudaStream_t s,
+								 int missing = 0);
 // the slots of x -> the dense x
 cudaError_t launch_cg_unpack(int ngroups, const int *groups, const CgWork &w, double *x, cudaStream_t s);
 

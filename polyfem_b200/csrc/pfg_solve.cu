@@ -234,6 +234,7 @@ __global__ void __launch_bounds__(CG_NT) k_cg_start_scalars(const double *__rest
 	sc[CG_THR] = thr;
 	sc[CG_DONE] = (s[2] == 0.0 || s[1] < thr) ? 1.0 : 0.0;
 	sc[CG_ITER] = 0.0;
+	sc[CG_ERR] = 0.0;
 }
 
 __global__ void __launch_bounds__(CG_NT) k_cg_unpack(int ngroups, const int *__restrict__ groups,
@@ -270,7 +271,7 @@ constexpr int CG_W = 16, CG_CTA = 32 * CG_W;
 // with three; P2 24^3 80.4, 78.9)
 constexpr int CG_COST = 736;
 constexpr int CG_BLOB = 180;              // ints of a chunk's descriptors and codes
-constexpr int CG_SPIN = 1 << 22;          // bound of every wait
+constexpr int CG_SPIN = 1 << 20;          // bound of every wait (an exchange: about a second)
 constexpr int CG_PK = 5, CG_MAX_CTAS = 32 * CG_PK; // packets per lane of an exchange; CTAs
 constexpr int CG_OWN = 256;               // own groups whose q (and, FUSED, p) stay in shared memory
 // a chunk's blob: head (first group, groups, -, -), a descriptor per group (first column * 4 +
@@ -341,7 +342,9 @@ __device__ __forceinline__ double warp_sum3(const double (&s)[3])
 // counter, a generation word and the partials.  DATA: what the CTAs wrote before the
 // exchange is visible to all after it (the two fences, ~1 us; only needed where others'
 // vector entries are read next).  Three packet arrays in turn: a CTA can only overwrite
-// one after all have read it.  Bounded: false once any wait has given up.
+// one after all have read it.  Bounded: false once any wait has given up.  A CTA that gives up
+// can leave others an exchange ahead, so every launch has numbers of its own (CgPlan::gen): the
+// packets such a launch leaves behind match nothing later.
 struct Sums
 {
 	double a, b;
@@ -353,9 +356,9 @@ __device__ __forceinline__ uint4 ld_packet(const uint4 *p)
 	return v;
 }
 template <int NV, bool DATA>
-__device__ __forceinline__ bool exchange(CgSmem &S, uint4 *pk, unsigned gen, double a, double b, int *err, Sums &out)
+__device__ __forceinline__ bool exchange(CgSmem &S, uint4 *pk, int G, unsigned gen, double a, double b, int *err, Sums &out)
 {
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, G = gridDim.x;
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	if (NV > 1)
 		warp_sum2(a, b, S.red[0] + warp, S.red[1] + warp);
 	else if (NV > 0)
@@ -520,12 +523,13 @@ __device__ __forceinline__ void group_products(const double *sv, const int *blob
 // FUSED (all runs resident): the new direction z + beta p_old is formed where H p gathers
 // it, which reads two slots per block but saves the third exchange of an iteration.
 template <bool FUSED, bool EDGE>
-__global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals, CgWork w, int iters, int *err)
+__global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals, CgWork w, int iters)
 {
 	extern __shared__ __align__(16) unsigned char cg_raw[];
 	CgSmem &S = *reinterpret_cast<CgSmem *>(cg_raw);
 	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 	double *sc = w.sc;
+	int *err = reinterpret_cast<int *>(sc + CG_ERR);
 	if (sc[CG_DONE] != 0.0) return; // the same for every CTA: written before this launch
 	const int it0 = (int)sc[CG_ITER];
 	if (tid == 0)
@@ -587,10 +591,36 @@ __global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals,
 	int2 vq[2] = {make_int2(0, 0), make_int2(0, 0)}; // first value and count of the chunk in each stage
 	const auto back = [&](int it) { return !resident && ((it0 + it) & 1); };
 	for (int i = 0; i < min(nch, 2); ++i) vq[i] = request(back(0) ? nch - 1 - i : i);
-	const int G = gridDim.x;
+	// the next chunk requested is here; false: gave up, nothing more is taken or requested
+	const auto take = [&]() {
+		const int st = used & 1;
+		bool here = false;
+		for (int spin = 0; !here && spin < CG_SPIN; ++spin) here = mbar_test(&S.full[warp][st], par[st]);
+		here = __all_sync(0xffffffffu, here);
+		if (here)
+		{
+			par[st] ^= 1u;
+			++used;
+		}
+		else if (lane == 0)
+		{
+			atomicExch(err, 1);
+			S.stop = 1;
+		}
+		return here;
+	};
+	int own_chunks = nch; // to multiply: none when a resident one did not come
+	if (resident)
+		while (used < load)
+			if (!take())
+			{
+				own_chunks = 0;
+				break;
+			}
+	const int G = pl.ctas;
 	double *q = nown <= CG_OWN ? S.q : w.q + 4 * (size_t)g0, *po = S.p;
-	unsigned gen = *(volatile unsigned *)pl.bar; // exchanges so far, of all launches
-	uint4 *pk = reinterpret_cast<uint4 *>(pl.bar + 4);
+	unsigned gen = pl.gen; // exchange numbers given to earlier launches
+	uint4 *pk = pl.packets + 1; // 16 bytes off the 32-byte sectors: P1 13^3 12.8 us an iteration, 13.1 on them
 	const double thr = sc[CG_THR];
 	double rz = sc[CG_RZ], rr = sc[CG_RR], alpha = 0.0, beta = it0 ? sc[CG_BETA] : 0.0;
 	bool done = false, ok = true;
@@ -625,19 +655,10 @@ __global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals,
 			}
 			pq = fma(pv, qc, pq);
 		};
-		for (int i = 0; i < nch; ++i)
+		for (int i = 0; i < own_chunks; ++i)
 		{
-			const int st = resident ? i : used++ & 1;
-			if (!resident || it == 0)
-			{
-				for (int spin = 0; !mbar_test(&S.full[warp][st], par[st]) && spin < CG_SPIN; ++spin)
-					if (spin == CG_SPIN - 1)
-					{
-						atomicExch(err, 1);
-						S.stop = 1;
-					}
-				par[st] ^= 1u;
-			}
+			const int st = resident ? i : used & 1;
+			if (!resident && !take()) break;
 			const CgStage &T = S.st[warp][st];
 			const int *blob = reinterpret_cast<const int *>(T.blob);
 			const int4 head = T.blob[0];
@@ -692,7 +713,7 @@ __global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals,
 			}
 		}
 		Sums sum;
-		if (!(ok = exchange<1, false>(S, pk, ++gen, pq, 0.0, err, sum))) break;
+		if (!(ok = exchange<1, false>(S, pk, G, ++gen, pq, 0.0, err, sum))) break;
 		alpha = rz / sum.a;
 		// x += alpha p, r -= alpha q, z = D^-1 r
 		const double *pown = FUSED && nown <= CG_OWN ? po : pout + 4 * (size_t)g0;
@@ -719,7 +740,7 @@ __global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals,
 				srz = fma(r.y, z.y, fma(r.x, z.x, srz));
 			}
 		}
-		if (!(ok = exchange<2, FUSED>(S, pk + 2 * G, ++gen, srr, srz, err, sum))) break;
+		if (!(ok = exchange<2, FUSED>(S, pk + 2 * G, G, ++gen, srr, srz, err, sum))) break;
 		rr = sum.a;
 		if (rr < thr)
 		{
@@ -743,21 +764,19 @@ __global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals,
 					*reinterpret_cast<double2 *>(w.p + o + h) = p;
 				}
 			}
-			if (!(ok = exchange<0, true>(S, pk + 4 * G, ++gen, 0.0, 0.0, err, sum))) break;
+			if (!(ok = exchange<0, true>(S, pk + 4 * G, G, ++gen, 0.0, 0.0, err, sum))) break;
 		}
 	}
-	// copies still in flight (a run that stopped early): wait for them before leaving
-	if (!resident)
-		for (; used < load; ++used)
-		{
-			const int st = used & 1;
-			for (int spin = 0; spin < CG_SPIN && !mbar_test(&S.full[warp][st], par[st]); ++spin)
-				;
-			par[st] ^= 1u;
-		}
+	// copies still in flight (the solve stopped, or a wait gave up): wait for them before leaving
+	for (; used < load; ++used)
+	{
+		const int st = used & 1;
+		for (int spin = 0; spin < CG_SPIN && !mbar_test(&S.full[warp][st], par[st]); ++spin)
+			;
+		par[st] ^= 1u;
+	}
 	if (tid == 0 && blockIdx.x == 0)
 	{
-		*pl.bar = gen;
 		sc[CG_ALPHA] = alpha;
 		sc[CG_BETA] = beta;
 		sc[CG_RZ] = rz;
@@ -886,12 +905,13 @@ cudaError_t build_cg_plan(int n, int ngroups, const int *groups, const int *oute
 		for (long long &x : at)
 			if (x < 0) x = big0 + (-1 - x);
 		blob.resize(blob.size() + (size_t)(nbig + 3) / 4);
-		const size_t bar_bytes = 16 + 96 * (size_t)ctas;
+		const size_t packet_bytes = 16 + 96 * (size_t)ctas;
 		if ((e = cudaMalloc(&pl->run, sizeof(int2) * run.size())) == cudaSuccess &&
 			(e = cudaMalloc(&pl->chunk, sizeof(int4) * chunk.size())) == cudaSuccess &&
 			(e = cudaMalloc(&pl->blob, sizeof(int4) * blob.size())) == cudaSuccess &&
 			(e = cudaMalloc(&d_at, sizeof(long long) * at.size())) == cudaSuccess &&
-			(e = cudaMalloc(&pl->bar, bar_bytes)) == cudaSuccess && (e = cudaMemsetAsync(pl->bar, 0, bar_bytes, s)) == cudaSuccess &&
+			(e = cudaMalloc(&pl->packets, packet_bytes)) == cudaSuccess &&
+			(e = cudaMemsetAsync(pl->packets, 0, packet_bytes, s)) == cudaSuccess &&
 			(e = cudaMemcpyAsync(pl->run, run.data(), sizeof(int2) * run.size(), cudaMemcpyHostToDevice, s)) == cudaSuccess &&
 			(e = cudaMemcpyAsync(pl->chunk, chunk.data(), sizeof(int4) * chunk.size(), cudaMemcpyHostToDevice, s)) == cudaSuccess &&
 			(e = cudaMemcpyAsync(pl->blob, blob.data(), sizeof(int4) * blob.size(), cudaMemcpyHostToDevice, s)) == cudaSuccess &&
@@ -911,7 +931,7 @@ cudaError_t build_cg_plan(int n, int ngroups, const int *groups, const int *oute
 
 void free_cg_plan(CgPlan *pl)
 {
-	void *ptrs[] = {pl->run, pl->chunk, pl->blob, pl->bar};
+	void *ptrs[] = {pl->run, pl->chunk, pl->blob, pl->packets};
 	for (void *p : ptrs)
 		if (p) cudaFree(p);
 	*pl = CgPlan();
@@ -932,8 +952,8 @@ cudaError_t launch_cg_start(int n, int ngroups, const int *groups, const int *ou
 	return cudaGetLastError();
 }
 
-cudaError_t launch_cg_iterations(int count, const CgPlan &pl, const double *vals, bool padded, const CgWork &w, int *err,
-								 cudaStream_t s)
+cudaError_t launch_cg_iterations(int count, CgPlan &pl, const double *vals, bool padded, const CgWork &w, cudaStream_t s,
+								 int missing)
 {
 	const bool edge = ((size_t)vals & 15) || ((pl.nnz & 1) && !padded);
 	// resident runs: the matrix's latency is gone and the exchanges are the cost
@@ -941,9 +961,10 @@ cudaError_t launch_cg_iterations(int count, const CgPlan &pl, const double *vals
 	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CgSmem));
 	if (e != cudaSuccess) return e;
 	CgPlan p = pl;
+	pl.gen += 3u * (unsigned)count; // at most three exchanges an iteration
 	CgWork ww = w;
-	void *args[] = {&p, &vals, &ww, &count, &err};
-	return cudaLaunchCooperativeKernel(kernel, dim3(pl.ctas), dim3(CG_CTA), args, sizeof(CgSmem), s);
+	void *args[] = {&p, &vals, &ww, &count};
+	return cudaLaunchCooperativeKernel(kernel, dim3(pl.ctas - missing), dim3(CG_CTA), args, sizeof(CgSmem), s);
 }
 
 cudaError_t launch_cg_unpack(int ngroups, const int *groups, const CgWork &w, double *x, cudaStream_t s)

@@ -13,7 +13,7 @@ import scipy.sparse.linalg as spla
 from oracle.binding import conjugate_gradient
 from polyfem_b200 import ConjugateGradient, NeoHookeanAssembler, PfgError
 from polyfem_b200 import mesh as M
-from polyfem_b200._lib import PFG_MEM_HOST, lib
+from polyfem_b200._lib import PFG_ERR_CUDA, PFG_MEM_HOST, lib
 
 from _cases import make_case, rel_err
 
@@ -221,4 +221,32 @@ def test_values_at_any_alignment(require_gpu, et, g, n_fixed):
     shifted[1:] = v
     cg.factorize(shifted[1:])
     assert torch.equal(cg.solve(b), x)
+    asm.close()
+
+
+@pytest.mark.parametrize("et,g", [(M.P1_TET, 8), (M.P2_TET, 13)], ids=["resident", "streaming"])
+@pytest.mark.parametrize("mem", ["host", "device"])
+def test_a_wait_that_gave_up_is_reported_and_leaves_nothing_behind(require_gpu, et, g, mem):
+    """A solve whose grid waits for a CTA that never comes ends with an error, and so does one
+    in which a CTA other than the first gave up, whatever state the first one left; the solves
+    after it return the bits of the one before."""
+    import torch
+    mesh, lam, mu, u, _ = make_case(et, g, seed=5)
+    asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
+    asm.set_dirichlet(np.arange(9))
+    asm.assemble_hessian_reduced(u, "fp64", project_to_psd=True)
+    b = np.random.default_rng(2).standard_normal(asm.n_free)
+    if mem == "device":
+        b = torch.tensor(b, device="cuda")
+    cg = ConjugateGradient(asm, "reduced")
+    cg.set_parameters({"tolerance": 1e-10, "max_iter": 120})
+    bits = lambda x: x.cpu().numpy() if mem == "device" else x
+    x = bits(cg.solve(b))
+    for how in (1, 2):
+        assert lib().pfg_selftest_cg_give_up(asm.handle, how) == 0
+        with pytest.raises(PfgError) as e:
+            cg.solve(b)
+        assert e.value.status == PFG_ERR_CUDA
+        for _ in range(2):
+            assert np.array_equal(bits(cg.solve(b)), x)
     asm.close()
