@@ -21,14 +21,13 @@
 //     the same launches, leaves first: A's lower entries are scattered into the
 //     zeroed fronts, the children's update matrices are added in child order,
 //     and each front is partially factorised in pairs of 64-column panels
-//     (Cholesky and inverse of each diagonal block, the rows below times the
-//     inverse, the first panel's update of the second, then one rank-128 update of
-//     the trailing lower triangle, all products on the FP64 tensor pipe); the
+//     (Cholesky of each diagonal block, the triangular solve of the rows below, the
+//     first panel's update of the second, then one rank-128 update of the trailing
+//     lower triangle, all products on the FP64 tensor pipe); the
 //     trailing block is the update matrix the parent adds.
 //   solve (device): forward substitution leaves first (each front adds its
 //     children's update vectors in child order), backward substitution from the
-//     root, then the inverse permutation.  The diagonal blocks hold the inverses of
-//     their triangles, so each panel step is two products in one launch.
+//     root, then the inverse permutation; each panel step is one launch.
 // Every sum is taken in a fixed order, so factor and solution are bitwise
 // deterministic.  Fronts are dense lower triangles of m (m + 1) / 2 doubles
 // (packed columns), all resident for the factor's lifetime.
@@ -814,25 +813,27 @@ __device__ __forceinline__ double pivot_rcp(double d)
 }
 
 // The factorisation runs in panels of 64 columns, two at a time:
-//   k_dir_diag: Cholesky of the 64 x 64 diagonal block; the block's place in the
-//     factor receives the inverse of its triangle, so that everything after it (the
-//     rows below, both substitutions) is a product instead of a dependent recurrence;
-//   k_dir_rows<true>: the rows below times that inverse, X = B L_d^-T;
-//   k_dir_rows<false>: the first panel's update of the second panel's columns;
-//   (the same two kernels for the second panel;)
+//   k_dir_diag: Cholesky of the 64 x 64 diagonal block;
+//   k_dir_solve_rows: the rows below, X L_d^T = B;
+//   k_dir_rows: the first panel's update of the second panel's columns;
+//   (the first two kernels for the second panel;)
 //   k_dir_update: the rank-128 update of the trailing lower triangle, so the
 //     trailing matrix is read and written once per 128 columns.
 //
+// The diagonal of L is stored as its reciprocal, which is all that its readers need.
+// Triangles are solved by substitution, not multiplied by their inverse: the inverse's error
+// is that of the block's condition (a 24-dof Gaussian Gram matrix: normwise backward error
+// 1e-12 against 2e-16; P2 with lambda / mu 1e8: 8e-16 against 1e-16).
+//
 // k_dir_diag, one CTA per front, the block in shared memory.  One warp factorises eight
 // columns (two rows per lane, pivots and multipliers by shuffle), then all warps apply
-// them to the rest in 8 x 8 tiles on the FP64 tensor pipe.  The triangle's inverse is
-// put together from the inverses of its eight 8 x 8 blocks by doubling:
-// [A 0; B C]^-1 = [A^-1 0; -C^-1 B A^-1 C^-1].  Bound by the 64 dependent pivot steps.
-// One barrier and one rank-1 update of all entries per column took 28 us a block at
-// P2 24^3 (two one-warp 32-column blocks with a substitution each: 60 us); this takes 20.
+// them to the rest in 8 x 8 tiles on the FP64 tensor pipe.  Bound by the 64 dependent
+// pivot steps.  One barrier and one rank-1 update of all entries per column took 28 us a
+// block at P2 24^3 (two one-warp 32-column blocks with a substitution each: 60 us); this
+// takes 16.
 constexpr int DIAG_LD = NBF + 4; // 4 mod 16: a fragment's rows fall on distinct banks
 constexpr int DIAG_SLD = 12;     // the same for the eight scaled panel columns
-constexpr size_t DIAG_SMEM = (2 * NBF * DIAG_LD + NBF * DIAG_SLD + NBF) * sizeof(double);
+constexpr size_t DIAG_SMEM = (NBF * DIAG_LD + NBF * DIAG_SLD + NBF) * sizeof(double);
 __global__ void __launch_bounds__(256) k_dir_diag(const DevFront *__restrict__ fr, const int *__restrict__ list,
 												  double *__restrict__ F, int j0, int *__restrict__ err)
 {
@@ -845,16 +846,14 @@ __global__ void __launch_bounds__(256) k_dir_diag(const DevFront *__restrict__ f
 	const int ld = f.m - j0;
 	extern __shared__ __align__(16) double dsm[];
 	double(*M)[DIAG_LD] = reinterpret_cast<double(*)[DIAG_LD]>(dsm);                  // the block, by rows
-	double(*V)[DIAG_LD] = reinterpret_cast<double(*)[DIAG_LD]>(dsm + NBF * DIAG_LD);  // its triangle's inverse
-	double(*S)[DIAG_SLD] = reinterpret_cast<double(*)[DIAG_SLD]>(dsm + 2 * NBF * DIAG_LD); // panel columns over their pivots
-	double *rs = dsm + 2 * NBF * DIAG_LD + NBF * DIAG_SLD;                            // pivots, then 1 / sqrt
+	double(*S)[DIAG_SLD] = reinterpret_cast<double(*)[DIAG_SLD]>(dsm + NBF * DIAG_LD); // panel columns over their pivots
+	double *rs = dsm + NBF * DIAG_LD + NBF * DIAG_SLD;                                 // pivots, then 1 / l_cc
 #pragma unroll
 	for (int i = 0; i < 16; ++i)
 	{
 		const int l = 4 * i + g;
 		// rows past the block's end continue it as the identity
 		M[r][l] = r < nb && l <= r ? Fb[l * ld - l * (l + 1) / 2 + r] : (r == l ? 1.0 : 0.0);
-		V[r][l] = 0.0;
 	}
 	__syncthreads();
 #pragma unroll 1
@@ -922,87 +921,129 @@ __global__ void __launch_bounds__(256) k_dir_diag(const DevFront *__restrict__ f
 		}
 		__syncthreads();
 	}
-	if (tid < NBF)
-	{
-		const double d = rs[tid];
-		rs[tid] = sqrt(d) / d; // 1 / l_cc
-	}
+	if (tid < NBF) rs[tid] = 1.0 / sqrt(rs[tid]);
 	__syncthreads();
 #pragma unroll 4
 	for (int i = 0; i < 16; ++i)
 	{
 		const int l = 4 * i + g;
-		M[r][l] *= rs[l]; // above the diagonal: never read
-	}
-	__syncthreads();
-	if (lane < 8)
-	{
-		// inverse of the warp's 8 x 8 diagonal triangle, a column per lane
-		const int h = 8 * warp;
-		double x[8];
-#pragma unroll
-		for (int i = 0; i < 8; ++i) x[i] = i == lane ? 1.0 : 0.0;
-#pragma unroll
-		for (int i = 0; i < 8; ++i)
-		{
-			x[i] *= rs[h + i];
-#pragma unroll
-			for (int l = i + 1; l < 8; ++l) x[l] = fma(-M[h + l][h + i], x[i], x[l]);
-		}
-#pragma unroll
-		for (int i = 0; i < 8; ++i) V[h + i][h + lane] = x[i];
-	}
-#pragma unroll 1
-	for (int w = 8; w < NBF; w *= 2)
-	{
-		const int tw = w / 8, tiles = NBF / (2 * w) * tw * tw; // 8 x 8 tiles of all pairs of w x w blocks
-		__syncthreads();
-		for (int x = warp; x < tiles; x += 8) // B A^-1 into the block above the diagonal
-		{
-			const int h = x / (tw * tw) * 2 * w, i = h + w + 8 * (x / tw % tw), j = h + 8 * (x % tw);
-			double c[2] = {};
-			for (int k = 0; k < w; k += 4) dmma_8x8(c, M[i + fr_][h + k + fk], V[h + k + fk][j + fr_]);
-			*reinterpret_cast<double2 *>(&M[i - w + fr_][j + w + 2 * fk]) = make_double2(c[0], c[1]);
-		}
-		__syncthreads();
-		for (int x = warp; x < tiles; x += 8) // -C^-1 (B A^-1)
-		{
-			const int h = x / (tw * tw) * 2 * w, i = h + w + 8 * (x / tw % tw), j = h + 8 * (x % tw);
-			double c[2] = {};
-			for (int k = 0; k < w; k += 4) dmma_8x8(c, -V[i + fr_][h + w + k + fk], M[h + k + fk][j + w + fr_]);
-			*reinterpret_cast<double2 *>(&V[i + fr_][j + 2 * fk]) = make_double2(c[0], c[1]);
-		}
-	}
-	__syncthreads();
-#pragma unroll 4
-	for (int i = 0; i < 16; ++i)
-	{
-		const int l = 4 * i + g;
-		if (r < nb && l <= r) Fb[l * ld - l * (l + 1) / 2 + r] = V[r][l];
+		if (r < nb && l <= r) Fb[l * ld - l * (l + 1) / 2 + r] = r == l ? rs[l] : M[r][l] * rs[l];
 	}
 }
 
-// 64 rows below the panel per CTA on the FP64 tensor pipe, K = 64 staged at once:
-//   INV: X = B V^T in place, V the inverse k_dir_diag left in the diagonal block;
-//   else the panel's update of the next panel's columns, C -= P Q^T with Q the rows of P
-//   that belong to those columns (rows and columns from j0 + 64 on).
-// Bound by latency: one wave of CTAs that load, multiply and store once.  A thread-per-row
-// substitution took 14.7 us and a thread-per-row update 22 us for 32 columns at P2 24^3;
-// these take 6 and 8 us for 64 on the last front (7,056 rows).
+// X L_d^T = B in place for 64 rows below the panel per CTA, L_d the panel's triangle.  A warp
+// takes 16 rows through the eight 8-column blocks: its values of the block go to shared
+// memory, a lane per row substitutes the eight columns (scaled by reciprocals of the
+// diagonal), and the solved columns update the later blocks, held as accumulator fragments,
+// on the FP64 tensor pipe.  Bound by that chain of eight steps: 18 us a panel on average at
+// P2 24^3, 16 for the product with the block's inverse that this replaced (and 21 us then for
+// its diagonal block).
 constexpr int ROWS_LD = NBF + 4; // 4 mod 16: the four k rows of a fragment fall on distinct banks
 constexpr size_t ROWS_SMEM = 2 * NBF * ROWS_LD * sizeof(double);
-template <bool INV>
+__global__ void __launch_bounds__(128, 3) k_dir_solve_rows(const DevFront *__restrict__ fr, const int *__restrict__ list,
+														   double *__restrict__ F, int j0)
+{
+	const DevFront f = fr[list[blockIdx.y]];
+	if (f.k <= j0) return;
+	const int nb = min(NBF, f.k - j0), o = j0 + nb, i0 = blockIdx.x * ROWS_TILE, t = f.m - o;
+	if (i0 >= t) return;
+	double *P = F + f.foff + pk(f.m, j0) + o; // column l of the panel from row o on: P + l ld - l (l + 1) / 2
+	const int ld = f.m - j0;
+	extern __shared__ __align__(16) double dsm[];
+	double(*A)[ROWS_LD] = reinterpret_cast<double(*)[ROWS_LD]>(dsm);                 // [column][row] of B, then of X
+	double(*D)[ROWS_LD] = reinterpret_cast<double(*)[ROWS_LD]>(dsm + NBF * ROWS_LD); // [column][row] of L_d, zeros past the panel
+	const int tid = threadIdx.x, r = tid % NBF, l1 = tid / NBF;
+	const bool ra = i0 + r < t;
+	{
+		int off = l1 * ld - l1; // l1 is 0 or 1
+		int step = 2 * ld - 2 * l1 - 3;
+#pragma unroll 8
+		for (int q = 0; q < NBF / 2; ++q)
+		{
+			const int l = l1 + 2 * q;
+			const bool oa = l < nb && ra, ob = l < nb && r >= l && r < nb;
+			cp_async8(&A[l][r], P + (oa ? off + i0 + r : 0), oa);
+			cp_async8(&D[l][r], P + (ob ? off + r - nb : 0), ob);
+			off += step;
+			step -= 4;
+		}
+	}
+	cp_async_commit();
+	cp_async_wait<0>();
+	__syncthreads();
+	const int lane = tid & 31, wr = (tid >> 5) * 16, fk = lane & 3, fr_ = lane >> 2, row = wr + (lane & 15);
+	double acc[8][2][2];
+#pragma unroll
+	for (int j = 0; j < 8; ++j)
+#pragma unroll
+		for (int h = 0; h < 2; ++h)
+#pragma unroll
+			for (int e = 0; e < 2; ++e) acc[j][h][e] = A[8 * j + 2 * fk + e][wr + fr_ + 8 * h];
+	__syncwarp();
+#pragma unroll
+	for (int j = 0; j < 8; ++j)
+	{
+		if (j > 0)
+		{
+#pragma unroll
+			for (int h = 0; h < 2; ++h)
+#pragma unroll
+				for (int e = 0; e < 2; ++e) A[8 * j + 2 * fk + e][wr + fr_ + 8 * h] = acc[j][h][e];
+			__syncwarp();
+		}
+		double x[8];
+#pragma unroll
+		for (int c = 0; c < 8; ++c) x[c] = A[8 * j + c][row];
+#pragma unroll
+		for (int c = 0; c < 8; ++c)
+		{
+			x[c] *= D[8 * j + c][8 * j + c];
+#pragma unroll
+			for (int l = c + 1; l < 8; ++l) x[l] = fma(-D[8 * j + c][8 * j + l], x[c], x[l]);
+		}
+		__syncwarp();
+		if (lane < 16)
+#pragma unroll
+			for (int c = 0; c < 8; ++c) A[8 * j + c][row] = x[c];
+		__syncwarp();
+		if (j == 7) break;
+		const double a[4] = {-A[8 * j + fk][wr + fr_], -A[8 * j + fk][wr + fr_ + 8], -A[8 * j + 4 + fk][wr + fr_],
+							 -A[8 * j + 4 + fk][wr + fr_ + 8]};
+#pragma unroll
+		for (int n = j + 1; n < 8; ++n)
+			dmma_k8(acc[n][0], acc[n][1], a, D[8 * j + fk][8 * n + fr_], D[8 * j + 4 + fk][8 * n + fr_]);
+	}
+	__syncthreads();
+	if (ra)
+	{
+		int off = l1 * ld - l1 + i0 + r, step = 2 * ld - 2 * l1 - 3;
+#pragma unroll 8
+		for (int l = l1; l < NBF; l += 2)
+		{
+			if (l < nb) P[off] = A[l][r];
+			off += step;
+			step -= 4;
+		}
+	}
+}
+
+// The first panel's update of the second panel's columns, C -= P Q^T with Q the rows of P that
+// belong to those columns (rows and columns from j0 + 64 on), 64 rows per CTA on the FP64
+// tensor pipe, K = 64 staged at once.
+// Bound by latency: one wave of CTAs that load, multiply and store once.  A thread-per-row
+// update took 22 us for 32 columns at P2 24^3; this takes 8 us for 64 on the last front
+// (7,056 rows).
 __global__ void __launch_bounds__(128, 3) k_dir_rows(const DevFront *__restrict__ fr, const int *__restrict__ list,
 													 double *__restrict__ F, int j0)
 {
 	const DevFront f = fr[list[blockIdx.y]];
-	if (f.k <= (INV ? j0 : j0 + NBF)) return;
-	const int nb = min(NBF, f.k - j0), o = j0 + nb, i0 = blockIdx.x * ROWS_TILE, t = f.m - o;
+	if (f.k <= j0 + NBF) return;
+	const int o = j0 + NBF, i0 = blockIdx.x * ROWS_TILE, t = f.m - o;
 	if (i0 >= t) return;
 	// column l of the panel from row o on: P + l ld - l (l + 1) / 2
-	double *P = F + f.foff + pk(f.m, j0) + o;
+	const double *P = F + f.foff + pk(f.m, j0) + o;
 	const int ld = f.m - j0;
-	const int nc = INV ? nb : min(NBF, f.k - o); // columns of the result
+	const int nc = min(NBF, f.k - o); // columns of the result
 	extern __shared__ __align__(16) double dsm[];
 	double(*A)[ROWS_LD] = reinterpret_cast<double(*)[ROWS_LD]>(dsm);
 	double(*B)[ROWS_LD] = reinterpret_cast<double(*)[ROWS_LD]>(dsm + NBF * ROWS_LD);
@@ -1015,9 +1056,8 @@ __global__ void __launch_bounds__(128, 3) k_dir_rows(const DevFront *__restrict_
 		for (int q = 0; q < NBF / 2; ++q)
 		{
 			const int l = l1 + 2 * q;
-			const bool oa = l < nb && ra, ob = l < nb && (INV ? r >= l && r < nb : r < nc);
-			cp_async8(&A[l][r], P + (oa ? off + i0 + r : 0), oa);
-			cp_async8(&B[l][r], P + (ob ? off + (INV ? r - nb : r) : 0), ob); // INV: B[l][c] = V(c, l)
+			cp_async8(&A[l][r], P + (ra ? off + i0 + r : 0), ra);
+			cp_async8(&B[l][r], P + (r < nc ? off + r : 0), r < nc);
 			off += step;
 			step -= 4;
 		}
@@ -1025,9 +1065,7 @@ __global__ void __launch_bounds__(128, 3) k_dir_rows(const DevFront *__restrict_
 	cp_async_commit();
 	const int lane = tid & 31, warp = tid >> 5, wr = (warp & 1) * 32, wc = (warp >> 1) * 32;
 	const int fk = lane & 3, fr_ = lane >> 2;
-	// the result: INV overwrites the panel's columns, else columns o .. of the front
-	double *C = INV ? P + i0 : F + f.foff + pk(f.m, o) + o + i0;
-	const int ldc = INV ? ld : t;
+	double *C = F + f.foff + pk(f.m, o) + o + i0; // columns o .. of the front
 	double acc[4][4][2];
 #pragma unroll
 	for (int q = 0; q < 4; ++q)
@@ -1035,19 +1073,18 @@ __global__ void __launch_bounds__(128, 3) k_dir_rows(const DevFront *__restrict_
 		for (int e = 0; e < 2; ++e)
 		{
 			const int c = wc + 8 * q + 2 * fk + e;
-			const double *src = C + (c * ldc - c * (c + 1) / 2);
+			const double *src = C + (c * t - c * (c + 1) / 2);
 #pragma unroll
 			for (int p = 0; p < 4; ++p)
 			{
 				const int i = wr + 8 * p + fr_;
-				acc[p][q][e] = !INV && c < nc && i0 + i < t && i0 + i >= c ? -src[i] : 0.0;
+				acc[p][q][e] = c < nc && i0 + i < t && i0 + i >= c ? -src[i] : 0.0;
 			}
 		}
 	cp_async_wait<0>();
 	__syncthreads();
-	const int ke = INV ? wc + 32 : NBF; // the inverse is lower triangular: column c needs l <= c
 #pragma unroll 4
-	for (int k = 0; k < ke; k += 4)
+	for (int k = 0; k < NBF; k += 4)
 	{
 		double a[4], b[4];
 #pragma unroll
@@ -1067,12 +1104,12 @@ __global__ void __launch_bounds__(128, 3) k_dir_rows(const DevFront *__restrict_
 		for (int e = 0; e < 2; ++e)
 		{
 			const int c = wc + 8 * q + 2 * fk + e;
-			double *dst = C + (c * ldc - c * (c + 1) / 2);
+			double *dst = C + (c * t - c * (c + 1) / 2);
 #pragma unroll
 			for (int p = 0; p < 4; ++p)
 			{
 				const int i = wr + 8 * p + fr_;
-				if (c < nc && i0 + i < t && (INV || i0 + i >= c)) dst[i] = INV ? acc[p][q][e] : -acc[p][q][e];
+				if (c < nc && i0 + i < t && i0 + i >= c) dst[i] = -acc[p][q][e];
 			}
 		}
 }
@@ -1212,10 +1249,53 @@ __global__ void k_dir_permute_out(int n, const int *__restrict__ perm, const dou
 // Forward substitution, level by level from the leaves, in the factorisation's
 // 64-column panels.  k_fwd_init: w = [b_cols; 0] plus the children's update vectors
 // (one CTA per front, children in order); k_fwd_step, one launch per panel: every CTA
-// multiplies the panel's right-hand side by the diagonal block's inverse (y, written to
-// Y once) and updates its own 64 rows below.  The loads of its 64 x 64 block of L are
-// issued before y is known.  Two launches per 32-column panel with a substitution in
-// one warp took 28 us each panel at P2 24^3.
+// solves the panel's right-hand side with the diagonal block (y, written to Y once) and
+// updates its own tiles of 64 rows below.  The loads of its first 64 x 64 block of L are issued
+// before y is known.  9 to 11 us a panel at P2 24^3; with a CTA per tile of rows, each
+// with its own solve of the block, 13.  Two launches per 32-column panel with a substitution
+// in one warp, column by column from memory, took 28.
+//
+// solve_block: one warp, the triangle L in shared memory (D[column][row], zeros past the
+// panel), lane i with entries i and i + 32 of w.  Eight entries at a time reach all
+// lanes by shuffle, every lane substitutes them (a chain of 16 operations), then takes them
+// out of its own two rows.  BACK: L^T, the last eight first.  The solution goes to x[64].
+constexpr int FWD_CTAS = 148 * 3;
+constexpr int SUB_LD = NBF + 1; // odd: a row across the columns falls on distinct banks too
+template <bool BACK>
+__device__ __forceinline__ void solve_block(const double (&D)[NBF][SUB_LD], double w0, double w1, double *x)
+{
+	const int lane = threadIdx.x & 31;
+#pragma unroll
+	for (int q = 0; q < 8; ++q)
+	{
+		const int c0 = 8 * (BACK ? 7 - q : q);
+		double v[8];
+#pragma unroll
+		for (int i = 0; i < 8; ++i) v[i] = __shfl_sync(0xffffffffu, c0 < 32 ? w0 : w1, (c0 + i) & 31);
+#pragma unroll
+		for (int j = 0; j < 8; ++j)
+		{
+			const int i = BACK ? 7 - j : j;
+			v[i] *= D[c0 + i][c0 + i];
+#pragma unroll
+			for (int l = 0; l < 8; ++l)
+				if (BACK ? l < i : l > i) v[l] = fma(BACK ? -D[c0 + l][c0 + i] : -D[c0 + i][c0 + l], v[i], v[l]);
+		}
+		if (lane == 0)
+#pragma unroll
+			for (int i = 0; i < 8; ++i) x[c0 + i] = v[i];
+		// rows (BACK: columns) already solved take part with entries that nobody reads again
+		double s0[2] = {}, s1[2] = {};
+#pragma unroll
+		for (int i = 0; i < 8; ++i)
+		{
+			s0[i & 1] = fma(BACK ? D[lane][c0 + i] : D[c0 + i][lane], v[i], s0[i & 1]);
+			s1[i & 1] = fma(BACK ? D[lane + 32][c0 + i] : D[c0 + i][lane + 32], v[i], s1[i & 1]);
+		}
+		w0 -= s0[0] + s0[1];
+		w1 -= s1[0] + s1[1];
+	}
+}
 __global__ void __launch_bounds__(256) k_fwd_init(const DevFront *__restrict__ fr, const int *__restrict__ list,
 												  const int *__restrict__ child, const int *__restrict__ relpos,
 												  const double *__restrict__ bp, double *__restrict__ W)
@@ -1235,7 +1315,7 @@ __global__ void __launch_bounds__(256) k_fwd_init(const DevFront *__restrict__ f
 	}
 }
 
-__global__ void __launch_bounds__(256) k_fwd_step(const DevFront *__restrict__ fr, const int *__restrict__ list,
+__global__ void __launch_bounds__(256, 3) k_fwd_step(const DevFront *__restrict__ fr, const int *__restrict__ list,
 												  const double *__restrict__ F, double *__restrict__ W,
 												  double *__restrict__ Y, int j0)
 {
@@ -1246,37 +1326,38 @@ __global__ void __launch_bounds__(256) k_fwd_step(const DevFront *__restrict__ f
 	const int r = threadIdx.x % NBF, g = threadIdx.x / NBF; // a row, columns 16 g .. 16 g + 15
 	double *w = W + f.woff;
 	const double *L = F + f.foff;
-	__shared__ double wb[NBF], y[NBF], part[4][NBF];
-	if (g == 0) wb[r] = r < nb ? w[j0 + r] : 0.0;
+	__shared__ double D[NBF][SUB_LD], y[NBF], part[4][NBF];
 	const bool row = i0 + r < f.m;
-	double v[16], b[16];
+	double b[16];
 #pragma unroll
 	for (int q = 0; q < 16; ++q)
 	{
 		const int c = 16 * g + q;
 		const double *Lc = L + pk(f.m, j0 + min(c, nb - 1));
-		v[q] = c < nb && r >= c && r < nb ? Lc[j0 + r] : 0.0;
+		D[c][r] = c < nb && r >= c && r < nb ? Lc[j0 + r] : 0.0;
 		b[q] = c < nb && row ? Lc[i0 + r] : 0.0;
 	}
+	const int lane = threadIdx.x;
+	const double w0 = lane < 32 && lane < nb ? w[j0 + lane] : 0.0, w1 = lane < 32 && lane + 32 < nb ? w[j0 + lane + 32] : 0.0;
 	__syncthreads();
-	double s = 0.0;
-#pragma unroll
-	for (int q = 0; q < 16; ++q) s = fma(v[q], wb[16 * g + q], s);
-	part[g][r] = s;
+	if (threadIdx.x < 32) solve_block<false>(D, w0, w1, y);
 	__syncthreads();
-	if (g == 0)
+	if (blockIdx.x == 0 && g == 0 && r < nb) Y[f.col0 + j0 + r] = y[r];
+	for (int x0 = i0; x0 < f.m; x0 += gridDim.x * ROWS_TILE)
 	{
-		const double yr = (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
-		y[r] = yr;
-		if (blockIdx.x == 0 && r < nb) Y[f.col0 + j0 + r] = yr;
-	}
-	__syncthreads();
-	s = 0.0;
+		const bool on = x0 + r < f.m;
+		if (x0 != i0)
 #pragma unroll
-	for (int q = 0; q < 16; ++q) s = fma(b[q], y[16 * g + q], s);
-	part[g][r] = s;
-	__syncthreads();
-	if (g == 0 && row) w[i0 + r] -= (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
+			for (int q = 0; q < 16; ++q)
+				b[q] = on && 16 * g + q < nb ? L[pk(f.m, j0 + 16 * g + q) + x0 + r] : 0.0;
+		double s = 0.0;
+#pragma unroll
+		for (int q = 0; q < 16; ++q) s = fma(b[q], y[16 * g + q], s);
+		part[g][r] = s;
+		__syncthreads();
+		if (g == 0 && on) w[x0 + r] -= (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
+		__syncthreads();
+	}
 }
 
 __device__ __forceinline__ double warp_sum_d(double v)
@@ -1288,8 +1369,8 @@ __device__ __forceinline__ double warp_sum_d(double v)
 
 // Backward substitution, level by level from the root.  k_bwd_gather: w2 = the rows'
 // solution (ancestors, already solved); k_bwd_l21: w1 = y - L21^T w2 (a warp per
-// column); k_bwd_step, one launch per panel from the last: every CTA multiplies the
-// panel's w1 by the transposed inverse of the diagonal block (x, written to X once) and
+// column); k_bwd_step, one launch per panel from the last: every CTA solves the panel's w1
+// with the transposed diagonal block (x, written to X once) and
 // subtracts the panel's rows times x from its own 64 earlier columns, a warp per
 // column, the loads issued before x is known.
 __global__ void __launch_bounds__(256) k_bwd_gather(const DevFront *__restrict__ fr, const int *__restrict__ list,
@@ -1330,28 +1411,24 @@ __global__ void __launch_bounds__(256) k_bwd_step(const DevFront *__restrict__ f
 	if (blockIdx.x && blockIdx.x * NBF >= j0) return;
 	double *w = W + f.woff;
 	const double *L = F + f.foff;
-	__shared__ double x[NBF];
+	__shared__ double D[NBF][SUB_LD], x[NBF];
 	const bool lo = lane < nb, hi = lane + 32 < nb;
-	double b[8][2], v[8][2];
+	double b[8][2];
 #pragma unroll
 	for (int q = 0; q < 8; ++q)
 	{
 		const int l = warp * 8 + q; // column of the diagonal block
 		const double *Lv = L + pk(f.m, j0 + min(l, nb - 1)) + j0;
-		v[q][0] = l < nb && lo && lane >= l ? Lv[lane] : 0.0;
-		v[q][1] = l < nb && hi && lane + 32 >= l ? Lv[lane + 32] : 0.0;
+		D[l][lane] = l < nb && lo && lane >= l ? Lv[lane] : 0.0;
+		D[l][lane + 32] = l < nb && hi && lane + 32 >= l ? Lv[lane + 32] : 0.0;
 		const bool on = c0 + q < j0;
 		const double *Lc = L + pk(f.m, on ? c0 + q : 0) + j0;
 		b[q][0] = on && lo ? Lc[lane] : 0.0;
 		b[q][1] = on && hi ? Lc[lane + 32] : 0.0;
 	}
 	const double w0 = lo ? w[j0 + lane] : 0.0, w1 = hi ? w[j0 + lane + 32] : 0.0;
-#pragma unroll
-	for (int q = 0; q < 8; ++q)
-	{
-		const double s = warp_sum_d(fma(v[q][0], w0, v[q][1] * w1));
-		if (lane == 0) x[warp * 8 + q] = s;
-	}
+	__syncthreads();
+	if (warp == 0) solve_block<true>(D, w0, w1, x);
 	__syncthreads();
 	const double x0 = x[lane], x1 = x[lane + 32];
 	if (blockIdx.x == 0 && warp == 0)
@@ -1380,8 +1457,8 @@ int direct_factorize(DirectFactor *f, const double *vals, cudaStream_t s, cudaEr
 	const auto smem = [&](const void *k, size_t bytes) {
 		return (*ce = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes)) == cudaSuccess;
 	};
-	if (!smem((const void *)k_dir_diag, DIAG_SMEM) || !smem((const void *)k_dir_rows<true>, ROWS_SMEM) ||
-		!smem((const void *)k_dir_rows<false>, ROWS_SMEM) || !smem((const void *)k_dir_update, UPDATE_SMEM))
+	if (!smem((const void *)k_dir_diag, DIAG_SMEM) || !smem((const void *)k_dir_solve_rows, ROWS_SMEM) ||
+		!smem((const void *)k_dir_rows, ROWS_SMEM) || !smem((const void *)k_dir_update, UPDATE_SMEM))
 		return 2;
 	size_t pi = 0;
 	for (int h = 0; h < nl; ++h)
@@ -1403,9 +1480,9 @@ int direct_factorize(DirectFactor *f, const double *vals, cudaStream_t s, cudaEr
 			const Panel &p = f->panels[pi];
 			const bool second = (p.j0 / NBF) & 1;
 			k_dir_diag<<<nf, 256, DIAG_SMEM, s>>>(f->d_fr, list, f->d_front, p.j0, f->d_err);
-			if (p.rows_grid > 0) k_dir_rows<true><<<dim3(p.rows_grid, nf), 128, ROWS_SMEM, s>>>(f->d_fr, list, f->d_front, p.j0);
+			if (p.rows_grid > 0) k_dir_solve_rows<<<dim3(p.rows_grid, nf), 128, ROWS_SMEM, s>>>(f->d_fr, list, f->d_front, p.j0);
 			if (!second && p.upd_grid > 0)
-				k_dir_rows<false><<<dim3(p.upd_grid, nf), 128, ROWS_SMEM, s>>>(f->d_fr, list, f->d_front, p.j0);
+				k_dir_rows<<<dim3(p.upd_grid, nf), 128, ROWS_SMEM, s>>>(f->d_fr, list, f->d_front, p.j0);
 			// the pair's trailing update, after its last panel on this level
 			const Panel &p0 = second ? f->panels[pi - 1] : p;
 			if ((second || p.upd_grid == 0) && p0.tiles_grid > 0)
@@ -1436,8 +1513,11 @@ cudaError_t direct_solve(DirectFactor *f, const double *b, double *x, cudaStream
 		const int *list = f->d_lvl_list + f->lvl_start[h];
 		k_fwd_init<<<nf, 256, 0, s>>>(f->d_fr, list, f->d_child, f->d_relpos, bp, f->d_work);
 		for (; pi < f->panels.size() && f->panels[pi].lvl == h; ++pi)
-			k_fwd_step<<<dim3(std::max(f->panels[pi].rows_grid, 1), nf), 256, 0, s>>>(f->d_fr, list, f->d_front, f->d_work, bp,
-																					  f->panels[pi].j0);
+		{
+			// every CTA solves the block again: no more of them than the chip holds at once
+			const int gx = std::max(1, std::min(f->panels[pi].rows_grid, (FWD_CTAS + nf - 1) / nf));
+			k_fwd_step<<<dim3(gx, nf), 256, 0, s>>>(f->d_fr, list, f->d_front, f->d_work, bp, f->panels[pi].j0);
+		}
 	}
 	for (int h = nl - 1; h >= 0; --h)
 	{

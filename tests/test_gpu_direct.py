@@ -219,3 +219,37 @@ def test_front_sizes_around_the_panel_edges(require_gpu, et, g, n):
     scale = abs(A).sum(axis=1).max() * np.abs(x).max()
     assert np.abs(b - A @ x).max() <= 1e-13 * scale
     asm.close()
+
+
+@pytest.mark.parametrize("width", [0.1, 0.25])
+@pytest.mark.parametrize("et,g", [(M.Q1_HEX, 1), (M.P2_TET, 1), (M.Q1_HEX, 2), (M.Q1_HEX, 6), (M.P2_TET, 4)], ids=str)
+def test_ill_conditioned_systems(require_gpu, et, g, width):
+    """Element matrices that are Gaussian Gram matrices (nearly singular, condition 1e11): the
+    residual of the solve stays at the bound of Cholesky and substitution.  The computed x
+    solves (A + dA) x = b with |dA| <= gamma(3n + 1) |L||L^T| (Higham, Accuracy and Stability,
+    theorem 10.4), and (|L||L^T|)_ij <= sqrt(a_ii a_jj); two roundings more a pivot where a
+    reciprocal takes the division's place: 5 n u.  A product with an explicit inverse of the
+    diagonal blocks misses it by the root of the blocks' condition."""
+    import torch
+    mesh, lam, mu, _, _ = make_case(et, g, seed=2)
+    asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
+    outer, inner = asm.hessian_pattern()
+    n, k = asm.n_dofs, 3 * mesh.conn.shape[1]
+    t = np.linspace(0.0, 1.0, k)
+    gram = np.exp(-(((t[:, None] - t) / width) ** 2)) + 1e-11 * np.eye(k)
+    dofs = (3 * mesh.conn[:, :, None] + np.arange(3)).reshape(mesh.n_elements, k)
+    A = sp.coo_matrix((np.tile(gram.ravel(), mesh.n_elements), (np.repeat(dofs, k, 1).ravel(), np.tile(dofs, (1, k)).ravel())),
+                      shape=(n, n)).tocsc()
+    A.sort_indices()
+    assert np.array_equal(A.indptr, outer) and np.array_equal(A.indices, inner)
+    ds = DirectSolver(asm, "full")
+    ds.analyze_pattern()
+    ds.factorize(torch.tensor(A.data, device="cuda"))
+    root = np.sqrt(A.diagonal())
+    R = A.tocsr()
+    for b in (A @ np.ones(n), np.random.default_rng(3).standard_normal(n)):
+        x = ds.solve(b)
+        Ax = np.add.reduceat(R.data.astype(np.longdouble) * x[R.indices], R.indptr[:-1])
+        bound = 5 * n * 2.0 ** -53 * root * (root @ np.abs(x))
+        assert np.all(np.abs(b - Ax) <= bound), float(np.max(np.abs(b - Ax) / bound))
+    asm.close()
