@@ -8,11 +8,14 @@
 // This is that family's algorithm laid out for the GPU:
 //   analysis (host, once per pattern): columns with identical patterns (the dofs
 //     of one node) are grouped; the group graph is ordered by nested dissection:
-//     of all cuts across the groups' positions along x, y and z (or, for a pattern
-//     without positions, along a breadth-first order) the one with the smallest
-//     vertex separator, weighted by balance.  P2 24^3: 2.29 TFLOP against 3.31 with
-//     the middle breadth-first level (whose surfaces bend around the start corner),
-//     Q1 24^3: 37 against 134 GFLOP.  The dissection tree is the assembly
+//     of all cuts across the groups' positions along x, y and z, where these are
+//     known, and along a breadth-first order the one with the smallest vertex
+//     separator, weighted by balance.  P2 24^3: 2.29 TFLOP against 3.31 with the
+//     middle breadth-first level (whose surfaces bend around the start corner),
+//     Q1 24^3: 37 against 134 GFLOP.  The cuts across positions find the planes of a
+//     body that lies along the axes, the breadth-first ones do not depend on how it
+//     lies: turned by 0.5 rad about (1, 2, 3) 2.63 TFLOP and 84 GFLOP, without them
+//     8.51 and 92.  The dissection tree is the assembly
 //     tree: every separator (and every leaf part) is one front whose columns are
 //     eliminated together, after its two halves.  Row structures, front sizes,
 //     the scatter of A's entries into the fronts and the extend-add maps are
@@ -51,6 +54,10 @@ constexpr int NBF = 64;         // panel width
 constexpr int LEAF_DOFS = 96;   // dissection stops at parts of at most this many dofs
 constexpr double MAX_HALF = 0.7; // largest share of a part that one side of a cut may keep
 constexpr double BALANCE = 1.0;  // weight of the imbalance in a cut's cost
+// A breadth-first cut has to be a tenth smaller than one across the positions, whose halves
+// have planes for their next cuts.  At 1.0 P2 24^3 takes 0.6% fewer operations but a level
+// more, 115.5 ms against 113; at 1.2 turned cubes of hexahedra take up to 2.6 times as many.
+constexpr double BFS_COST = 1.1;
 constexpr int ROWS_TILE = 64;   // rows per CTA of the panel solve and of the forward substitution
 
 struct DevFront
@@ -175,11 +182,12 @@ struct NdBuilder
 		return d;
 	}
 
-	// A part of the graph: its vertices sorted by x, y and z where they have positions,
-	// else in any order in ord[0].
+	// A part of the graph: its vertices sorted by x, y and z where they have positions, and in
+	// the pattern's order in ord[3] (the breadth-first orders start from it, as they do for a
+	// pattern without positions).
 	struct Part
 	{
-		std::vector<int> ord[3];
+		std::vector<int> ord[4];
 	};
 
 	// Best vertex separator over every cut of one order: the vertices of rank >= c with
@@ -231,7 +239,7 @@ struct NdBuilder
 				// leaves a larger half to dissect
 				const double big = (double)std::max(a, b) / (double)(a + b); // 0.5 .. 1
 				if (big > MAX_HALF) continue;
-				const double cost = (double)sep * (1.0 + BALANCE * (big - 0.5));
+				const double cost = (double)sep * (1.0 + BALANCE * (big - 0.5)) * (axis == 3 ? BFS_COST : 1.0);
 				if (cost < best.cost) best = {cost, axis, c, k != 0};
 			}
 		}
@@ -241,9 +249,9 @@ struct NdBuilder
 	std::vector<int> build(Part P)
 	{
 		std::vector<int> roots;
-		const std::vector<int> &S = P.ord[0];
+		const std::vector<int> &S = P.ord[3];
 		if (S.empty()) return roots;
-		const int axes = xyz.empty() ? 1 : 3;
+		const int first = xyz.empty() ? 3 : 0; // the first order that the part has
 		const int lab = ++label;
 		for (int v : S) mark[v] = lab;
 		std::vector<int> order, ls;
@@ -263,7 +271,7 @@ struct NdBuilder
 					}
 					parts.emplace_back();
 				}
-			for (int d = 0; d < axes; ++d)
+			for (int d = first; d < 4; ++d)
 				for (int v : P.ord[d]) parts[lev[v]].ord[d].push_back(v);
 			P = Part();
 			for (auto &c : parts)
@@ -282,33 +290,28 @@ struct NdBuilder
 		}
 		Cut best;
 		std::vector<int> level_order;
-		if (axes == 3)
-			for (int d = 0; d < 3; ++d) try_order(P.ord[d], d, lab, best);
-		if (best.axis < 0 || axes == 1)
+		for (int d = first; d < 3; ++d) try_order(P.ord[d], d, lab, best);
+		// the breadth-first order from a pseudo-peripheral vertex, restarting from a
+		// minimum-degree vertex of the last level while the eccentricity grows
+		int h = (int)ls.size() - 1;
+		for (int it = 0; it < 4; ++it)
 		{
-			// no positions (or no cut along them): the breadth-first order from a
-			// pseudo-peripheral vertex, restarting from a minimum-degree vertex of the
-			// last level while the eccentricity grows
-			int h = (int)ls.size() - 1;
-			for (int it = 0; it < 4; ++it)
+			int bv = -1, bd = 1 << 30;
+			for (int q = ls[h - 1]; q < ls[h]; ++q)
 			{
-				int bv = -1, bd = 1 << 30;
-				for (int q = ls[h - 1]; q < ls[h]; ++q)
-				{
-					const int d = degree_in(order[q], lab);
-					if (d < bd) bd = d, bv = order[q];
-				}
-				std::vector<int> o2, l2;
-				bfs(bv, lab, o2, l2);
-				const int h2 = (int)l2.size() - 1;
-				if (h2 <= h) break;
-				h = h2;
-				order.swap(o2);
-				ls.swap(l2);
+				const int d = degree_in(order[q], lab);
+				if (d < bd) bd = d, bv = order[q];
 			}
-			level_order = order;
-			try_order(level_order, 3, lab, best);
+			std::vector<int> o2, l2;
+			bfs(bv, lab, o2, l2);
+			const int h2 = (int)l2.size() - 1;
+			if (h2 <= h) break;
+			h = h2;
+			order.swap(o2);
+			ls.swap(l2);
 		}
+		level_order = order;
+		try_order(level_order, 3, lab, best);
 		if (best.axis < 0)
 		{
 			roots.push_back(make_node(S, {}));
@@ -337,7 +340,7 @@ struct NdBuilder
 			if (sd == 2) Sep.push_back(v);
 		}
 		Part A, B;
-		for (int d = 0; d < axes; ++d)
+		for (int d = first; d < 4; ++d)
 			for (int v : P.ord[d])
 			{
 				const char sd = side[lev[v]];
@@ -434,8 +437,8 @@ int direct_symbolic(int n, const int *outer, const int *inner, const double *nod
 	nd.vis.assign(ng, 0);
 	nd.lev.assign(ng, 0);
 	NdBuilder::Part all;
-	all.ord[0].resize(ng);
-	std::iota(all.ord[0].begin(), all.ord[0].end(), 0);
+	all.ord[3].resize(ng);
+	std::iota(all.ord[3].begin(), all.ord[3].end(), 0);
 	if (node_pos)
 	{
 		nd.xyz.resize(3 * (size_t)ng);
@@ -445,9 +448,9 @@ int direct_symbolic(int n, const int *outer, const int *inner, const double *nod
 				const double x = node_pos[3 * (size_t)gfirst[g] + d];
 				nd.xyz[3 * (size_t)g + d] = std::isfinite(x) ? x : 0.0;
 			}
-		for (int d = 2; d >= 0; --d)
+		for (int d = 0; d < 3; ++d)
 		{
-			if (d) all.ord[d] = all.ord[0]; // ord[0] is still the identity
+			all.ord[d] = all.ord[3];
 			const double *x = nd.xyz.data() + d;
 			std::stable_sort(all.ord[d].begin(), all.ord[d].end(), [&](int a, int b) { return x[3 * (size_t)a] < x[3 * (size_t)b]; });
 		}
