@@ -57,7 +57,7 @@ struct pfg_context
 	// staging buffers (allocated on first use): element contributions / element Hessian blocks
 	double *d_vec_stage = nullptr;
 	// nodal sums per tile of elements (TilePlan), FE and geometric nodes (built on first use)
-	void *d_tile[2][5] = {};
+	void *d_tile[2] = {};
 	bool tile_tried[2] = {false, false};
 	void *d_hess_stage[2] = {nullptr, nullptr}; // [0] FP64, [1] FP32
 	std::vector<int> h_conn; // row-major E x n copy for the host pattern build
@@ -221,13 +221,17 @@ int check_material_prec(pfg_context *c, int prec)
 }
 int check_prec(int prec) { return prec == PFG_FP64 || prec == PFG_FP32 || prec == PFG_SPLIT32 || prec == PFG_SPLIT32_SIMT; }
 
-int ensure_staging(pfg_context *c, size_t out_doubles)
+// Device copies of a host-memory call's inputs (u, and a second vector behind it) and result;
+// a call on device memory needs none.
+int ensure_staging(pfg_context *c, int mem, size_t out_doubles)
 {
+	if (mem == PFG_MEM_DEVICE) return PFG_OK;
 	const size_t ndof = 3 * (size_t)c->m.N;
 	if (!c->d_u)
 	{
-		PFG_CUDA(c, cudaMalloc(&c->d_u, std::max<size_t>(ndof, 1) * sizeof(double)));
-		PFG_CUDA(c, cudaMalloc(&c->d_p, std::max<size_t>(ndof, 1) * sizeof(double)));
+		const size_t each = (ndof + 32) / 32 * 32; // both aligned as allocations are
+		PFG_CUDA(c, cudaMalloc(&c->d_u, 2 * each * sizeof(double)));
+		c->d_p = c->d_u + each;
 	}
 	if (out_doubles > c->out_cap)
 	{
@@ -240,61 +244,75 @@ int ensure_staging(pfg_context *c, size_t out_doubles)
 	return PFG_OK;
 }
 
-// The tile plan of a connectivity, built on the device (one read of the slot count).  None
-// when the tiles' elements share too few nodes: at more than TILE_KEEP slots per incidence
-// the pass through shared memory costs more than the slots it saves (P1 48^3
-// shuffled, 0.97 slots per incidence: 109 us tiled, 102 without; numbered, 0.18: 47 and 69).
-constexpr double TILE_KEEP = 0.75;
-int build_tile_plan(pfg_context *c, const int *conn, int nn, int N, const int *inc_off, const int *inc_eb, void **dev, TilePlan *tp)
+// When nodal sums go by tiles: from `incidences` on (below, the pass through shared memory is
+// longer than the slots' traffic in L2) and up to `slots` per incidence (a shuffled numbering
+// shares less in a tile).  Gradient, us, a slot per incidence -> tiles:
+//   P1 20^3 (192,000 incidences) 8.9 -> 8.7, 17^3 7.1 -> 7.8, 48^3 64 -> 41; 48^3 with part of its
+//   elements shuffled, at 0.48 slots per incidence 74 -> 59, at 0.58 78 -> 77, at 1.0 94 -> 107
+//   P2 12^3 (103,680) 15.5 -> 11.2, 32^3 (0.31) 62 -> 53; 24^3 at 0.32 27.8 -> 27.6, at 0.41 28 -> 31
+//   Q1 48^3 (884,736) 43 -> 39, 36^3 (373,248) 23.4 -> 23.9; 63^3 at 0.38 98 -> 89, at 0.48 99 -> 100
+struct TileRule
+{
+	long long incidences;
+	double slots;
+};
+TileRule tile_rule(int nn) { return nn == 4 ? TileRule{200000, 0.5} : nn == 10 ? TileRule{100000, 0.35} : TileRule{500000, 0.4}; }
+
+// The tile plan of a connectivity, built on the device by the first call that sums nodal
+// contributions: counts in the stage (not in use yet), one read of the number of slots, one
+// allocation.  No plan, and a slot per incidence, where it does not pay, where the memory is
+// short, and, for the time being, while the stream is captured.
+int build_tile_plan(pfg_context *c, int nn, int N, const int *inc_off, const int *inc_eb, size_t stage_bytes, void **mem, TilePlan *tp)
 {
 	const int E = c->m.E, tiles = (E + TILE_E - 1) / TILE_E;
-	int *node_off = nullptr, *off = nullptr, n_slots = 0;
-	PFG_CUDA(c, cudaMalloc(&dev[0], sizeof(int) * ((size_t)N + 1)));
-	node_off = (int *)dev[0];
-	PFG_CUDA(c, cudaMalloc(&dev[1], sizeof(int) * ((size_t)tiles + 1)));
-	off = (int *)dev[1];
-	PFG_CUDA(c, launch_tile_counts(E, N, nn, inc_off, inc_eb, node_off, off, c->stream));
-	PFG_CUDA(c, cudaMemcpyAsync(&n_slots, node_off + N, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+	const long long n_inc = (long long)E * nn;
+	const size_t n_counts = tile_count_ints(E, N);
+	const TileRule rule = tile_rule(nn);
+	if (n_inc < rule.incidences || sizeof(int) * n_counts > stage_bytes) return PFG_OK;
+	int *counts = reinterpret_cast<int *>(c->d_vec_stage), n_slots = 0;
+	PFG_CUDA(c, launch_tile_counts(E, N, nn, inc_off, inc_eb, counts, c->stream));
+	PFG_CUDA(c, cudaMemcpyAsync(&n_slots, counts + N + 1 + tiles, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
 	PFG_CUDA(c, cudaStreamSynchronize(c->stream));
-	if ((double)n_slots > TILE_KEEP * (double)E * nn) return PFG_OK;
-	PFG_CUDA(c, cudaMalloc(&dev[2], sizeof(unsigned short) * (size_t)E * nn));
-	PFG_CUDA(c, cudaMalloc(&dev[3], sizeof(unsigned short) * ((size_t)n_slots + tiles)));
-	PFG_CUDA(c, cudaMalloc(&dev[4], sizeof(int) * (size_t)n_slots));
-	PFG_CUDA(c, launch_tile_build(E, nn, conn, inc_off, inc_eb, off, node_off, (unsigned short *)dev[2], (unsigned short *)dev[3],
-								  (int *)dev[4], c->stream));
-	tp->pos = (const unsigned short *)dev[2];
-	tp->off = off;
-	tp->start = (const unsigned short *)dev[3];
-	tp->slot = (const int *)dev[4];
-	tp->node_off = node_off;
+	if ((double)n_slots > rule.slots * (double)n_inc) return PFG_OK;
+	const size_t ints = n_counts + (size_t)tiles + (size_t)n_slots, shorts = (size_t)n_inc + (size_t)n_slots + (size_t)tiles;
+	if (cudaMalloc(mem, sizeof(int) * ints + sizeof(unsigned short) * shorts) != cudaSuccess)
+	{
+		cudaGetLastError();
+		*mem = nullptr;
+		return PFG_OK;
+	}
+	int *kept = static_cast<int *>(*mem), *slot = kept + n_counts + tiles;
+	unsigned *cur = reinterpret_cast<unsigned *>(kept + n_counts);
+	unsigned short *pos = reinterpret_cast<unsigned short *>(slot + n_slots), *start = pos + n_inc;
+	PFG_CUDA(c, cudaMemcpyAsync(kept, counts, sizeof(int) * n_counts, cudaMemcpyDeviceToDevice, c->stream));
+	PFG_CUDA(c, launch_tile_build(E, N, nn, inc_off, inc_eb, kept, cur, pos, start, slot, c->stream));
+	tp->pos = pos;
+	tp->off = kept + N + 1;
+	tp->start = start;
+	tp->slot = slot;
+	tp->node_off = kept;
 	tp->n_slots = n_slots;
 	return PFG_OK;
 }
 
-// Element-contribution staging of the gradient / shape term and the plan of its nodal sums
-// (geom: over the geometric nodes); first use builds them.
-int ensure_vec_stage(pfg_context *c, bool geom = false)
+// Element-contribution staging of the gradient / shape term and the plan of its nodal sums;
+// first use builds them.  shape: over the geometric nodes, where launch_shape_vjp reads a plan.
+int ensure_vec_stage(pfg_context *c, bool shape = false)
 {
-	const bool iso = c->d_gconn == nullptr;
-	const int k = geom && !iso ? 1 : 0;
-	if (c->m.E > 0 && !c->tile_tried[k])
-	{
-		c->tile_tried[k] = true;
-		int st;
-		if (k == 0)
-			st = build_tile_plan(c, c->m.conn, c->n, c->m.N, c->m.inc_off, c->m.inc_eb, c->d_tile[0], &c->m.tile);
-		else
-			st = build_tile_plan(c, c->m.gconn, c->ng, c->m.Ng, c->m.ginc_off, c->m.ginc_eb, c->d_tile[1], &c->m.gtile);
-		if (iso) c->m.gtile = c->m.tile;
-		if (st) return st;
-	}
-	if (!c->d_vec_stage)
-	{
-		const size_t n = (size_t)std::max(c->m.E, 1) * std::max(c->n, c->ng) * 4;
-		PFG_CUDA(c, cudaMalloc(&c->d_vec_stage, n * sizeof(double)));
-	}
+	const size_t bytes = sizeof(double) * 4 * (size_t)std::max(c->m.E, 1) * std::max(c->n, c->ng);
+	if (!c->d_vec_stage) PFG_CUDA(c, cudaMalloc(&c->d_vec_stage, bytes));
 	c->sc.vec_stage = c->d_vec_stage;
-	return PFG_OK;
+	const bool own = shape && c->d_gconn != nullptr; // geometric nodes with a numbering of their own
+	const int k = own ? 1 : 0;
+	if (c->m.E == 0 || c->tile_tried[k] || (shape && !shape_vjp_tiled(c->m))) return PFG_OK;
+	cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+	PFG_CUDA(c, cudaStreamIsCapturing(c->stream, &capture));
+	if (capture != cudaStreamCaptureStatusNone) return PFG_OK;
+	c->tile_tried[k] = true;
+	if (own) return build_tile_plan(c, c->ng, c->m.Ng, c->m.ginc_off, c->m.ginc_eb, bytes, &c->d_tile[1], &c->m.gtile);
+	const int st = build_tile_plan(c, c->n, c->m.N, c->m.inc_off, c->m.inc_eb, bytes, &c->d_tile[0], &c->m.tile);
+	if (!c->d_gconn) c->m.gtile = c->m.tile;
+	return st;
 }
 
 // Element-block staging of the Hessian for one precision (first use allocates).
@@ -733,16 +751,15 @@ void free_all(pfg_context *c)
 {
 	void *ptrs[] = {c->d_conn, c->d_gconn, c->d_X, c->d_lame, c->d_outer, c->d_inner, c->d_values, c->d_contrib, c->d_blk_rel, c->d_eb_inc, c->d_g_eb_inc,
 					c->d_inc_off, c->d_inc_eb, c->d_ginc_off, c->d_ginc_eb, c->d_vec_stage, c->d_hess_stage[0],
-					c->d_hess_stage[1], c->sc.partials, c->sc.ticket, c->sc.inverted, c->d_result, c->d_u, c->d_p, c->d_out};
+					c->d_hess_stage[1], c->sc.partials, c->sc.ticket, c->sc.inverted, c->d_result, c->d_u, c->d_out};
 	for (void *p : ptrs)
 		if (p) cudaFree(p);
 	void *rptrs[] = {c->d_old_to_new, c->d_free, c->d_red_col_start, c->d_red_outer, c->d_red_inner, c->d_red_row_off,
 					 c->d_red_values, c->d_full_tmp, c->d_red_groups};
 	for (void *p : rptrs)
 		if (p) cudaFree(p);
-	for (auto &tile : c->d_tile)
-		for (void *p : tile)
-			if (p) cudaFree(p);
+	for (void *p : c->d_tile)
+		if (p) cudaFree(p);
 	if (c->d_cg) cudaFree(c->d_cg);
 	for (CgPlan &p : c->cg_plan) free_cg_plan(&p);
 	free_direct(c);
@@ -1127,7 +1144,7 @@ int pfg_energy(pfg_context *c, const double *u, int mem, int prec, double *out)
 	if (c->m.N && !u) return fail(c, PFG_ERR_INVALID, "u NULL");
 	if (int st_m = check_material_prec(c, prec)) return st_m;
 	DeviceGuard g(c->device);
-	int st = ensure_staging(c, 1);
+	int st = ensure_staging(c, mem, 1);
 	if (st) return st;
 	const double *du;
 	if ((st = stage_in(c, u, mem, c->d_u, 3 * (size_t)c->m.N, &du))) return st;
@@ -1150,7 +1167,7 @@ int pfg_energy_per_element(pfg_context *c, const double *u, int mem, int prec, d
 	if (c->m.N && !u) return fail(c, PFG_ERR_INVALID, "u NULL");
 	if (int st_m = check_material_prec(c, prec)) return st_m;
 	DeviceGuard g(c->device);
-	int st = ensure_staging(c, std::max(c->m.E, 1));
+	int st = ensure_staging(c, mem, std::max(c->m.E, 1));
 	if (st) return st;
 	const double *du;
 	if ((st = stage_in(c, u, mem, c->d_u, 3 * (size_t)c->m.N, &du))) return st;
@@ -1172,7 +1189,7 @@ int pfg_gradient(pfg_context *c, const double *u, int mem, int prec, double *gou
 	if (int st_m = check_material_prec(c, prec)) return st_m;
 	DeviceGuard g(c->device);
 	const size_t ndof = 3 * (size_t)c->m.N;
-	int st = ensure_staging(c, std::max<size_t>(ndof, 1));
+	int st = ensure_staging(c, mem, std::max<size_t>(ndof, 1));
 	if (st) return st;
 	const double *du;
 	if ((st = stage_in(c, u, mem, c->d_u, ndof, &du))) return st;
@@ -1221,7 +1238,7 @@ int pfg_hessian(pfg_context *c, const double *u, int mem, int prec, int project_
 	DeviceGuard g(c->device);
 	int st;
 	if (!c->has_pattern && (st = build_pattern(c))) return st;
-	if ((st = ensure_staging(c, 1))) return st;
+	if ((st = ensure_staging(c, mem, 1))) return st;
 	const double *du;
 	if ((st = stage_in(c, u, mem, c->d_u, 3 * (size_t)c->m.N, &du))) return st;
 	if ((st = ensure_hess_stage(c, prec))) return st;
@@ -1249,7 +1266,7 @@ int pfg_hessian_apply(pfg_context *c, const double *values, const double *p, int
 	if (!c->has_pattern) return fail(c, PFG_ERR_STATE, "no Hessian assembled yet (pattern not built)");
 	DeviceGuard g(c->device);
 	const size_t ndof = 3 * (size_t)c->m.N;
-	int st = ensure_staging(c, std::max<size_t>(ndof, 1));
+	int st = ensure_staging(c, mem, std::max<size_t>(ndof, 1));
 	if (st) return st;
 	const double *dp;
 	if ((st = stage_in(c, p, mem, c->d_p, ndof, &dp))) return st;
@@ -1266,7 +1283,7 @@ int pfg_hessian_vector(pfg_context *c, const double *u, const double *p, int mem
 		return fail(c, PFG_ERR_UNSUPPORTED, "the matrix-free product exists for NeoHookean only");
 	DeviceGuard g(c->device);
 	const size_t ndof = 3 * (size_t)c->m.N;
-	int st = ensure_staging(c, std::max<size_t>(ndof, 1));
+	int st = ensure_staging(c, mem, std::max<size_t>(ndof, 1));
 	if (st) return st;
 	const double *du, *dp;
 	if ((st = stage_in(c, u, mem, c->d_u, ndof, &du))) return st;
@@ -1297,7 +1314,7 @@ int pfg_material_vjp(pfg_context *c, const double *u, const double *p, int mem, 
 		return fail(c, PFG_ERR_UNSUPPORTED, "the material derivative exists for NeoHookean and LinearElasticity only");
 	DeviceGuard g(c->device);
 	const size_t ndof = 3 * (size_t)c->m.N;
-	int st = ensure_staging(c, std::max<size_t>(2 * (size_t)c->m.E, 1));
+	int st = ensure_staging(c, mem, std::max<size_t>(2 * (size_t)c->m.E, 1));
 	if (st) return st;
 	const double *du, *dp;
 	if ((st = stage_in(c, u, mem, c->d_u, ndof, &du))) return st;
@@ -1320,7 +1337,7 @@ int pfg_shape_vjp(pfg_context *c, const double *u, const double *p, int mem, int
 	if (int st_m = check_material_prec(c, prec)) return st_m;
 	DeviceGuard g(c->device);
 	const size_t ndof = 3 * (size_t)c->m.N;
-	int st = ensure_staging(c, std::max<size_t>(3 * (size_t)c->m.Ng, 1));
+	int st = ensure_staging(c, mem, std::max<size_t>(3 * (size_t)c->m.Ng, 1));
 	if (st) return st;
 	const double *du, *dp;
 	if ((st = stage_in(c, u, mem, c->d_u, ndof, &du))) return st;
@@ -1400,7 +1417,7 @@ int pfg_hessian_reduced(pfg_context *c, const double *u, int mem, int prec, int 
 	if (int st_m = check_material_prec(c, prec)) return st_m;
 	DeviceGuard g(c->device);
 	int st;
-	if ((st = ensure_staging(c, 1))) return st;
+	if ((st = ensure_staging(c, mem, 1))) return st;
 	const double *du;
 	if ((st = stage_in(c, u, mem, c->d_u, 3 * (size_t)c->m.N, &du))) return st;
 	if ((st = ensure_hess_stage(c, prec))) return st;
@@ -1426,7 +1443,7 @@ int pfg_gradient_reduced(pfg_context *c, const double *u, int mem, int prec, dou
 	if (int st_m = check_material_prec(c, prec)) return st_m;
 	DeviceGuard g(c->device);
 	const size_t ndof = 3 * (size_t)c->m.N;
-	int st = ensure_staging(c, std::max<size_t>(ndof, 1));
+	int st = ensure_staging(c, mem, std::max<size_t>(ndof, 1));
 	if (st) return st;
 	if (!c->d_full_tmp) PFG_CUDA(c, cudaMalloc(&c->d_full_tmp, sizeof(double) * std::max<size_t>(ndof, 1)));
 	const double *du;
@@ -1812,7 +1829,7 @@ int pfg_reduced_to_full(pfg_context *c, const double *y, const double *x_bc, int
 	if (!c->has_dirichlet) return fail(c, PFG_ERR_STATE, "no Dirichlet set (pfg_set_dirichlet)");
 	DeviceGuard g(c->device);
 	const size_t ndof = 3 * (size_t)c->m.N;
-	int st = ensure_staging(c, std::max<size_t>(ndof, 1));
+	int st = ensure_staging(c, mem, std::max<size_t>(ndof, 1));
 	if (st) return st;
 	const double *dy = y, *dbc = x_bc;
 	if (mem == PFG_MEM_HOST)

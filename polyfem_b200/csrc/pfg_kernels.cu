@@ -358,39 +358,64 @@ static void launch_vec_gather(int n_nodes, const int *off, long long n_inc, cons
 // TilePlan on the device.  A node's incidences are in element order, so those of one tile
 // follow one another: a slot per such run.
 // ---------------------------------------------------------------------------
-__global__ void k_tile_count(int n_nodes, int nn, const int *__restrict__ inc_off, const int *__restrict__ inc_eb,
-							 int *__restrict__ node_cnt, int *__restrict__ tile_cnt)
+constexpr int TILE_SCAN = 256; // nodes per block of the slot counts
+// node_cnt: slots before the node among its block's, block_cnt: slots of the block
+__global__ void __launch_bounds__(TILE_SCAN) k_tile_count(int n_nodes, int nn, const int *__restrict__ inc_off,
+														  const int *__restrict__ inc_eb, int *__restrict__ node_cnt,
+														  int *__restrict__ block_cnt, int *__restrict__ tile_cnt)
 {
-	const int B = blockIdx.x * blockDim.x + threadIdx.x;
-	if (B >= n_nodes) return;
-	int last = -1, c = 0;
-	for (int k = __ldg(inc_off + B); k < __ldg(inc_off + B + 1); ++k)
+	__shared__ int part[TILE_SCAN / 32];
+	const int B = blockIdx.x * TILE_SCAN + threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+	int c = 0;
+	if (B < n_nodes)
 	{
-		const int t = __ldg(inc_eb + k) / (nn * TILE_E);
-		if (t == last) continue;
-		last = t;
-		++c;
-		atomicAdd(tile_cnt + t, 1);
+		int last = -1;
+		for (int k = __ldg(inc_off + B); k < __ldg(inc_off + B + 1); ++k)
+		{
+			const int t = __ldg(inc_eb + k) / (nn * TILE_E);
+			if (t == last) continue;
+			last = t;
+			++c;
+			atomicAdd(tile_cnt + t, 1);
+		}
 	}
-	node_cnt[B] = c;
+	int incl = c;
+#pragma unroll
+	for (int o = 1; o < 32; o *= 2)
+	{
+		const int y = __shfl_up_sync(0xffffffffu, incl, o);
+		if (lane >= o) incl += y;
+	}
+	if (lane == 31) part[warp] = incl;
+	__syncthreads();
+	int base = 0, total = 0;
+#pragma unroll
+	for (int w = 0; w < TILE_SCAN / 32; ++w)
+	{
+		if (w < warp) base += part[w];
+		total += part[w];
+	}
+	if (B < n_nodes) node_cnt[B] = base + incl - c;
+	if (threadIdx.x == 0) block_cnt[blockIdx.x] = total;
 }
 
-// exclusive prefix sums of x[0 .. n) in place, the total in x[n]; one block
-__global__ void __launch_bounds__(1024) k_exclusive_scan(int *x, int n)
+// exclusive prefix sums in place, the total behind them: a block for x[0 .. nx), one for y[0 .. ny)
+__global__ void __launch_bounds__(1024) k_exclusive_scan(int *x, int nx, int *y, int ny)
 {
 	__shared__ int part[32];
 	__shared__ int carry;
+	if (blockIdx.x) x = y, nx = ny;
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 	if (threadIdx.x == 0) carry = 0;
 	__syncthreads();
-	for (int i0 = 0; i0 < n; i0 += 4096)
+	for (int i0 = 0; i0 < nx; i0 += 4096)
 	{
 		const int i = i0 + 4 * threadIdx.x;
 		int v[4], s = 0;
 #pragma unroll
 		for (int j = 0; j < 4; ++j)
 		{
-			v[j] = i + j < n ? x[i + j] : 0;
+			v[j] = i + j < nx ? x[i + j] : 0;
 			s += v[j];
 		}
 		int incl = s;
@@ -418,112 +443,72 @@ __global__ void __launch_bounds__(1024) k_exclusive_scan(int *x, int n)
 #pragma unroll
 		for (int j = 0; j < 4; ++j)
 		{
-			if (i + j < n) x[i + j] = e;
+			if (i + j < nx) x[i + j] = e;
 			e += v[j];
 		}
 		__syncthreads();
 		if (threadIdx.x == 0) carry += part[31];
 		__syncthreads();
 	}
-	if (threadIdx.x == 0) x[n] = carry;
+	if (threadIdx.x == 0) x[nx] = carry;
 }
 
-// A block per tile: its incidences sorted by (node, element, local node), a run per node.
-template <int NN>
-__global__ void __launch_bounds__(TILE_E) k_tile_build(int E, const int *__restrict__ conn, const int *__restrict__ inc_off,
-													   const int *__restrict__ inc_eb, const int *__restrict__ off,
-													   const int *__restrict__ node_off, unsigned short *__restrict__ pos,
-													   unsigned short *__restrict__ start, int *__restrict__ slot)
+// A thread per node: its runs (the incidences of one tile) take places and a slot entry in
+// their tiles, in the order they come: where a run lies in a tile's buffer does not matter to
+// the sums, only the order inside it.  cur (cleared before): of each tile, the runs placed so
+// far in the upper half, their incidences in the lower.
+__global__ void __launch_bounds__(256) k_tile_build(int E, int n_nodes, int nn, const int *__restrict__ inc_off,
+													const int *__restrict__ inc_eb, const int *__restrict__ block_cnt,
+													const int *__restrict__ off, int *__restrict__ node_off, unsigned *__restrict__ cur,
+													unsigned short *__restrict__ pos, unsigned short *__restrict__ start,
+													int *__restrict__ slot)
 {
-	constexpr int P = NN * TILE_E <= 512 ? 512 : NN * TILE_E <= 1024 ? 1024 : 2048, PER = P / TILE_E;
-	__shared__ unsigned long long key[P];
-	__shared__ int warp_runs[TILE_E / 32];
-	const int tile = blockIdx.x, e0 = tile * TILE_E, ne = min(TILE_E, E - e0), tid = threadIdx.x, lane = tid & 31;
-	for (int i = tid; i < P; i += TILE_E)
+	const int B = blockIdx.x * 256 + threadIdx.x, tiles = (E + TILE_E - 1) / TILE_E;
+	if (B < tiles) start[__ldg(off + B + 1) + B] = (unsigned short)(min(TILE_E, E - B * TILE_E) * nn);
+	if (B == n_nodes) node_off[B] = __ldg(off + tiles);
+	if (B >= n_nodes) return;
+	int s = node_off[B] + __ldg(block_cnt + B / TILE_SCAN);
+	node_off[B] = s;
+	const int k1 = __ldg(inc_off + B + 1);
+	for (int k = __ldg(inc_off + B); k < k1;)
 	{
-		const int el = i / NN, a = i % NN;
-		key[i] = el < ne ? (unsigned long long)__ldg(conn + (size_t)a * E + e0 + el) << 11 | (unsigned)i : ~0ull;
+		const int t = __ldg(inc_eb + k) / (nn * TILE_E);
+		int e = k + 1;
+		while (e < k1 && __ldg(inc_eb + e) / (nn * TILE_E) == t) ++e;
+		const unsigned at = atomicAdd(cur + t, 0x10000u + (unsigned)(e - k));
+		const int j = (int)(at >> 16), t0 = __ldg(off + t);
+		unsigned p = at & 0xffffu;
+		start[t0 + t + j] = (unsigned short)p;
+		slot[t0 + j] = s++;
+		for (; k < e; ++k) pos[__ldg(inc_eb + k)] = (unsigned short)p++;
 	}
-	for (int k = 2; k <= P; k *= 2)
-		for (int j = k / 2; j > 0; j /= 2)
-		{
-			__syncthreads();
-			for (int i = tid; i < P / 2; i += TILE_E)
-			{
-				const int lo = 2 * i - (i & (j - 1)), hi = lo + j; // bit j of lo is clear
-				const unsigned long long x = key[lo], y = key[hi];
-				if ((x > y) == ((lo & k) == 0))
-				{
-					key[lo] = y;
-					key[hi] = x;
-				}
-			}
-		}
-	__syncthreads();
-	int runs = 0;
-	for (int q = 0; q < PER; ++q)
-	{
-		const int i = tid * PER + q;
-		runs += key[i] != ~0ull && (i == 0 || key[i] >> 11 != key[i - 1] >> 11);
-	}
-	int incl = runs;
-#pragma unroll
-	for (int o = 1; o < 32; o *= 2)
-	{
-		const int y = __shfl_up_sync(0xffffffffu, incl, o);
-		if (lane >= o) incl += y;
-	}
-	if (lane == 31) warp_runs[tid >> 5] = incl;
-	__syncthreads();
-	int r = incl - runs;
-	for (int w = 0; w < tid >> 5; ++w) r += warp_runs[w];
-	const int t0 = __ldg(off + tile);
-	for (int q = 0; q < PER; ++q)
-	{
-		const int i = tid * PER + q;
-		if (key[i] == ~0ull) break;
-		const int node = (int)(key[i] >> 11);
-		pos[(size_t)e0 * NN + (unsigned)(key[i] & 2047)] = (unsigned short)i;
-		if (i > 0 && (int)(key[i - 1] >> 11) == node) continue;
-		// the node's slot: its runs in earlier tiles come first
-		int last = -1, s = __ldg(node_off + node);
-		for (int k = __ldg(inc_off + node);; ++k)
-		{
-			const int t = __ldg(inc_eb + k) / (NN * TILE_E);
-			if (t >= tile) break;
-			s += t != last;
-			last = t;
-		}
-		start[t0 + tile + r] = (unsigned short)i;
-		slot[t0 + r] = s;
-		++r;
-	}
-	if (tid == 0) start[__ldg(off + tile + 1) + tile] = (unsigned short)(ne * NN);
 }
 
-cudaError_t launch_tile_counts(int E, int n_nodes, int nn, const int *inc_off, const int *inc_eb, int *node_off, int *off,
-							   cudaStream_t s)
+size_t tile_count_ints(int E, int n_nodes)
 {
-	const int tiles = (E + TILE_E - 1) / TILE_E;
-	cudaError_t e = cudaMemsetAsync(off, 0, sizeof(int) * (size_t)(tiles + 1), s);
+	return (size_t)n_nodes + 1 + (size_t)(E + TILE_E - 1) / TILE_E + 1 + (size_t)(n_nodes + TILE_SCAN - 1) / TILE_SCAN + 1;
+}
+
+cudaError_t launch_tile_counts(int E, int n_nodes, int nn, const int *inc_off, const int *inc_eb, int *counts, cudaStream_t s)
+{
+	const int tiles = (E + TILE_E - 1) / TILE_E, nb = (n_nodes + TILE_SCAN - 1) / TILE_SCAN;
+	int *node_off = counts, *off = node_off + n_nodes + 1, *block_cnt = off + tiles + 1;
+	cudaError_t e = cudaMemsetAsync(off, 0, sizeof(int) * (size_t)tiles, s);
 	if (e != cudaSuccess) return e;
-	if (n_nodes > 0) k_tile_count<<<(n_nodes + 255) / 256, 256, 0, s>>>(n_nodes, nn, inc_off, inc_eb, node_off, off);
-	k_exclusive_scan<<<1, 1024, 0, s>>>(node_off, n_nodes);
-	k_exclusive_scan<<<1, 1024, 0, s>>>(off, tiles);
+	if (nb > 0) k_tile_count<<<nb, TILE_SCAN, 0, s>>>(n_nodes, nn, inc_off, inc_eb, node_off, block_cnt, off);
+	k_exclusive_scan<<<2, 1024, 0, s>>>(block_cnt, nb, off, tiles);
 	return cudaGetLastError();
 }
 
-cudaError_t launch_tile_build(int E, int nn, const int *conn, const int *inc_off, const int *inc_eb, const int *off,
-							  const int *node_off, unsigned short *pos, unsigned short *start, int *slot, cudaStream_t s)
+cudaError_t launch_tile_build(int E, int n_nodes, int nn, const int *inc_off, const int *inc_eb, int *counts, unsigned *cur,
+							  unsigned short *pos, unsigned short *start, int *slot, cudaStream_t s)
 {
 	const int tiles = (E + TILE_E - 1) / TILE_E;
-	switch (nn)
-	{
-	case 4: k_tile_build<4><<<tiles, TILE_E, 0, s>>>(E, conn, inc_off, inc_eb, off, node_off, pos, start, slot); break;
-	case 8: k_tile_build<8><<<tiles, TILE_E, 0, s>>>(E, conn, inc_off, inc_eb, off, node_off, pos, start, slot); break;
-	case 10: k_tile_build<10><<<tiles, TILE_E, 0, s>>>(E, conn, inc_off, inc_eb, off, node_off, pos, start, slot); break;
-	default: return cudaErrorInvalidValue;
-	}
+	int *node_off = counts, *off = node_off + n_nodes + 1, *block_cnt = off + tiles + 1;
+	cudaError_t e = cudaMemsetAsync(cur, 0, sizeof(unsigned) * (size_t)tiles, s);
+	if (e != cudaSuccess) return e;
+	k_tile_build<<<(std::max(n_nodes + 1, tiles) + 255) / 256, 256, 0, s>>>(E, n_nodes, nn, inc_off, inc_eb, block_cnt, off, node_off,
+																			cur, pos, start, slot);
 	return cudaGetLastError();
 }
 
@@ -3008,6 +2993,10 @@ cudaError_t launch_material_vjp(const DevMesh &m, const double *u, const double 
 	return cudaGetLastError();
 }
 
+// Tiles for P1 NeoHookean only (48^3: 81 -> 64 us): P2 and Q1 have few geometric slots for
+// their arithmetic, and lose 1-4% to the pass through shared memory.
+bool shape_vjp_tiled(const DevMesh &m) { return m.et == 1 && m.mat == 0; }
+
 cudaError_t launch_shape_vjp(const DevMesh &m, const double *u, const double *adj, int prec, double *out,
 							 const Scratch &sc, cudaStream_t s)
 {
@@ -3016,9 +3005,7 @@ cudaError_t launch_shape_vjp(const DevMesh &m, const double *u, const double *ad
 	const int nb = blocks_for(m.E, NT);
 	const bool f32 = prec != PREC_FP64;
 	double *st = sc.vec_stage;
-	// tiles for P1 NeoHookean only (48^3: 81 -> 64 us): P2 and Q1 have few geometric slots for
-	// their arithmetic, and lose 1-4% to the pass through shared memory
-	const TilePlan plan = m.et == 1 && m.mat == 0 ? m.gtile : TilePlan();
+	const TilePlan plan = shape_vjp_tiled(m) ? m.gtile : TilePlan();
 	if (m.mat != 0)
 	{
 		cudaError_t e = launch_ad_shape_vjp_stage(m, u, adj, sc, s);

@@ -302,3 +302,96 @@ def test_gradient_tiles_at_block_edges(require_gpu, et, E):
         assert np.array_equal(asm.assemble_gradient(u), g) and asm.inverted_count() == 0
         assert rel_err(asm.force_shape_derivative(u, p), orc.shape_vjp(u, p)) <= 1e-12
         asm.close()
+
+
+def _first(mesh, E):
+    import copy
+    sub = copy.copy(mesh)
+    sub.conn = np.ascontiguousarray(mesh.conn[:E])
+    sub.gconn = sub.conn if mesh.gconn is mesh.conn else np.ascontiguousarray(mesh.gconn[:E])
+    return sub
+
+
+def _slots_per_incidence(conn):
+    """(tile of 128 elements, node) pairs over incidences: what decides whether sums go by tiles."""
+    E, n = conn.shape
+    pairs = (np.arange(E, dtype=np.int64)[:, None] // 128) * (int(conn.max()) + 1) + conn
+    return np.unique(pairs).size / conn.size
+
+
+@pytest.mark.parametrize("rest", [0, 1, 127])
+@pytest.mark.parametrize("et,g,tiles", [(M.P1_TET, 21, 391), (M.P2_TET, 12, 79), (M.Q1_HEX, 40, 489)], ids=["P1", "P2", "Q1"])
+def test_nodal_sums_per_tile_and_per_incidence(require_gpu, et, g, tiles, rest):
+    """Meshes large enough for nodal sums per tile of 128 elements, their last tile whole, with one
+    element or one short, and with nodes of no element: gradient and H p against the oracle and
+    the assembled matrix, and every formulation family, MultiModels and the shape derivative
+    against the same elements shuffled, whose sums go per incidence.  Repeated calls agree
+    bitwise, and the inverted count is the last call's."""
+    from oracle.binding import Oracle
+    mesh, lam, mu, u, p = make_case(et, g, seed=12)
+    E = tiles * 128 + rest
+    sub = _first(mesh, E)
+    assert E <= mesh.n_elements and _slots_per_incidence(sub.conn) <= {M.P1_TET: 0.3, M.P2_TET: 0.33, M.Q1_HEX: 0.39}[et]
+    order = np.random.default_rng(E).permutation(E)
+    shuf = _first(mesh, E)
+    shuf.conn = np.ascontiguousarray(sub.conn[order])
+    shuf.gconn = shuf.conn if mesh.gconn is mesh.conn else np.ascontiguousarray(sub.gconn[order])
+    assert _slots_per_incidence(shuf.conn) >= 0.9
+    asm = NeoHookeanAssembler.from_mesh(sub, lam[:E], mu[:E])
+    ash = NeoHookeanAssembler.from_mesh(shuf, lam[:E][order], mu[:E][order])
+    g0 = asm.assemble_gradient(u)
+    assert rel_err(g0, Oracle(sub, lam[:E], mu[:E], n_threads=8).gradient(u)) <= 1e-12
+    assert rel_err(ash.assemble_gradient(u), g0) <= 1e-12
+    assert rel_err(ash.assemble_gradient(u, "fp32"), asm.assemble_gradient(u, "fp32")) <= 1e-6
+    assert np.array_equal(asm.assemble_gradient(u), g0) and asm.inverted_count() == 0
+    q = asm.hessian_vector(u, p)
+    assert rel_err(q, asm.assemble_hessian(u) @ p) <= 1e-13
+    assert rel_err(ash.hessian_vector(u, p), q) <= 1e-12
+    assert rel_err(ash.force_shape_derivative(u, p), asm.force_shape_derivative(u, p)) <= 1e-12
+    flipped = u.copy()
+    flipped.reshape(-1, 3)[sub.conn[E // 2, 0]] += 10 * mesh.h
+    for a in (asm, ash):
+        a.assemble_energy(flipped)
+        n_bad = a.inverted_count()
+        a.assemble_gradient(flipped)
+        assert n_bad >= 1 and a.inverted_count() == n_bad
+        a.assemble_gradient(u)
+        assert a.inverted_count() == 0
+    sel = (np.arange(E) % 3 == 0).astype(np.int32)
+    for set_up in (lambda a, s: a.set_material("SaintVenant"), lambda a, s: a.set_material("VolumePenalty", k=2e5),
+                   lambda a, s: a.set_composite([{"formulation": "NeoHookean"}, {"formulation": "SaintVenant"}], sel[s])):
+        set_up(asm, np.arange(E))
+        set_up(ash, order)
+        assert rel_err(ash.assemble_gradient(u), asm.assemble_gradient(u)) <= 1e-12
+    asm.close()
+    ash.close()
+
+
+@pytest.mark.parametrize("et,g", [(M.P1_TET, 21), (M.P2_TET, 12), (M.Q1_HEX, 40)], ids=["P1", "P2", "Q1"])
+def test_nodal_sums_under_capture(require_gpu, et, g):
+    """After an eager gradient the shape derivative is captured on its first call, and a first
+    gradient is captured where the capture allows allocations, as before there were tiles: the
+    replays return the eager results."""
+    import torch
+    mesh, lam, mu, u, p = make_case(et, g, seed=12)
+    du, dp = torch.tensor(u, device="cuda"), torch.tensor(p, device="cuda")
+
+    def captured(f, mode):
+        g_ = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g_, capture_error_mode=mode):
+            out = f()
+        out.zero_()
+        g_.replay()
+        torch.cuda.synchronize()
+        return out.cpu().numpy()
+
+    asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
+    grad = asm.assemble_gradient(du).cpu().numpy()
+    shape = captured(lambda: asm.force_shape_derivative(du, dp), "global")
+    assert rel_err(shape, asm.force_shape_derivative(du, dp).cpu().numpy()) <= 1e-13
+    asm.close()
+    asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
+    first = captured(lambda: asm.assemble_gradient(du), "relaxed")
+    assert rel_err(first, grad) <= 1e-13
+    assert np.array_equal(asm.assemble_gradient(du).cpu().numpy(), grad)
+    asm.close()
