@@ -157,6 +157,14 @@ int pfg_hessian_apply(pfg_context *ctx, const double *values, const double *p, i
  * needed nor touched.  PFG_ERR_UNSUPPORTED for other materials and compositions. */
 int pfg_hessian_vector(pfg_context *ctx, const double *u, const double *p, int mem, double *q);
 
+/* Makes the NeoHookean Hessian at u in FP64, with the Lame parameters and rest positions
+ * set now, the context's matrix, as pfg_hessian(ctx, u, mem, PFG_FP64, 0, NULL) does, but
+ * assembles it only when a call reads that matrix or its device pointer is asked for
+ * (pfg_hessian_apply, pfg_cg_solve and pfg_direct_factorize with NULL values on the full
+ * system, pfg_hessian_device_csc).  u, the parameters and the positions are copied.  On a
+ * stream under capture the matrix is assembled at once. */
+int pfg_hessian_later(pfg_context *ctx, const double *u, int mem);
+
 /* Device pointers of the context-owned CSC arrays (valid until pfg_destroy). */
 int pfg_hessian_device_csc(pfg_context *ctx, const int **outer, const int **inner, double **values);
 

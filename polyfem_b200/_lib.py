@@ -110,6 +110,7 @@ SIGNATURES = {
     "pfg_hessian": (ctypes.c_int, [_vp, _vp, ctypes.c_int, ctypes.c_int, ctypes.c_int, _vp]),
     "pfg_hessian_apply": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int, _vp]),
     "pfg_hessian_vector": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int, _vp]),
+    "pfg_hessian_later": (ctypes.c_int, [_vp, _vp, ctypes.c_int]),
     "pfg_hessian_device_csc": (ctypes.c_int, [_vp, ctypes.POINTER(_vp), ctypes.POINTER(_vp), ctypes.POINTER(_vp)]),
     "pfg_material_vjp": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int, _vp]),
     "pfg_shape_vjp": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int, ctypes.c_int, _vp]),

@@ -236,6 +236,13 @@ class NeoHookeanAssembler:
         check(lib().pfg_hessian_vector(self._h, ptrs[0], ptrs[1], mem, optr), self._h, "pfg_hessian_vector")
         return out
 
+    def hessian_later(self, u):
+        """assemble_hessian_into_context(u) in FP64 (NeoHookean only), put off until something
+        reads the context's matrix (pfg_hessian_later)."""
+        self._check_len(u, self.n_dofs, "u")
+        mem, ptrs, keep = self._prepare(u)
+        check(lib().pfg_hessian_later(self._h, ptrs[0], mem), self._h, "pfg_hessian_later")
+
     def assemble_hessian_into_context(self, u, precision="fp64", project_to_psd: bool = False):
         """Assemble the Hessian into the context's own device buffer (no copy out)."""
         self._check_len(u, self.n_dofs, "u")

@@ -12,9 +12,10 @@ backward(p) returns the vector-Jacobian products of f:
       (ElasticForceDerivative.cpp:207-260), which equals +p . df/dX_rest;
   d(p.f)/du                  : H p, bitwise deterministic.  In FP64, for NeoHookean,
       the directional derivative of the gradient along p, without the matrix
-      (pfg_hessian_vector: 72 us at P2 32^3, where assembling and applying H takes 881); in the other modes the Hessian assembled
-      in that mode (structurally and numerically symmetric) times p
-      (pfg_hessian_apply).
+      (pfg_hessian_vector: 72 us at P2 32^3, where assembling and applying H takes 881);
+      in the other modes the Hessian assembled in that mode (structurally and numerically
+      symmetric) times p (pfg_hessian_apply).  In every mode H is the context's matrix
+      afterwards, in FP64 assembled when it is first read.
 Each backward term recomputes F and the basis gradients per quadrature point
 from (u, lambda, mu, X); nothing from the forward pass is stored on the device
 beyond the four inputs.
@@ -63,6 +64,7 @@ class ElasticForce(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             if asm.material == "NeoHookean" and ctx.precision in ("fp64", PFG_FP64):
                 g_u = asm.hessian_vector(u, p)
+                asm.hessian_later(u)  # the context's matrix is H here too, when it is read
             else:
                 asm.assemble_hessian_into_context(u, ctx.precision)
                 g_u = asm.hessian_apply(p)

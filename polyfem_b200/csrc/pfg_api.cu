@@ -60,6 +60,9 @@ struct pfg_context
 	void *d_tile[2] = {};
 	bool tile_tried[2] = {false, false};
 	void *d_hess_stage[2] = {nullptr, nullptr}; // [0] FP64, [1] FP32
+	// pfg_hessian_later: the matrix is still to be assembled, from these copies of (lambda, mu), u and X
+	bool later = false;
+	double *d_later = nullptr;
 	std::vector<int> h_conn; // row-major E x n copy for the host pattern build
 	// scratch and host-mode staging
 	Scratch sc;
@@ -516,6 +519,26 @@ int build_pattern(pfg_context *c)
 	return PFG_OK;
 }
 
+// Before anything reads the context's matrix (values) or its pattern: what pfg_hessian_later
+// left to be done.
+int settle_hessian(pfg_context *c, bool values)
+{
+	if (!c->later) return PFG_OK;
+	DeviceGuard g(c->device);
+	int st;
+	if (!c->has_pattern && (st = build_pattern(c))) return st;
+	if (!values) return PFG_OK;
+	if ((st = ensure_hess_stage(c, PFG_FP64))) return st;
+	DevMesh m = c->m;
+	m.mat = PFG_MAT_NEOHOOKEAN;
+	m.lame = reinterpret_cast<const double2 *>(c->d_later);
+	const double *u = c->d_later + 2 * (size_t)m.E;
+	m.X = u + 3 * (size_t)m.N;
+	PFG_CUDA(c, launch_hessian(m, c->pat, u, PFG_FP64, false, c->d_hess_stage[0], c->stream));
+	c->later = false;
+	return PFG_OK;
+}
+
 // node -> incidence lists (grouped by node, elements ascending) of a connectivity
 void build_incidence(const int *conn, int E, int n, int N, std::vector<long long> &off, std::vector<int> &elem,
 					 std::vector<int> &eb)
@@ -760,6 +783,7 @@ void free_all(pfg_context *c)
 		if (p) cudaFree(p);
 	for (void *p : c->d_tile)
 		if (p) cudaFree(p);
+	if (c->d_later) cudaFree(c->d_later);
 	if (c->d_cg) cudaFree(c->d_cg);
 	for (CgPlan &p : c->cg_plan) free_cg_plan(&p);
 	free_direct(c);
@@ -1221,6 +1245,7 @@ int pfg_hessian_pattern(pfg_context *c, long long *nnz)
 int pfg_hessian_pattern_copy(pfg_context *c, int *outer, int *inner, int mem)
 {
 	if (!c || !check_mem(mem)) return fail(c, PFG_ERR_INVALID, "bad arguments");
+	if (int st = settle_hessian(c, false)) return st;
 	if (!c->has_pattern) return fail(c, PFG_ERR_STATE, "pattern not built");
 	DeviceGuard g(c->device);
 	const cudaMemcpyKind k = mem == PFG_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
@@ -1245,6 +1270,7 @@ int pfg_hessian(pfg_context *c, const double *u, int mem, int prec, int project_
 	// device output goes straight into the caller's array; otherwise into the context's
 	DevPattern p = c->pat;
 	if (values && mem == PFG_MEM_DEVICE) p.values = values;
+	else c->later = false;
 	if (c->composite)
 	{
 		if ((st = composite_hessian(c, p, du, project_psd))) return st;
@@ -1260,9 +1286,33 @@ int pfg_hessian(pfg_context *c, const double *u, int mem, int prec, int project_
 	return PFG_OK;
 }
 
+int pfg_hessian_later(pfg_context *c, const double *u, int mem)
+{
+	if (!c || !check_mem(mem) || (c->m.N && !u)) return fail(c, PFG_ERR_INVALID, "bad arguments");
+	if (c->composite || c->m.mat != PFG_MAT_NEOHOOKEAN)
+		return fail(c, PFG_ERR_UNSUPPORTED, "the matrix can be left for later for NeoHookean only");
+	DeviceGuard g(c->device);
+	cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+	PFG_CUDA(c, cudaStreamIsCapturing(c->stream, &capture));
+	// a replay has to leave its own matrix
+	if (capture != cudaStreamCaptureStatusNone) return pfg_hessian(c, u, mem, PFG_FP64, 0, nullptr);
+	const long long ndof = 3LL * c->m.N, nx = 3LL * c->m.Ng, nl = 2LL * c->m.E;
+	int st;
+	if ((st = ensure_staging(c, mem, 1))) return st;
+	const double *du;
+	if ((st = stage_in(c, u, mem, c->d_u, ndof, &du))) return st;
+	if (!c->d_later) PFG_CUDA(c, cudaMalloc(&c->d_later, sizeof(double) * std::max(nl + ndof + nx, 1LL)));
+	// (lambda, mu) first: pairs on 16 bytes
+	PFG_CUDA(c, launch_copy3(reinterpret_cast<const double *>(c->d_lame), nl, du, ndof, c->d_X, nx, c->d_later, c->stream));
+	c->later = true;
+	if (mem == PFG_MEM_HOST) PFG_CUDA(c, cudaStreamSynchronize(c->stream));
+	return PFG_OK;
+}
+
 int pfg_hessian_apply(pfg_context *c, const double *values, const double *p, int mem, double *q)
 {
 	if (!c || !check_mem(mem) || (c->m.N && (!p || !q))) return fail(c, PFG_ERR_INVALID, "bad arguments");
+	if (int st_l = settle_hessian(c, values == nullptr)) return st_l;
 	if (!c->has_pattern) return fail(c, PFG_ERR_STATE, "no Hessian assembled yet (pattern not built)");
 	DeviceGuard g(c->device);
 	const size_t ndof = 3 * (size_t)c->m.N;
@@ -1298,6 +1348,7 @@ int pfg_hessian_vector(pfg_context *c, const double *u, const double *p, int mem
 int pfg_hessian_device_csc(pfg_context *c, const int **outer, const int **inner, double **values)
 {
 	if (!c) return PFG_ERR_INVALID;
+	if (int st = settle_hessian(c, values != nullptr)) return st;
 	if (!c->has_pattern) return fail(c, PFG_ERR_STATE, "pattern not built");
 	if (outer) *outer = c->d_outer;
 	if (inner) *inner = c->d_inner;
@@ -1552,6 +1603,7 @@ int pfg_cg_solve(pfg_context *c, int system, const double *values, const double 
 	int n, ngroups;
 	if (system == PFG_SYS_FULL)
 	{
+		if (int st_l = settle_hessian(c, values == nullptr)) return st_l;
 		if (!c->has_pattern) return fail(c, PFG_ERR_STATE, "no Hessian assembled (pfg_hessian)");
 		outer = c->d_outer;
 		inner = c->d_inner;
@@ -1662,10 +1714,11 @@ int pfg_selftest_cg_give_up(pfg_context *c, int how)
 
 // the system's device pattern: n, nnz, outer, inner, values; PFG_OK or a state error
 static int system_pattern(pfg_context *c, int system, int &n, long long &nnz, const int *&outer, const int *&inner,
-						  const double *&vals)
+						  const double *&vals, bool read_values)
 {
 	if (system == PFG_SYS_FULL)
 	{
+		if (int st = settle_hessian(c, read_values)) return st;
 		if (!c->has_pattern) return fail(c, PFG_ERR_STATE, "no Hessian assembled (pfg_hessian)");
 		n = 3 * c->m.N;
 		nnz = c->pat.nnz;
@@ -1723,7 +1776,7 @@ int pfg_direct_analyze(pfg_context *c, int system)
 	long long nnz;
 	const int *d_outer, *d_inner;
 	const double *vals;
-	if (int st = system_pattern(c, system, n, nnz, d_outer, d_inner, vals)) return st;
+	if (int st = system_pattern(c, system, n, nnz, d_outer, d_inner, vals, false)) return st;
 	DeviceGuard g(c->device);
 	free_direct(c);
 	std::vector<int> outer((size_t)n + 1), inner((size_t)std::max<long long>(nnz, 1));
@@ -1752,7 +1805,7 @@ int pfg_direct_factorize(pfg_context *c, int system, const double *values)
 	long long nnz;
 	const int *d_outer, *d_inner;
 	const double *vals;
-	if (int st = system_pattern(c, system, n, nnz, d_outer, d_inner, vals)) return st;
+	if (int st = system_pattern(c, system, n, nnz, d_outer, d_inner, vals, values == nullptr)) return st;
 	if (!c->direct || c->direct_system != system || direct_n(c->direct) != n || direct_nnz(c->direct) != nnz)
 		return fail(c, PFG_ERR_STATE, "pattern not analysed (pfg_direct_analyze)");
 	if (values) vals = values;

@@ -188,6 +188,8 @@ cudaError_t launch_tile_build(int E, int n_nodes, int nn, const int *inc_off, co
 // H p of the NeoHookean Hessian at u without the matrix (FP64); sc.vec_stage as the gradient's
 cudaError_t launch_hessian_vector(const DevMesh &m, const double *u, const double *p, double *out, const Scratch &sc,
 								  cudaStream_t s);
+cudaError_t launch_copy3(const double *a, long long na, const double *b, long long nb, const double *c, long long nc, double *dst,
+						 cudaStream_t s);
 cudaError_t launch_pack_lame(int E, const double *lambda, const double *mu, double2 *lame, cudaStream_t s);
 cudaError_t launch_material_vjp(const DevMesh &m, const double *u, const double *adj, double *out, cudaStream_t s);
 bool shape_vjp_tiled(const DevMesh &m); // whether launch_shape_vjp reads m.gtile

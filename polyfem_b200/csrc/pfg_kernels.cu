@@ -2637,6 +2637,56 @@ __global__ void k_pack_lame(int E, const double *__restrict__ lambda, const doub
 	if (e < E) lame[e] = make_double2(lambda[e], mu[e]);
 }
 
+// three vectors into one buffer, one behind the other (one launch instead of three copies; a
+// block of 1,024 doubles of one vector, in pairs where source and place allow): P2 32^3, 10.6 MB
+// read and written, 3.9 us
+__global__ void __launch_bounds__(256) k_copy3(const double *__restrict__ a, long long na, const double *__restrict__ b, long long nb,
+											   const double *__restrict__ c, long long nc, double *__restrict__ dst)
+{
+	long long i0 = blockIdx.x * 1024LL;
+	const double *src = a;
+	long long n = na;
+	if (i0 >= (na + 1023) / 1024 * 1024)
+	{
+		i0 -= (na + 1023) / 1024 * 1024;
+		dst += na;
+		src = b;
+		n = nb;
+		if (i0 >= (nb + 1023) / 1024 * 1024)
+		{
+			i0 -= (nb + 1023) / 1024 * 1024;
+			dst += nb;
+			src = c;
+			n = nc;
+		}
+	}
+	src += i0;
+	dst += i0;
+	const int m = (int)min(1024LL, n - i0);
+	if (m == 1024 && (((size_t)src | (size_t)dst) & 15) == 0)
+	{
+		const double2 *s2 = reinterpret_cast<const double2 *>(src);
+		double2 *d2 = reinterpret_cast<double2 *>(dst);
+		const double2 x = s2[threadIdx.x], y = s2[threadIdx.x + 256];
+		d2[threadIdx.x] = x;
+		d2[threadIdx.x + 256] = y;
+		return;
+	}
+	double v[4];
+#pragma unroll
+	for (int k = 0; k < 4; ++k) v[k] = threadIdx.x + 256 * k < m ? src[threadIdx.x + 256 * k] : 0.0;
+#pragma unroll
+	for (int k = 0; k < 4; ++k)
+		if (threadIdx.x + 256 * k < m) dst[threadIdx.x + 256 * k] = v[k];
+}
+cudaError_t launch_copy3(const double *a, long long na, const double *b, long long nb, const double *c, long long nc, double *dst,
+						 cudaStream_t s)
+{
+	const long long blocks = (na + 1023) / 1024 + (nb + 1023) / 1024 + (nc + 1023) / 1024;
+	if (blocks > 0) k_copy3<<<(unsigned)blocks, 256, 0, s>>>(a, na, b, nb, c, nc, dst);
+	return cudaGetLastError();
+}
+
 // ---------------------------------------------------------------------------
 // adjoint: material derivative (ElasticForceDerivative.cpp:91-132)
 // ---------------------------------------------------------------------------

@@ -98,3 +98,84 @@ def test_hessian_vector_equals_assembled_product(require_gpu, et, g):
     with pytest.raises(PfgError):
         asm.hessian_vector(u2, p)
     asm.close()
+
+
+@pytest.mark.parametrize("et", [M.P1_TET, M.P2_TET, M.Q1_HEX], ids=["P1", "P2", "Q1"])
+def test_backward_leaves_its_hessian_in_the_context(require_gpu, et):
+    """After a backward the context's matrix is H at the u, lambda, mu and X of that backward,
+    whatever was set, evaluated or overwritten in place since; a later assembly replaces it, an
+    assembly into the caller's array does not; and a captured backward leaves the matrix of
+    each replay."""
+    import ctypes
+
+    import torch
+
+    from polyfem_b200 import _lib
+    from polyfem_b200.autograd import elastic_force
+
+    mesh, lam, mu, u, p = make_case(et, 3, seed=5, jitter=0.1)
+    t = lambda a: torch.tensor(a, dtype=torch.float64, device="cuda")
+    X = np.ascontiguousarray(mesh.X).reshape(-1)
+
+    def assembled(u_, lam_, mu_, X_):
+        ref = NeoHookeanAssembler.from_mesh(mesh, lam_, mu_)
+        ref.set_rest_positions(t(X_))
+        v = ref.assemble_hessian_values(t(u_))
+        ref.close()
+        return v
+
+    def backward(asm, u_, lam_, mu_, X_):
+        leaves = [t(a).requires_grad_(True) for a in (u_, lam_, mu_, X_)]
+        (elastic_force(*leaves, asm) * t(p)).sum().backward()
+        return leaves
+
+    asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
+    leaves = backward(asm, u, lam, mu, X)
+    with torch.no_grad():
+        for a in leaves:
+            a.data.mul_(1.5)  # an optimiser's step
+        elastic_force(*leaves, asm)  # the next forward, other parameters
+    v = assembled(u, lam, mu, X)
+    asm.assemble_hessian_values(t(0.5 * u))  # into the caller's array
+    asm.set_material("SaintVenant")
+    asm.assemble_gradient(t(u))
+    q = asm.hessian_apply(t(p))
+    assert torch.equal(q, asm.hessian_apply(t(p), v))
+    asm.set_material("NeoHookean")
+    ptr = ctypes.c_void_p()
+    _lib.check(_lib.lib().pfg_hessian_device_csc(asm.handle, None, None, ctypes.byref(ptr)), asm.handle, "csc")
+    assert ptr.value
+    # another backward, then an assembly that replaces its matrix
+    backward(asm, 0.7 * u, 2 * lam, mu, X)
+    assert torch.equal(asm.hessian_apply(t(p)), asm.hessian_apply(t(p), assembled(0.7 * u, 2 * lam, mu, X)))
+    backward(asm, u, lam, mu, X)
+    asm.assemble_hessian_into_context(t(0.3 * u))
+    assert torch.equal(asm.hessian_apply(t(p)), asm.hessian_apply(t(p), assembled(0.3 * u, lam, mu, X)))
+    asm.close()
+
+    # the first read is the solver's
+    asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
+    backward(asm, 0 * u, lam, mu, X)
+    from polyfem_b200 import ConjugateGradient
+    cg = ConjugateGradient(asm, "full")
+    cg.set_parameters({"max_iter": 7, "tolerance": 0.0})
+    b = t(p)
+    x = cg.solve(b)
+    cg.factorize(assembled(0 * u, lam, mu, X))
+    assert torch.equal(cg.solve(b), x)
+    asm.close()
+
+    # captured
+    asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
+    leaves = backward(asm, u, lam, mu, X)  # buffers of the first call
+    asm.hessian_apply(t(p))
+    uu, pp = t(u), t(p)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        asm.hessian_later(uu)
+    for f in (1.0, 0.4):
+        uu.copy_(t(f * u))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(asm.hessian_apply(pp), asm.hessian_apply(pp, assembled(f * u, lam, mu, X)))
+    asm.close()
