@@ -11,6 +11,7 @@
 #include "pfg_internal.h"
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <limits>
 #include <cstdio>
@@ -76,6 +77,7 @@ struct pfg_context
 	size_t cg_n = 0;
 	CgPlan cg_plan[2];
 	int cg_give_up = 0; // pfg_selftest_cg_give_up
+	int cg_most = 0;    // pfg_selftest_cg_most
 	// mass matrix (pfg_mass_matrix): values for host-mode calls, staged densities
 	double *d_mass = nullptr, *d_rho = nullptr;
 	// lumped diagonal for host-mode pfg_lump_matrix calls (3N doubles)
@@ -1625,7 +1627,8 @@ int pfg_cg_solve(pfg_context *c, int system, const double *values, const double 
 	if (n > 0 && (!b || !x)) return fail(c, PFG_ERR_INVALID, "b or x NULL");
 	DeviceGuard g(c->device);
 	CgPlan &plan = c->cg_plan[system];
-	if (n > 0 && !plan.run) PFG_CUDA(c, build_cg_plan(n, ngroups, groups, outer, inner, &plan, c->stream));
+	if (plan.run && plan.limited && plan.stream != c->stream) free_cg_plan(&plan); // another stream may have more SMs
+	if (n > 0 && !plan.run) PFG_CUDA(c, build_cg_plan(n, ngroups, groups, outer, inner, INT_MAX, &plan, c->stream));
 	const size_t nn = std::max<size_t>(n, 1), ns = 4 * (size_t)std::max(ngroups, 1);
 	const size_t need = 7 * ns + 4 * nn + cg_partials_doubles() + CG_NSC;
 	if (c->cg_n < need)
@@ -1671,6 +1674,11 @@ int pfg_cg_solve(pfg_context *c, int system, const double *values, const double 
 		};
 		int st;
 		PFG_CUDA(c, launch_cg_start(n, ngroups, groups, outer, inner, vals, db, guess != 0, tol, dx, w, c->stream));
+		const auto fits = [&](int ctas, cudaError_t &e) {
+			e = c->cg_most && ctas > c->cg_most ? cudaErrorCooperativeLaunchTooLarge : launch_cg_probe(ctas, plan, vals, w, c->stream);
+			if (e == cudaErrorCooperativeLaunchTooLarge) cudaGetLastError();
+			return e == cudaSuccess;
+		};
 		// iterations in batches, stopped on the device at convergence: one launch and one
 		// read of the scalars each; a batch of the largest matrix takes about a second
 		constexpr int CG_BATCH = 256;
@@ -1681,7 +1689,29 @@ int pfg_cg_solve(pfg_context *c, int system, const double *values, const double 
 			if (k > 0)
 			{
 				const int missing = c->cg_give_up == 2 && plan.ctas > 1 ? 1 : 0;
-				PFG_CUDA(c, launch_cg_iterations(k, plan, vals, values == nullptr, w, c->stream, missing));
+				cudaError_t e = c->cg_most && plan.ctas > c->cg_most ? cudaErrorCooperativeLaunchTooLarge
+																	 : launch_cg_iterations(k, plan, vals, values == nullptr, w, c->stream, missing);
+				if (e == cudaErrorCooperativeLaunchTooLarge && queued == 0)
+				{
+					// the stream has part of the SMs (a limited context): the most CTAs it takes
+					cudaGetLastError();
+					int lo = 0, hi = plan.ctas;
+					while (hi - lo > 1)
+					{
+						const int mid = (lo + hi) / 2;
+						if (fits(mid, e)) lo = mid;
+						else if (e == cudaErrorCooperativeLaunchTooLarge) hi = mid;
+						else return cuda_fail(c, e, "conjugate gradient launch");
+					}
+					if (lo == 0) return cuda_fail(c, cudaErrorCooperativeLaunchTooLarge, "conjugate gradient launch");
+					free_cg_plan(&plan);
+					PFG_CUDA(c, build_cg_plan(n, ngroups, groups, outer, inner, lo, &plan, c->stream));
+					plan.limited = true;
+					plan.stream = c->stream;
+					PFG_CUDA(c, launch_cg_start(n, ngroups, groups, outer, inner, vals, db, guess != 0, tol, dx, w, c->stream));
+					e = launch_cg_iterations(k, plan, vals, values == nullptr, w, c->stream);
+				}
+				if (e != cudaSuccess) return cuda_fail(c, e, "conjugate gradient launch");
 				if (c->cg_give_up == 1) PFG_CUDA(c, cudaMemsetAsync(w.sc + CG_ERR, 1, sizeof(int), c->stream));
 				c->cg_give_up = 0;
 			}
@@ -1709,6 +1739,18 @@ int pfg_selftest_cg_give_up(pfg_context *c, int how)
 {
 	if (!c || how < 0 || how > 2) return PFG_ERR_INVALID;
 	c->cg_give_up = how;
+	return PFG_OK;
+}
+
+// For the tests, not part of the API: launches of more than `most` CTAs (0: any) are answered as
+// the runtime answers them where the stream has only so many SMs; the plans are built anew.
+int pfg_selftest_cg_most(pfg_context *c, int most)
+{
+	if (!c || most < 0) return PFG_ERR_INVALID;
+	DeviceGuard g(c->device);
+	PFG_CUDA(c, cudaStreamSynchronize(c->stream));
+	for (CgPlan &p : c->cg_plan) free_cg_plan(&p);
+	c->cg_most = most;
 	return PFG_OK;
 }
 

@@ -237,9 +237,14 @@ struct CgPlan
 	uint4 *packets = nullptr;
 	unsigned gen = 0;
 	int ctas = 0, nnz = 0, chunks = 0;
+	int missing = 0; // CTAs that a launch leaves out and still waits for (a test)
 	bool resident = false; // every run is at most two chunks
+	bool limited = false;  // fewer CTAs than the device has SMs, because `stream` takes no more
+	cudaStream_t stream = nullptr;
 };
-cudaError_t build_cg_plan(int n, int ngroups, const int *groups, const int *outer, const int *inner, CgPlan *pl, cudaStream_t s);
+// max_ctas: at most so many CTAs (one per SM the launch can have)
+cudaError_t build_cg_plan(int n, int ngroups, const int *groups, const int *outer, const int *inner, int max_ctas, CgPlan *pl,
+						  cudaStream_t s);
 void free_cg_plan(CgPlan *pl);
 size_t cg_partials_doubles();
 // invd[j] = 1 / H(j, j), or 1 where the diagonal is zero or structurally absent
@@ -263,6 +268,8 @@ cudaError_t launch_cg_start(int n, int ngroups, const int *groups, const int *ou
 // the launch (the give-up test's way to have a wait run out)
 cudaError_t launch_cg_iterations(int count, CgPlan &pl, const double *vals, bool padded, const CgWork &w, cudaStream_t s,
 								 int missing = 0);
+// whether the stream takes the iterations' kernel with so many CTAs (it runs, and does nothing)
+cudaError_t launch_cg_probe(int ctas, CgPlan &pl, const double *vals, const CgWork &w, cudaStream_t s);
 // the slots of x -> the dense x
 cudaError_t launch_cg_unpack(int ngroups, const int *groups, const CgWork &w, double *x, cudaStream_t s);
 

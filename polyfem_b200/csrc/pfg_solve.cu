@@ -617,7 +617,7 @@ __global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals,
 				own_chunks = 0;
 				break;
 			}
-	const int G = pl.ctas;
+	const int G = gridDim.x + pl.missing; // (pl.ctas, the same, from the parameters: 0.1 us an iteration slower at P1 13^3)
 	double *q = nown <= CG_OWN ? S.q : w.q + 4 * (size_t)g0, *po = S.p;
 	unsigned gen = pl.gen; // exchange numbers given to earlier launches
 	uint4 *pk = pl.packets + 1; // 16 bytes off the 32-byte sectors: P1 13^3 12.8 us an iteration, 13.1 on them
@@ -810,7 +810,8 @@ cudaError_t launch_cg_diag_inv(int n, const int *outer, const int *inner, const 
 
 // The plan of a system, from its device pattern: descriptors, chunks and runs on the host
 // (a few words per group), neighbour codes on the device.
-cudaError_t build_cg_plan(int n, int ngroups, const int *groups, const int *outer, const int *inner, CgPlan *pl, cudaStream_t s)
+cudaError_t build_cg_plan(int n, int ngroups, const int *groups, const int *outer, const int *inner, int max_ctas, CgPlan *pl,
+						  cudaStream_t s)
 {
 	*pl = CgPlan();
 	if (ngroups <= 0) return cudaSuccess;
@@ -845,7 +846,7 @@ cudaError_t build_cg_plan(int n, int ngroups, const int *groups, const int *oute
 		long long total = 0;
 		for (int g = 0; g < ngroups; ++g) total += values_of(g);
 		// two groups for a warp at least: each CTA more costs every exchange
-		const int ctas = std::min({sms, CG_MAX_CTAS, (ngroups + 2 * CG_W - 1) / (2 * CG_W)}), warps = ctas * CG_W;
+		const int ctas = std::min({sms, max_ctas, CG_MAX_CTAS, (ngroups + 2 * CG_W - 1) / (2 * CG_W)}), warps = ctas * CG_W;
 		std::vector<int4> chunk, blob; // blob: codes are filled in on the device
 		std::vector<int2> run;
 		std::vector<long long> at(ngroups);
@@ -961,10 +962,17 @@ cudaError_t launch_cg_iterations(int count, CgPlan &pl, const double *vals, bool
 	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(CgSmem));
 	if (e != cudaSuccess) return e;
 	CgPlan p = pl;
+	p.missing = missing;
 	pl.gen += 3u * (unsigned)count; // at most three exchanges an iteration
 	CgWork ww = w;
 	void *args[] = {&p, &vals, &ww, &count};
 	return cudaLaunchCooperativeKernel(kernel, dim3(pl.ctas - missing), dim3(CG_CTA), args, sizeof(CgSmem), s);
+}
+
+cudaError_t launch_cg_probe(int ctas, CgPlan &pl, const double *vals, const CgWork &w, cudaStream_t s)
+{
+	const cudaError_t e = cudaMemsetAsync(w.sc + CG_DONE, 0xff, sizeof(double), s); // not zero: k_cg returns at once
+	return e == cudaSuccess ? launch_cg_iterations(0, pl, vals, true, w, s, pl.ctas - ctas) : e;
 }
 
 cudaError_t launch_cg_unpack(int ngroups, const int *groups, const CgWork &w, double *x, cudaStream_t s)

@@ -250,3 +250,33 @@ def test_a_wait_that_gave_up_is_reported_and_leaves_nothing_behind(require_gpu, 
         for _ in range(2):
             assert np.array_equal(bits(cg.solve(b)), x)
     asm.close()
+
+
+@pytest.mark.parametrize("most", [1, 2, 7])
+@pytest.mark.parametrize("et,g", [(M.P1_TET, 3), (M.P1_TET, 9), (M.Q1_HEX, 13)], ids=["small", "P1-9", "Q1-13"])
+def test_streams_with_part_of_the_device(require_gpu, et, g, most):
+    """Where the stream takes fewer CTAs than the plan has (a context limited to part of the
+    SMs), the solve goes on with as many as it takes: the oracle's iteration count and the same
+    residual, also with runs of many chunks and more than 256 groups a CTA; on another stream
+    the whole device again."""
+    import torch
+    mesh, lam, mu, u, _ = make_case(et, g, seed=8)
+    asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
+    asm.set_dirichlet(np.arange(12))
+    H = asm.assemble_hessian_reduced(u, "fp64", project_to_psd=True)
+    b = np.random.default_rng(3).standard_normal(H.shape[0])
+    cg = ConjugateGradient(asm, "reduced")
+    cg.set_parameters({"tolerance": 1e-10, "max_iter": 5000})
+    x = cg.solve(b)
+    _, it_o, _ = conjugate_gradient(H.indptr, H.indices, H.data, b, 1e-10, 5000)
+    assert lib().pfg_selftest_cg_most(asm.handle, most) == 0
+    for _ in range(2):
+        y = cg.solve(b)
+        assert np.linalg.norm(b - H @ y) <= 2e-10 * np.linalg.norm(b)
+        assert abs(cg.get_info()["solver_iter"] - it_o) <= max(2, it_o // 20)
+    with torch.cuda.stream(torch.cuda.Stream()):
+        z = cg.solve(torch.tensor(b, device="cuda")).cpu().numpy()
+    assert np.linalg.norm(b - H @ z) <= 2e-10 * np.linalg.norm(b)
+    assert lib().pfg_selftest_cg_most(asm.handle, 0) == 0
+    assert np.array_equal(cg.solve(b), x)
+    asm.close()
