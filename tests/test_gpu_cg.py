@@ -280,3 +280,39 @@ def test_streams_with_part_of_the_device(require_gpu, et, g, most):
     assert lib().pfg_selftest_cg_most(asm.handle, 0) == 0
     assert np.array_equal(cg.solve(b), x)
     asm.close()
+
+
+def test_many_groups_per_cta(require_gpu):
+    """More than 256 column groups a CTA, whose H p (and, with resident runs, direction) stay in
+    global memory: P1 34^3 on the whole device (streaming), and 2,000 single tetrahedra on 20
+    CTAs (resident), against a host product and the oracle's iteration count."""
+    mesh, lam, mu, u, _ = make_case(M.P1_TET, 34, seed=8)
+    asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
+    face = np.flatnonzero(mesh.node_pos[:, 0] <= 1e-12)
+    asm.set_dirichlet((3 * face[:, None] + np.arange(3)).ravel())
+    H = asm.assemble_hessian_reduced(u, "fp64", project_to_psd=True)
+    _check_solve(ConjugateGradient(asm, "reduced"), H, None)
+    asm.close()
+
+    import torch
+    rng = np.random.default_rng(4)
+    corner = np.array([[0, 0, 0], [1, 0, 0], [0, 1, 0], [0, 0, 1.0]])
+    X = (corner[None] + 3 * np.arange(2000)[:, None, None] + 0.1 * rng.uniform(-1, 1, (2000, 4, 3))).reshape(-1, 3)
+    asm = NeoHookeanAssembler(M.P1_TET, np.arange(8000, dtype=np.int32).reshape(2000, 4), X, 1e5, 5e4)
+    H = asm.assemble_hessian(np.zeros(24000))
+    H.sort_indices()
+    H.setdiag(H.diagonal() + 10.0 ** rng.uniform(3, 5, 24000))  # free bodies: a shift for a definite matrix
+    assert lib().pfg_selftest_cg_most(asm.handle, 20) == 0
+    _check_solve(ConjugateGradient(asm, "full"), H, torch.tensor(H.data, device="cuda"))
+    asm.close()
+
+
+def _check_solve(cg, H, values):
+    cg.factorize(values)
+    cg.set_parameters({"tolerance": 1e-10, "max_iter": 5000})
+    b = np.random.default_rng(3).standard_normal(H.shape[0])
+    x = cg.solve(b)
+    assert np.linalg.norm(b - H @ x) <= 2e-10 * np.linalg.norm(b)
+    _, it_o, _ = conjugate_gradient(H.indptr, H.indices, H.data, b, 1e-10, 5000)
+    assert abs(cg.get_info()["solver_iter"] - it_o) <= max(2, it_o // 20)
+    assert np.array_equal(cg.solve(b), x)
