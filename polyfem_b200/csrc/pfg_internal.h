@@ -227,7 +227,7 @@ struct CgWork
 // Static plan of a system's pattern, built once: the groups in chunks that a warp's stage
 // of k_cg holds (chunk: blob, its size, first value, values or 0 for one group too large to
 // stage; blob: descriptors and neighbour codes; big: the codes of those large groups), every
-// warp's run of chunks with its first group, three arrays of 32-byte packets per CTA, the
+// warp's run of chunks with its first group, three arrays of packets, two per CTA, the
 // exchange numbers handed out so far; the counts of values and chunks
 struct CgPlan
 {

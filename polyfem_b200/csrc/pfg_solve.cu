@@ -273,6 +273,11 @@ constexpr int CG_COST = 736;
 constexpr int CG_BLOB = 180;              // ints of a chunk's descriptors and codes
 constexpr int CG_SPIN = 1 << 20;          // bound of every wait (an exchange: about a second)
 constexpr int CG_PK = 5, CG_MAX_CTAS = 32 * CG_PK; // packets per lane of an exchange; CTAs
+// uint4 from one CTA's packet to the next.  Packets side by side share the L2 slices that all
+// CTAs poll, and what an exchange takes then hangs on where the array lies: P1 13^3 9.7 to
+// 13.3 us an iteration at 19 places within 512 KB, 256 bytes apart 9.8 to 10.3 (P1 8^3 8.0 to
+// 10.7, 6.9 to 7.8); streaming P2 20^3 49.5 to 51.9, 128 bytes apart 47.1 to 48.4, 256 47.9 to 48.8
+constexpr int CG_PITCH = 16;
 constexpr int CG_OWN = 256;               // own groups whose q (and, FUSED, p) stay in shared memory
 // a chunk's blob: head (first group, groups, -, -), a descriptor per group (first column * 4 +
 // columns, first value in the chunk, rows | all blocks 3 x 3 << 30, first code in the blob)
@@ -355,7 +360,7 @@ __device__ __forceinline__ uint4 ld_packet(const uint4 *p)
 	asm volatile("ld.relaxed.gpu.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
 	return v;
 }
-template <int NV, bool DATA>
+template <int NV, bool DATA, int PITCH>
 __device__ __forceinline__ bool exchange(CgSmem &S, uint4 *pk, int G, unsigned gen, double a, double b, int *err, Sums &out)
 {
 	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -374,7 +379,7 @@ __device__ __forceinline__ bool exchange(CgSmem &S, uint4 *pk, int G, unsigned g
 		if (lane == 0)
 		{
 			if (DATA) __threadfence(); // the CTA's writes before its packet
-			uint4 *mine = pk + 2 * blockIdx.x;
+			uint4 *mine = pk + PITCH * blockIdx.x;
 			asm volatile("st.relaxed.gpu.global.v4.u32 [%0], {%1, %2, %3, %2};" ::"l"(mine), "r"(__double2loint(a)), "r"(gen),
 						 "r"(__double2hiint(a))
 						 : "memory");
@@ -393,8 +398,8 @@ __device__ __forceinline__ bool exchange(CgSmem &S, uint4 *pk, int G, unsigned g
 			for (int j = 0; j < CG_PK; ++j)
 			{
 				const int i = min(lane + 32 * j, G - 1);
-				u[j] = ld_packet(pk + 2 * i);
-				if (NV > 1) v[j] = ld_packet(pk + 2 * i + 1);
+				u[j] = ld_packet(pk + PITCH * i);
+				if (NV > 1) v[j] = ld_packet(pk + PITCH * i + 1);
 			}
 			wait = false;
 #pragma unroll
@@ -620,7 +625,8 @@ __global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals,
 	const int G = gridDim.x + pl.missing; // (pl.ctas, the same, from the parameters: 0.1 us an iteration slower at P1 13^3)
 	double *q = nown <= CG_OWN ? S.q : w.q + 4 * (size_t)g0, *po = S.p;
 	unsigned gen = pl.gen; // exchange numbers given to earlier launches
-	uint4 *pk = pl.packets + 1; // 16 bytes off the 32-byte sectors: P1 13^3 12.8 us an iteration, 13.1 on them
+	uint4 *pk = pl.packets;
+	constexpr int PITCH = FUSED ? CG_PITCH : CG_PITCH / 2;
 	const double thr = sc[CG_THR];
 	double rz = sc[CG_RZ], rr = sc[CG_RR], alpha = 0.0, beta = it0 ? sc[CG_BETA] : 0.0;
 	bool done = false, ok = true;
@@ -713,7 +719,7 @@ __global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals,
 			}
 		}
 		Sums sum;
-		if (!(ok = exchange<1, false>(S, pk, G, ++gen, pq, 0.0, err, sum))) break;
+		if (!(ok = exchange<1, false, PITCH>(S, pk, G, ++gen, pq, 0.0, err, sum))) break;
 		alpha = rz / sum.a;
 		// x += alpha p, r -= alpha q, z = D^-1 r
 		const double *pown = FUSED && nown <= CG_OWN ? po : pout + 4 * (size_t)g0;
@@ -740,7 +746,7 @@ __global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals,
 				srz = fma(r.y, z.y, fma(r.x, z.x, srz));
 			}
 		}
-		if (!(ok = exchange<2, FUSED>(S, pk + 2 * G, G, ++gen, srr, srz, err, sum))) break;
+		if (!(ok = exchange<2, FUSED, PITCH>(S, pk + PITCH * G, G, ++gen, srr, srz, err, sum))) break;
 		rr = sum.a;
 		if (rr < thr)
 		{
@@ -764,7 +770,7 @@ __global__ void __launch_bounds__(CG_CTA, 1) k_cg(CgPlan pl, const double *vals,
 					*reinterpret_cast<double2 *>(w.p + o + h) = p;
 				}
 			}
-			if (!(ok = exchange<0, true>(S, pk + 4 * G, G, ++gen, 0.0, 0.0, err, sum))) break;
+			if (!(ok = exchange<0, true, PITCH>(S, pk + 2 * PITCH * G, G, ++gen, 0.0, 0.0, err, sum))) break;
 		}
 	}
 	// copies still in flight (the solve stopped, or a wait gave up): wait for them before leaving
@@ -906,7 +912,7 @@ cudaError_t build_cg_plan(int n, int ngroups, const int *groups, const int *oute
 		for (long long &x : at)
 			if (x < 0) x = big0 + (-1 - x);
 		blob.resize(blob.size() + (size_t)(nbig + 3) / 4);
-		const size_t packet_bytes = 16 + 96 * (size_t)ctas;
+		const size_t packet_bytes = 3 * sizeof(uint4) * CG_PITCH * (size_t)ctas;
 		if ((e = cudaMalloc(&pl->run, sizeof(int2) * run.size())) == cudaSuccess &&
 			(e = cudaMalloc(&pl->chunk, sizeof(int4) * chunk.size())) == cudaSuccess &&
 			(e = cudaMalloc(&pl->blob, sizeof(int4) * blob.size())) == cudaSuccess &&
