@@ -153,6 +153,17 @@ __device__ __forceinline__ void put_contributions(const DevMesh &m, const TilePl
 	}
 }
 
+// 1/q: hardware approximation refined by two Newton-Raphson steps r += r (1 - q r)
+__device__ __forceinline__ double rcp_nr(double q)
+{
+	double r;
+	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(q));
+	double e = fma(-q, r, 1.0);
+	r = fma(r, e, r);
+	e = fma(-q, r, 1.0);
+	return fma(r, e, r);
+}
+
 __device__ __forceinline__ double warp_sum(double v)
 {
 #pragma unroll

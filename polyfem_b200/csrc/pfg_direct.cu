@@ -34,7 +34,7 @@
 // Every sum is taken in a fixed order, so factor and solution are bitwise
 // deterministic.  Fronts are dense lower triangles of m (m + 1) / 2 doubles
 // (packed columns), all resident for the factor's lifetime.
-#include "pfg_internal.h"
+#include "pfg_device.cuh"
 #include "pfgpu.h"
 
 #include <algorithm>
@@ -804,15 +804,11 @@ __device__ __forceinline__ void dmma_8x8(double (&c)[2], double a, double b)
 	asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1},{%2},{%3},{%0,%1};" : "+d"(c[0]), "+d"(c[1]) : "d"(a), "d"(b));
 }
 
-// 1 / d of a positive finite d: hardware approximation and two Newton steps where its
-// flush-to-zero range is safe, else the division
+// 1 / d of a positive finite d: rcp_nr where its flush-to-zero range is safe, else the division
 __device__ __forceinline__ double pivot_rcp(double d)
 {
 	if (!(d > 1e-290 && d < 1e290)) return 1.0 / d;
-	double r;
-	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
-	r = fma(fma(-d, r, 1.0), r, r);
-	return fma(fma(-d, r, 1.0), r, r);
+	return rcp_nr(d);
 }
 
 // The factorisation runs in panels of 64 columns, two at a time:

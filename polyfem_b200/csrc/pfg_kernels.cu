@@ -137,11 +137,11 @@ __global__ void __launch_bounds__(NT) k_energy_per_element(DevMesh m, const doub
 // ---------------------------------------------------------------------------
 // gradient (NLAssembler::assemble_gradient)
 // ---------------------------------------------------------------------------
-#ifndef PFG_P1_CTAS
-#define PFG_P1_CTAS 6
-#endif
+// P1 CTAs per SM: with tiles the nodal sums' buffer leaves room for six (48^3: 47.3 us, for eight 49.7)
+template <class EL, bool TILED>
+__host__ __device__ constexpr int gradient_min_ctas() { return EL::ET == 1 ? (TILED ? 6 : 8) : 1; }
 template <class EL, class T, int NT, bool TILED>
-__global__ void __launch_bounds__(NT, EL::ET == 1 ? (TILED ? PFG_P1_CTAS : 8) : 1) k_gradient(DevMesh m, const double *__restrict__ u, double *__restrict__ stage,
+__global__ void __launch_bounds__(NT, gradient_min_ctas<EL, TILED>()) k_gradient(DevMesh m, const double *__restrict__ u, double *__restrict__ stage,
 												 unsigned long long *inverted)
 {
 	const bool on = blockIdx.x * NT + threadIdx.x < m.E;
@@ -1359,17 +1359,6 @@ __device__ __forceinline__ double warp_allmax(double v)
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
 	return v;
-}
-
-// 1/q: hardware approximation refined by two Newton-Raphson steps r += r (1 - q r)
-__device__ __forceinline__ double rcp_nr(double q)
-{
-	double r;
-	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(q));
-	double e = fma(-q, r, 1.0);
-	r = fma(r, e, r);
-	e = fma(-q, r, 1.0);
-	return fma(r, e, r);
 }
 
 // Number of eigenvalues of the scaled T below x: the sign changes of the leading

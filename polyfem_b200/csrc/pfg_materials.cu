@@ -1125,13 +1125,12 @@ __global__ void __launch_bounds__(NT) k_le_material_vjp(DevMesh m, const double 
 //   (C:M + P V^T - tr(V) P) : grad p = a.(Q g) + (P g).grad p[:, d] - g_d (P : grad p),
 // with a = grad u[:, d] and Q = C : grad p (C is symmetric in its index pairs).
 // Element contributions into one slot per geometric incidence.
-template <class EL, int MAT, int NT, bool TILED>
+template <class EL, int MAT, int NT>
 __global__ void __launch_bounds__(NT) k_ad_shape_vjp(DevMesh m, const double *__restrict__ u,
 													 const double *__restrict__ adj, double *__restrict__ stage)
 {
-	const bool on = blockIdx.x * NT + threadIdx.x < m.E;
-	if (!TILED && !on) return;
-	const int e = on ? blockIdx.x * NT + threadIdx.x : m.E - 1;
+	const int e = blockIdx.x * NT + threadIdx.x;
+	if (e >= m.E) return;
 	double Xg[EL::NG][3], U[EL::N][3], Pn[EL::N][3], acc[EL::NG][3];
 	int nodes[EL::N];
 	load_geom<EL, double>(m, e, Xg);
@@ -1182,7 +1181,7 @@ __global__ void __launch_bounds__(NT) k_ad_shape_vjp(DevMesh m, const double *__
 			}
 		}
 	}
-	put_contributions<EL::NG, NT, TILED>(m, m.gtile, m.g_eb_inc, stage, e, on, acc);
+	put_contributions<EL::NG, NT, false>(m, m.gtile, m.g_eb_inc, stage, e, true, acc);
 }
 
 // ---------------------------------------------------------------------------
@@ -1294,7 +1293,7 @@ cudaError_t launch_ad_shape_vjp_stage(const DevMesh &m, const double *u, const d
 	const int nb = ad_blocks_for(m.E, NT);
 	auto launch = [&](auto el, auto mat) {
 		using EL = decltype(el);
-		k_ad_shape_vjp<EL, decltype(mat)::value, NT, false><<<nb, NT, 0, s>>>(m, u, adj, sc.vec_stage);
+		k_ad_shape_vjp<EL, decltype(mat)::value, NT><<<nb, NT, 0, s>>>(m, u, adj, sc.vec_stage);
 	};
 	auto by_el = [&](auto mat) -> cudaError_t {
 		switch (m.et)
