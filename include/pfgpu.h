@@ -162,7 +162,8 @@ int pfg_hessian_vector(pfg_context *ctx, const double *u, const double *p, int m
  * assembles it only when a call reads that matrix or its device pointer is asked for
  * (pfg_hessian_apply, pfg_cg_solve and pfg_direct_factorize with NULL values on the full
  * system, pfg_hessian_device_csc).  u, the parameters and the positions are copied.  On a
- * stream under capture the matrix is assembled at once. */
+ * stream under capture the matrix is assembled at once, and a matrix left for later before
+ * the capture cannot be read for the first time in it (PFG_ERR_STATE). */
 int pfg_hessian_later(pfg_context *ctx, const double *u, int mem);
 
 /* Device pointers of the context-owned CSC arrays (valid until pfg_destroy). */

@@ -527,6 +527,11 @@ int settle_hessian(pfg_context *c, bool values)
 {
 	if (!c->later) return PFG_OK;
 	DeviceGuard g(c->device);
+	// captured, the assembly would be done again by every replay, over whatever matrix there is then
+	cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+	PFG_CUDA(c, cudaStreamIsCapturing(c->stream, &capture));
+	if (capture != cudaStreamCaptureStatusNone)
+		return fail(c, PFG_ERR_STATE, "the context's matrix is still to be assembled (pfg_hessian_later): read it once before the capture");
 	int st;
 	if (!c->has_pattern && (st = build_pattern(c))) return st;
 	if (!values) return PFG_OK;

@@ -261,10 +261,11 @@ __global__ void __launch_bounds__(CG_NT) k_cg_unpack(int ngroups, const int *__r
 // 32-byte slot of p and nine values from shared memory (a lane per row gathered p in 8-byte
 // pieces and read an index per row instead of per block).
 //
-// Per iteration at P2 24^3 / P1 13^3: 115 / 24.8 us with five launches, 79 / 12.0 us here
-// (8 and 20 warps, or stages of 500 values: 105, 96 and 96 us at P2 24^3).  What is left at
-// P2 24^3 is 41 us of streaming (240 MB, half of it from L2), the products that do not
-// overlap it, and 4 us an exchange; at P1 13^3 two exchanges and the chains behind them.
+// Per iteration at P2 24^3 / P1 13^3: 115 / 24.8 us with five launches, 75 / 10.1 us here
+// (before CG_PITCH 79 / 12.0; then 8 and 20 warps, or stages of 500 values: 105, 96 and 96 us
+// at P2 24^3).  What is left at P2 24^3 is 41 us of streaming (240 MB, half of it from L2), the
+// products that do not overlap it, and three exchanges; at P1 13^3 two exchanges and the chains
+// behind them.
 constexpr int CG_W = 16, CG_CTA = 32 * CG_W;
 // doubles of values a stage holds: three whole groups of 27 3 x 3 blocks, an inner node of a
 // hexahedral mesh (640 values, two of them: Q1 64^3 / 96^3 181 / 622 us an iteration, 169 / 543

@@ -3,7 +3,7 @@ the adjoint kernels, checked against the CPU oracle and central finite differenc
 import numpy as np
 import pytest
 
-from polyfem_b200 import NeoHookeanAssembler
+from polyfem_b200 import NeoHookeanAssembler, PfgError
 from polyfem_b200 import mesh as M
 
 from _cases import make_case, rel_err
@@ -79,7 +79,6 @@ def test_hessian_vector_equals_assembled_product(require_gpu, et, g):
     the rows of inverted elements; refused for another formulation."""
     import torch
 
-    from polyfem_b200 import PfgError
     from _cases import permuted
     mesh, lam, mu, u, p = make_case(et, g, seed=31, jitter=0.1 if g > 1 else 0.0)
     m2, u2, _, pe = permuted(mesh, u, seed=2)
@@ -167,8 +166,14 @@ def test_backward_leaves_its_hessian_in_the_context(require_gpu, et):
 
     # captured
     asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
-    leaves = backward(asm, u, lam, mu, X)  # buffers of the first call
-    asm.hessian_apply(t(p))
+    leaves = backward(asm, u, lam, mu, X)
+    graph = torch.cuda.CUDAGraph()
+    qq, pp = asm.hessian_vector(t(u), t(p)), t(p)
+    with torch.cuda.graph(graph):
+        qq.add_(0.0)
+        with pytest.raises(PfgError):  # its first read cannot be part of a graph
+            asm.hessian_apply(pp)
+    asm.hessian_apply(t(p))  # buffers of the first call
     uu, pp = t(u), t(p)
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
