@@ -272,7 +272,7 @@ constexpr int CG_W = 16, CG_CTA = 32 * CG_W;
 // with three; P2 24^3 80.4, 78.9)
 constexpr int CG_COST = 736;
 constexpr int CG_BLOB = 180;              // ints of a chunk's descriptors and codes
-constexpr int CG_SPIN = 1 << 20;          // bound of every wait (an exchange: about a second)
+constexpr int CG_SPIN = 1 << 22;          // bound of every wait (an exchange: about a second)
 constexpr int CG_PK = 5, CG_MAX_CTAS = 32 * CG_PK; // packets per lane of an exchange; CTAs
 // uint4 from one CTA's packet to the next.  Packets side by side share the L2 slices that all
 // CTAs poll, and what an exchange takes then hangs on where the array lies: P1 13^3 9.7 to

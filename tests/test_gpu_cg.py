@@ -316,3 +316,45 @@ def _check_solve(cg, H, values):
     _, it_o, _ = conjugate_gradient(H.indptr, H.indices, H.data, b, 1e-10, 5000)
     assert abs(cg.get_info()["solver_iter"] - it_o) <= max(2, it_o // 20)
     assert np.array_equal(cg.solve(b), x)
+
+
+def test_two_threads_on_two_streams(require_gpu):
+    """Two contexts solve at the same time from two threads, each on its own stream, with launches
+    that each want the whole device: both return the bits of a solve alone."""
+    import threading
+
+    import torch
+    solvers = []
+    for et, g in ((M.P1_TET, 20), (M.Q1_HEX, 16)):
+        mesh, lam, mu, u, _ = make_case(et, g, seed=5)
+        asm = NeoHookeanAssembler.from_mesh(mesh, lam, mu)
+        asm.set_dirichlet(np.arange(9))
+        v = asm.assemble_hessian_reduced_values(torch.tensor(u, device="cuda"), project_to_psd=True)
+        b = torch.tensor(np.random.default_rng(2).standard_normal(asm.n_free), device="cuda")
+        cg = ConjugateGradient(asm, "reduced")
+        cg.set_parameters({"tolerance": 0.0, "max_iter": 300})
+        cg.factorize(v)
+        solvers.append((asm, cg, b, cg.solve(b).clone()))
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(k):
+        _, cg, b, x = solvers[k]
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                for _ in range(8):
+                    y = cg.solve(b)
+                    torch.cuda.current_stream().synchronize()
+                    if not torch.equal(y, x):
+                        wrong.append(k)
+        except Exception as e:
+            wrong.append(repr(e))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
+    for asm, _, _, _ in solvers:
+        asm.close()
