@@ -226,14 +226,17 @@ class NeoHookeanAssembler:
         check(lib().pfg_hessian_apply(self._h, vptr, ptrs[0], mem, optr), self._h, "pfg_hessian_apply")
         return out
 
-    def hessian_vector(self, u, p):
+    def hessian_vector(self, u, p, later: bool = False):
         """q = H(u) p in FP64 without assembling H (pfg_hessian_vector; NeoHookean only):
-        one element pass and a gather.  Deterministic; the context's matrix is not touched."""
+        one element pass and a gather.  Deterministic; the context's matrix is not touched,
+        or with ``later`` becomes H(u) as hessian_later(u) makes it."""
         self._check_len(u, self.n_dofs, "u")
         self._check_len(p, self.n_dofs, "p")
         mem, ptrs, keep = self._prepare(u, p)
         out, optr = self._alloc(mem, self.n_dofs)
         check(lib().pfg_hessian_vector(self._h, ptrs[0], ptrs[1], mem, optr), self._h, "pfg_hessian_vector")
+        if later:
+            check(lib().pfg_hessian_later(self._h, ptrs[0], mem), self._h, "pfg_hessian_later")
         return out
 
     def hessian_later(self, u):

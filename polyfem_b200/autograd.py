@@ -63,8 +63,7 @@ class ElasticForce(torch.autograd.Function):
             g_X = asm.force_shape_derivative(u, p, ctx.precision).reshape(X.shape)
         if ctx.needs_input_grad[0]:
             if asm.material == "NeoHookean" and ctx.precision in ("fp64", PFG_FP64):
-                g_u = asm.hessian_vector(u, p)
-                asm.hessian_later(u)  # the context's matrix is H here too, when it is read
+                g_u = asm.hessian_vector(u, p, later=True)  # the context's matrix is H here too, when it is read
             else:
                 asm.assemble_hessian_into_context(u, ctx.precision)
                 g_u = asm.hessian_apply(p)

@@ -254,14 +254,14 @@ int ensure_staging(pfg_context *c, int mem, size_t out_doubles)
 // shares less in a tile).  Gradient, us, a slot per incidence -> tiles:
 //   P1 20^3 (192,000 incidences) 8.9 -> 8.7, 17^3 7.1 -> 7.8, 48^3 64 -> 41; 48^3 with part of its
 //   elements shuffled, at 0.48 slots per incidence 74 -> 59, at 0.58 78 -> 77, at 1.0 94 -> 107
-//   P2 12^3 (103,680) 15.5 -> 11.2, 32^3 (0.31) 62 -> 53; 24^3 at 0.32 27.8 -> 27.6, at 0.41 28 -> 31
+//   P2 6^3 (12,960) 14.3 -> 9.7, 32^3 (0.31) 62 -> 53; 24^3 at 0.32 27.8 -> 27.6, at 0.41 28 -> 31
 //   Q1 48^3 (884,736) 43 -> 39, 36^3 (373,248) 23.4 -> 23.9; 63^3 at 0.38 98 -> 89, at 0.48 99 -> 100
 struct TileRule
 {
 	long long incidences;
 	double slots;
 };
-TileRule tile_rule(int nn) { return nn == 4 ? TileRule{200000, 0.5} : nn == 10 ? TileRule{100000, 0.35} : TileRule{500000, 0.4}; }
+TileRule tile_rule(int nn) { return nn == 4 ? TileRule{200000, 0.5} : nn == 10 ? TileRule{10000, 0.35} : TileRule{500000, 0.4}; }
 
 // The tile plan of a connectivity, built on the device by the first call that sums nodal
 // contributions: counts in the stage (not in use yet), one read of the number of slots, one
@@ -279,18 +279,21 @@ int build_tile_plan(pfg_context *c, int nn, int N, const int *inc_off, const int
 	PFG_CUDA(c, cudaMemcpyAsync(&n_slots, counts + N + 1 + tiles, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
 	PFG_CUDA(c, cudaStreamSynchronize(c->stream));
 	if ((double)n_slots > rule.slots * (double)n_inc) return PFG_OK;
-	const size_t ints = n_counts + (size_t)tiles + (size_t)n_slots, shorts = (size_t)n_inc + (size_t)n_slots + (size_t)tiles;
+	// the build's scratch lies in the stage too, behind the counts
+	const size_t scratch = (sizeof(int) * n_counts + 15) / 16 * 16;
+	if (scratch + tile_scratch_bytes(E, n_slots) > stage_bytes) return PFG_OK;
+	const size_t ints = n_counts + (size_t)n_slots, shorts = (size_t)n_inc + (size_t)n_slots + (size_t)tiles;
 	if (cudaMalloc(mem, sizeof(int) * ints + sizeof(unsigned short) * shorts) != cudaSuccess)
 	{
 		cudaGetLastError();
 		*mem = nullptr;
 		return PFG_OK;
 	}
-	int *kept = static_cast<int *>(*mem), *slot = kept + n_counts + tiles;
-	unsigned *cur = reinterpret_cast<unsigned *>(kept + n_counts);
+	int *kept = static_cast<int *>(*mem), *slot = kept + n_counts;
 	unsigned short *pos = reinterpret_cast<unsigned short *>(slot + n_slots), *start = pos + n_inc;
 	PFG_CUDA(c, cudaMemcpyAsync(kept, counts, sizeof(int) * n_counts, cudaMemcpyDeviceToDevice, c->stream));
-	PFG_CUDA(c, launch_tile_build(E, N, nn, inc_off, inc_eb, kept, cur, pos, start, slot, c->stream));
+	PFG_CUDA(c, launch_tile_build(E, N, nn, inc_off, inc_eb, kept, n_slots,
+								  reinterpret_cast<char *>(c->d_vec_stage) + scratch, pos, start, slot, c->stream));
 	tp->pos = pos;
 	tp->off = kept + N + 1;
 	tp->start = start;

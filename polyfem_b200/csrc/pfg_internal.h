@@ -15,7 +15,6 @@ constexpr int TILE_E = 128;
 // summed over the tile in shared memory first, one slot per (tile, node), so most of the
 // traffic to the slots and back disappears (the tile's elements share most of their nodes).
 //  pos      : [E*n] place of (e, a) in the tile's buffer, grouped by node, elements ascending
-//             (the groups in any order: it does not enter the sums)
 //  off      : [tiles+1] first tile node of every tile
 //  start    : [nodes of all tiles + tiles] first place of every tile node, an end entry per tile
 //  slot     : [nodes of all tiles] the slot of the tile node's sum, slots in node order, tiles ascending
@@ -180,11 +179,12 @@ cudaError_t launch_ad_shape_vjp_stage(const DevMesh &m, const double *u, const d
 									  cudaStream_t s);
 // TilePlan arrays.  counts (tile_count_ints ints): node_off (N+1), off (tiles+1) and block
 // sums; launch_tile_counts fills off, its last entry the number of slots, launch_tile_build
-// finishes node_off and fills the rest (cur: an int per tile, scratch)
+// finishes node_off and fills the rest (scratch: tile_scratch_bytes, 8-byte aligned)
 size_t tile_count_ints(int E, int n_nodes);
 cudaError_t launch_tile_counts(int E, int n_nodes, int nn, const int *inc_off, const int *inc_eb, int *counts, cudaStream_t s);
-cudaError_t launch_tile_build(int E, int n_nodes, int nn, const int *inc_off, const int *inc_eb, int *counts, unsigned *cur,
-							  unsigned short *pos, unsigned short *start, int *slot, cudaStream_t s);
+size_t tile_scratch_bytes(int E, int n_slots);
+cudaError_t launch_tile_build(int E, int n_nodes, int nn, const int *inc_off, const int *inc_eb, int *counts, int n_slots,
+							  void *scratch, unsigned short *pos, unsigned short *start, int *slot, cudaStream_t s);
 // H p of the NeoHookean Hessian at u without the matrix (FP64); sc.vec_stage as the gradient's
 cudaError_t launch_hessian_vector(const DevMesh &m, const double *u, const double *p, double *out, const Scratch &sc,
 								  cudaStream_t s);
