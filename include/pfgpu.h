@@ -142,8 +142,8 @@ int pfg_hessian_pattern_copy(pfg_context *ctx, int *outer, int *inner, int mem);
 int pfg_hessian(pfg_context *ctx, const double *u, int mem, int prec, int project_psd, double *values);
 
 /* q = H p (3N doubles each, in `mem`) with the Hessian in the full pattern:
- * `values` (device memory, nnz doubles) or, when NULL, the values of the last
- * pfg_hessian call that wrote into the context.  H is symmetric, so this is also
+ * `values` (device memory, nnz doubles) or, when NULL, the context's matrix: of the last
+ * pfg_hessian call that wrote into the context, or pfg_hessian_later.  H is symmetric, so this is also
  * H^T p, the product the reference's adjoint terms form with Eigen's sparse
  * matrix-vector product (e.g. `term = -hessian.transpose() * adjoint_zeroed`,
  * optimization/force_derivatives/PressureForceDerivative.cpp:24).  One warp per
