@@ -3,7 +3,7 @@ the adjoint kernels, checked against the CPU oracle and central finite differenc
 import numpy as np
 import pytest
 
-from polyfem_b200 import NeoHookeanAssembler, PfgError
+from polyfem_b200 import NeoHookeanAssembler
 from polyfem_b200 import mesh as M
 
 from _cases import make_case, rel_err
@@ -79,6 +79,7 @@ def test_hessian_vector_equals_assembled_product(require_gpu, et, g):
     the rows of inverted elements; refused for another formulation."""
     import torch
 
+    from polyfem_b200 import PfgError
     from _cases import permuted
     mesh, lam, mu, u, p = make_case(et, g, seed=31, jitter=0.1 if g > 1 else 0.0)
     m2, u2, _, pe = permuted(mesh, u, seed=2)
@@ -109,7 +110,7 @@ def test_backward_leaves_its_hessian_in_the_context(require_gpu, et):
 
     import torch
 
-    from polyfem_b200 import _lib
+    from polyfem_b200 import PfgError, _lib
     from polyfem_b200.autograd import elastic_force
 
     mesh, lam, mu, u, p = make_case(et, 3, seed=5, jitter=0.1)
